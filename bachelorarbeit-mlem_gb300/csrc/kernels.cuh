@@ -76,7 +76,7 @@ void launch_csr_tma(const DevCsr& op, const float* x, const EpiArgs& epi, uint32
 void launch_scatter_tma(const DevCsr& A, const float* ratio, float* bp, uint32_t* err, L2Window win,
                         cudaStream_t s);
 // bp[idx] += val * ratio[row] over the rows of A (calcBwProj_none_trans, kernel.cu:165-177);
-// lanes per row 8/16/32, unroll = 16-byte vectors per lane in flight (1 or 2).
+// lanes per row 8/16/32, unroll = entries per lane in flight (2 or 4).
 void launch_scatter(const DevCsr& A, const float* ratio, float* bp, int lanes, int unroll, L2Window win,
                     cudaStream_t s);
 // One pass over A: sum = A[r,:]·x, ratio = g[r]/sum, bp[idx] += val*ratio.

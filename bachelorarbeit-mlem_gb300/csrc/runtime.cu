@@ -161,10 +161,10 @@ static void cols_out(const mlem_matrix* m, float* dst, const float* src, cudaStr
 }
 static bool permuted(const mlem_matrix* m) { return m->lor_of || m->vox_of; }
 
-// Lanes per row of A (8, 16 or 32) and 16-byte vectors per lane in flight (1
-// or 2) for the scatter back projection, timed once per matrix (ratio 1 into a
+// Lanes per row of A (8, 16 or 32) and entries per lane in flight (2 or 4)
+// for the scatter back projection, timed once per matrix (ratio 1 into a
 // scratch image), and whether the TMA-ring scatter beats the best of them.
-// Returns the lanes; m->scatter_unroll holds the vectors, m->scatter_tma the
+// Returns the lanes; m->scatter_unroll holds the entries, m->scatter_tma the
 // choice of the TMA ring inside the MLEM iteration.
 int scatter_lanes(mlem_matrix* m) {
     if (m->scatter_lanes) return m->scatter_lanes;
@@ -172,7 +172,7 @@ int scatter_lanes(mlem_matrix* m) {
     cudaStream_t s = m->stream;
     float *r = nullptr, *bp = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
-    int best_l = pick_lanes(A.nnz, A.nrows) < 8 ? 8 : pick_lanes(A.nnz, A.nrows), best_u = 1;
+    int best_l = pick_lanes(A.nnz, A.nrows) < 8 ? 8 : pick_lanes(A.nnz, A.nrows), best_u = 4;
     float best = 1e30f;
     try {
         MLEM_CUDA(cudaMalloc(&r, sizeof(float) * std::max<uint32_t>(A.nrows, 1)));
@@ -183,7 +183,7 @@ int scatter_lanes(mlem_matrix* m) {
         MLEM_CUDA(cudaEventCreate(&e0));
         MLEM_CUDA(cudaEventCreate(&e1));
         for (int lanes : {8, 16, 32})
-            for (int u : {1, 2}) {
+            for (int u : {2, 4}) {
                 launch_scatter(A, r, bp, lanes, u, {}, s);
                 MLEM_CUDA(cudaEventRecord(e0, s));
                 for (int q = 0; q < 2; ++q) launch_scatter(A, r, bp, lanes, u, {}, s);

@@ -1,7 +1,8 @@
 // scatter.cuh — grouped vector reductions of the scatter back projection
-// (bp[col] += val · ratio[row], calcBwProj_none_trans, kernel.cu:165-177),
-// shared by the scatter kernel (spmv.cu) and the fused single pass
-// (spmv_fused.cu).
+// (bp[col] += val · ratio[row], calcBwProj_none_trans, kernel.cu:165-177) for
+// the kernels whose lanes hold four consecutive entries: the register and the
+// staged form of the fused single pass (spmv.cu, spmv_fused.cu) and the
+// scatter through shared-memory rings (spmv_tma.cu).
 #pragma once
 
 #include "common.cuh"

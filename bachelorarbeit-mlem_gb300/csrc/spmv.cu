@@ -274,13 +274,49 @@ __device__ __forceinline__ void scatter4(float* __restrict__ bp, uint32_t ncols,
     scatter4_mask(bp, ncols, c, p, use);
 }
 
-// LPR lanes per row of A; each lane loads U 16-byte vectors of (column,
-// value) before it scatters them (U loads per lane in flight).
+// Adds val * r of the entries [s, t) of one row to bp, by one lane of an
+// LPR-lane group: LPR consecutive entries per instruction, U of them loaded
+// before they are added.  What bounds the scatter is the number of 32-byte
+// sectors that the reductions send to L2, and the lanes of one instruction
+// that add into the same sector share a request.  Consecutive entries of a row
+// mostly do (ascending columns): 0.31 / 0.28 sectors per nonzero on the 3-D
+// mid / 12 GB-class matrix in the locality layout (0.42 / 0.36 in the natural
+// one), against 0.54 / 0.48 requests when each lane held four consecutive
+// entries and sent them as 16-byte vector reductions.  Measured, every ratio
+// nonzero: k_scatter 0.717 -> 0.485 ms (mid) and 4.12 -> 2.87 ms (12 GB
+// class); k_fused_rescan 4.40 -> 3.19 ms.  No slower in sum, hence not built:
+// 16-byte groups compacted in shared memory (3.01 ms), the next entries
+// loaded before the reductions (3.06), the row prefetched into L2 (2.98), 8
+// entries in flight (2.95).
+template <typename V, int LPR, int U>
+__device__ __forceinline__ void scatter_row(const uint32_t* __restrict__ idx, const V* __restrict__ val, uint64_t s,
+                                            uint64_t t, int sub, float r, float* __restrict__ bp) {
+    // from a 32-byte boundary, so that a group's loads split no more sectors than they must
+    for (uint64_t e = (s & ~7ull) + sub; e < t; e += LPR * U) {
+        uint32_t c[U];
+        float a[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint64_t q = e + u * LPR;
+            if (q < t) {
+                c[u] = ld_cached(idx + q);
+                a[u] = Val4<V>::one_cached(val, q);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint64_t q = e + u * LPR;
+            if (q >= s && q < t) atomicAdd(bp + c[u], __fmul_rn(a[u], r));
+        }
+    }
+}
+
+// LPR lanes per row of A.
 template <typename V, int LPR, int U>
 __global__ void __launch_bounds__(256)
 k_scatter(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ idx,
           const V* __restrict__ val, const float* __restrict__ ratio, uint32_t nrows,
-          float* __restrict__ bp, uint32_t ncols) {
+          float* __restrict__ bp) {
     const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t row = gt / LPR;
     const int sub = threadIdx.x & (LPR - 1);
@@ -289,24 +325,7 @@ k_scatter(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ idx,
     const float r = ratio[row];
     const uint64_t s = rowptr[row], t = rowptr[row + 1];
     if (r == 0.0f) return;  // adds of val*0 leave bp unchanged
-    const uint4* idx4 = reinterpret_cast<const uint4*>(idx);
-    const uint64_t v1 = (t + 3) >> 2;
-    for (uint64_t v = (s >> 2) + sub; v < v1; v += (uint64_t)LPR * U) {
-        Vec4<V> p[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (v + (uint64_t)u * LPR < v1) p[u].load(idx4, val, v + (uint64_t)u * LPR);
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const uint64_t vu = v + (uint64_t)u * LPR;
-            if (vu < v1) {
-                float prod[4];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) prod[k] = __fmul_rn(p[u].a[k], r);
-                scatter4(bp, ncols, p[u].c, prod, vu << 2, s, t);
-            }
-        }
-    }
+    scatter_row<V, LPR, U>(idx, val, s, t, sub, r, bp);
 }
 
 // One warp per row of A: the row's vectors stay in registers between the
@@ -376,14 +395,13 @@ k_fused(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ idx,
 // LPR lanes per row sums the row exactly as k_csrvec<V, LPR, U> does (same
 // order of additions), computes the ratio, then walks the row a second time
 // (its vectors were streamed a moment before, so L2 serves them) and
-// scatters val * ratio with the grouped vector reductions.  A crosses HBM
-// once per iteration.
+// scatters val * ratio (scatter_row).  A crosses HBM once per iteration.
 template <typename V, int LPR, int U, bool ORD>
 __global__ void __launch_bounds__(256)
 k_fused_rescan(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ idx,
                const V* __restrict__ val, const float* __restrict__ x, uint32_t nrows,
                const int32_t* __restrict__ g, float* __restrict__ bp, float* __restrict__ fwproj,
-               uint32_t ncols, const uint32_t* __restrict__ order) {
+               const uint32_t* __restrict__ order) {
     const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t k = gt / LPR;
     const int sub = threadIdx.x & (LPR - 1);
@@ -403,16 +421,7 @@ k_fused_rescan(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__
     if (sub == 0 && fwproj) fwproj[row] = acc;
     const float r = (acc != 0.0f) ? __fdiv_rn((float)gr, acc) : 0.0f;
     if (r == 0.0f) return;  // adds of val*0 leave bp unchanged
-    const uint4* idx4 = reinterpret_cast<const uint4*>(idx);
-    const uint64_t v1 = (t + 3) >> 2;
-    for (uint64_t v = (s >> 2) + sub; v < v1; v += LPR) {
-        Vec4<V> p;
-        p.load(idx4, val, v);
-        float prod[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) prod[q] = __fmul_rn(p.a[q], r);
-        scatter4(bp, ncols, p.c, prod, v << 2, s, t);
-    }
+    scatter_row<V, LPR, 4>(idx, val, s, t, sub, r, bp);
 }
 
 // calcUpdate (kernel.cu:34-37) for the scatter forms: f * bp / norm, left to right.
@@ -613,16 +622,16 @@ void scatter_dispatch(const DevCsr& A, const float* ratio, float* bp, int lanes,
     auto go = [&](auto kern, int lpr) {
         const uint64_t threads = (uint64_t)A.nrows * lpr;
         launch_ex(kern, dim3(ceil_div_u(threads, 256)), dim3(256), 0, s, win, A.rowptr, A.idx, val,
-                  ratio, A.nrows, bp, A.ncols);
+                  ratio, A.nrows, bp);
     };
-    if (unroll >= 2) {
+    if (unroll >= 4) {
+        if (lanes >= 32) go(k_scatter<V, 32, 4>, 32);
+        else if (lanes >= 16) go(k_scatter<V, 16, 4>, 16);
+        else go(k_scatter<V, 8, 4>, 8);
+    } else {
         if (lanes >= 32) go(k_scatter<V, 32, 2>, 32);
         else if (lanes >= 16) go(k_scatter<V, 16, 2>, 16);
         else go(k_scatter<V, 8, 2>, 8);
-    } else {
-        if (lanes >= 32) go(k_scatter<V, 32, 1>, 32);
-        else if (lanes >= 16) go(k_scatter<V, 16, 1>, 16);
-        else go(k_scatter<V, 8, 1>, 8);
     }
 }
 
@@ -709,10 +718,10 @@ void rescan_ord(const DevCsr& A, const float* x, const int32_t* g, float* bp, fl
     const V* val = static_cast<const V*>(A.val);
     if (ordered)
         launch_ex(k_fused_rescan<V, LPR, U, true>, grid, block, 0, s, win, A.rowptr, A.idx, val, x, A.nrows, g, bp,
-                  fwproj, A.ncols, (const uint32_t*)A.order);
+                  fwproj, (const uint32_t*)A.order);
     else
         launch_ex(k_fused_rescan<V, LPR, U, false>, grid, block, 0, s, win, A.rowptr, A.idx, val, x, A.nrows, g, bp,
-                  fwproj, A.ncols, (const uint32_t*)nullptr);
+                  fwproj, (const uint32_t*)nullptr);
 }
 template <typename V>
 void rescan_cfg(const DevCsr& A, const float* x, const int32_t* g, float* bp, float* fwproj, int lanes, int unroll,
