@@ -54,7 +54,14 @@ void launch_csr_ilv(const DevCsr& op, const float* x, const EpiArgs& epi, int un
                     cudaStream_t s);
 // Delta-compressed (16-bit) column indices: build from the u32 indices, and
 // the projection that reads them.
-void build_d16(DevCsr& op, cudaStream_t s);
+// Rows out of column order are sorted on the host first (sort_rows) or leave
+// the operand without the copy (returns false).
+bool build_d16(DevCsr& op, bool sort_rows, cudaStream_t s);
+void free_d16(DevCsr& op);
+// Mean row length from which rows get 8 lanes: bfloat16 A / A^T of rows of 239 /
+// 210 entries 0.109 / 0.118 ms with 8 lanes, 0.121 / 0.126 ms with 4; below
+// 128 the padding to 64 entries outweighs it.
+constexpr uint64_t kD16LongRow = 128;
 // unroll: 1 or 2 vectors of 8 entries in flight per lane (the lanes per row
 // are those the layout was built for).
 void launch_csr_d16(const DevCsr& op, const float* x, const EpiArgs& epi, int unroll, L2Window win, cudaStream_t s);

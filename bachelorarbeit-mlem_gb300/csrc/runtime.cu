@@ -89,10 +89,7 @@ static void free_csr(DevCsr& c) {
     cudaFree(c.rowptr);
     cudaFree(c.idx);
     cudaFree(c.val);
-    cudaFree(c.dvptr);
-    cudaFree(c.dbase);
-    cudaFree(c.d16);
-    cudaFree(c.dval);
+    free_d16(c);
     cudaFree(c.idx_ilv);
     cudaFree(c.val_ilv);
     cudaFree(c.order);
@@ -457,12 +454,34 @@ static void launch_cfg(mlem_matrix* m, const DevCsr& op, const float* x, const E
     }
 }
 
+static void d16_cands(const DevCsr& op, std::vector<ProjCfg>& cand) {
+    for (int u : {1, 2}) cand.push_back(ProjCfg{MLEM_KERNEL_D16, op.d16_lanes, u, 0.f});
+}
+
+// Whether the tuner may give the operand a delta-coded copy of its own (a
+// handle created without compress_indices): the stream it would replace
+// crosses HBM on every projection (an operand that fits in L2 gains nothing:
+// 2-D ring 8.9 us per iteration without the copy, 9.9 with it), the copy takes
+// at most a quarter of the free memory, and the handle outlives the build.
+// Building a copy costs about 15 projections and saves a fifth of each, so a
+// handle made for one call of fewer than kCopyPays iterations goes without.
+constexpr uint32_t kCopyPays = 100;
+static bool may_copy_d16(const mlem_matrix* m, const DevCsr& op) {
+    if (op.d16 || m->sym.fp_rowptr || (m->one_call && m->one_call < kCopyPays)) return false;
+    int l2 = 0;
+    size_t avail = 0, total = 0;
+    MLEM_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, m->device));
+    MLEM_CUDA(cudaMemGetInfo(&avail, &total));
+    const uint64_t stream = op.nnz * (4 + val_bytes(op.vt)), copy = op.nnz * (2 + val_bytes(op.vt)) / 4 * 5;
+    return stream > (uint64_t)l2 && copy <= avail / 4;
+}
+
 // Times every candidate configuration on the operand itself (Raw epilogue
 // into a scratch vector, x = 1) and keeps the fastest.  Runs once per
 // operand, outside any stream capture.
 static void tune_projection(mlem_matrix* m, bool transposed) {
     if (m->tuned[transposed]) return;
-    const DevCsr& op = transposed ? m->AT : m->A;
+    DevCsr& op = transposed ? m->AT : m->A;
     cudaStream_t s = m->stream;
     std::vector<ProjCfg> cand;
     const int base = pick_lanes(op.nnz, op.nrows);
@@ -478,8 +497,7 @@ static void tune_projection(mlem_matrix* m, bool transposed) {
         }
     if (base >= 16) cand.push_back(ProjCfg{MLEM_KERNEL_PERSISTENT, base, 1, 0.f, false, false});
     cand.push_back(ProjCfg{MLEM_KERNEL_TMA, 32, 2, 0.f});
-    if (op.d16)
-        for (int u : {1, 2}) cand.push_back(ProjCfg{MLEM_KERNEL_D16, op.d16_lanes, u, 0.f});
+    if (op.d16) d16_cands(op, cand);
     if (op.idx_ilv)
         for (int u : {1, 2, 4}) cand.push_back(ProjCfg{MLEM_KERNEL_ILV, 32, u, 0.f});
     if (m->sym.fp_rowptr)
@@ -503,7 +521,7 @@ static void tune_projection(mlem_matrix* m, bool transposed) {
         e.kind = Epi::Raw;
         e.out = y;
         const int reps = op.nnz > (50ull << 20) ? 2 : 4;
-        for (ProjCfg& c : cand) {
+        auto time = [&](ProjCfg& c) {
             launch_cfg(m, op, x, e, c, {}, s);  // warm-up
             MLEM_CUDA(cudaEventRecord(e0, s));
             for (int r = 0; r < reps; ++r) launch_cfg(m, op, x, e, c, {}, s);
@@ -513,6 +531,26 @@ static void tune_projection(mlem_matrix* m, bool transposed) {
             MLEM_CUDA(cudaEventElapsedTime(&ms, e0, e1));
             c.ms = ms / reps;
             if (c.ms < best.ms) best = c;
+        };
+        for (ProjCfg& c : cand) time(c);
+        if (may_copy_d16(m, op)) {
+            bool built = false;
+            try {
+                built = build_d16(op, false, s);
+            } catch (const Error& err) {  // no room after all: the operand stays as it is
+                if (err.code != MLEM_ENOMEM) throw;
+                cudaGetLastError();
+            }
+            if (built) {
+                op.d16_tuned = true;
+                std::vector<ProjCfg> more;
+                d16_cands(op, more);
+                for (ProjCfg& c : more) time(c);
+                if (best.kind != MLEM_KERNEL_D16) {
+                    free_d16(op);
+                    op.d16_tuned = false;
+                }
+            }
         }
         check_device_error(m, s);
     } catch (...) {
@@ -554,7 +592,8 @@ static ProjCfg resolve_cfg(const mlem_matrix* m, bool transposed, const mlem_run
     } else if (o.kernel == MLEM_KERNEL_TMA) {
         c.kind = MLEM_KERNEL_TMA;
     } else if (o.kernel == MLEM_KERNEL_D16) {
-        MLEM_REQUIRE(op.d16 != nullptr, MLEM_EINVAL, "kernel D16 needs a matrix created with compress_indices = 1");
+        MLEM_REQUIRE(op.d16 != nullptr && !op.d16_tuned, MLEM_EINVAL,
+                     "kernel D16 needs a matrix created with compress_indices = 1");
         c.kind = MLEM_KERNEL_D16;
         c.lanes = op.d16_lanes;
         c.unroll = o.unroll == 1 ? 1 : 2;
@@ -832,8 +871,8 @@ static void postprocess_matrix(mlem_matrix* m, const mlem_matrix_opts& o) {
     }
     m->vt = o.value_type;
     if (o.compress_indices) {
-        build_d16(A, s);
-        if (m->has_t) build_d16(m->AT, s);
+        build_d16(A, true, s);
+        if (m->has_t) build_d16(m->AT, true, s);
     }
     if (o.interleave) {
         build_ilv(A, s);
@@ -1168,10 +1207,11 @@ mlem_status mlem_matrix_get_info(const mlem_matrix* m, mlem_matrix_info* info) {
         info->sym_voxel_rows = m->sym.J;
         info->sym_fp_nnz = m->sym.fp_nnz;
         info->sym_bp_nnz = m->sym.bp_nnz;
-        info->d16_slots = 8 * m->A.dvec;
-        info->d16_slots_t = m->has_t ? 8 * m->AT.dvec : 0;
-        info->d16_lanes = (uint32_t)m->A.d16_lanes;
-        info->d16_lanes_t = m->has_t ? (uint32_t)m->AT.d16_lanes : 0;
+        const bool d = m->A.d16 && !m->A.d16_tuned, dt = m->has_t && m->AT.d16 && !m->AT.d16_tuned;
+        info->d16_slots = d ? 8 * m->A.dvec : 0;
+        info->d16_slots_t = dt ? 8 * m->AT.dvec : 0;
+        info->d16_lanes = d ? (uint32_t)m->A.d16_lanes : 0;
+        info->d16_lanes_t = dt ? (uint32_t)m->AT.d16_lanes : 0;
     });
 }
 
@@ -1618,6 +1658,7 @@ mlem_status mlem_reconstruct(const uint64_t* csr_rows, const uint32_t* csr_cols,
         mlem_matrix* m = nullptr;
         mlem_status st = mlem_matrix_create(&c, &mo, &m);
         if (st != MLEM_OK) fail(st, get_error());
+        m->one_call = iterations;
         try {
             if (host_t) {
                 // the caller supplied Aᵀ (as main.cu:100-105 does): upload it as is

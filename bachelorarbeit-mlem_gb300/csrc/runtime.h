@@ -141,6 +141,7 @@ struct mlem_matrix {
     bool scatter_tma = false;         // the TMA-ring scatter timed faster than those lanes
     mlem::FusedPlan fused;            // chunks of the staged fused pass
     mlem::FusedForm fused_auto;       // fastest form of the fused pass (timed once; ms = 0: not yet)
+    uint32_t one_call = 0;            // iterations of the only call this handle is made for (0: a caller's handle)
     bool tuned[2] = {false, false};   // csr-vector configuration of A / Aᵀ measured
     mlem::ProjCfg proj[2];
     std::mutex mu;

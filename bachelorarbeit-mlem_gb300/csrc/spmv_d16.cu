@@ -12,12 +12,19 @@
 //             dvptr[r] + k·L + l holds lane l's elements 8k..8k+7
 //   dbase[r]  first column of row r
 //   d16[8 v + j], dval[8 v + j]  the delta and the value (the operand's type)
-// A difference of 65,536 or more is bridged by dummy entries (value 0,
-// column = the earlier column + 65,535); rows are padded to whole steps with
-// delta 0 and value 0.  Dummies and padding add 4% (L = 4) to 9% (L = 8) on
-// the generated matrices in the locality layout: with FP16 values ~4.2 bytes
-// per nonzero instead of 8 (u32 + f32).  The lane sums are reduced by a fixed
-// xor tree: deterministic.
+// A difference of 65,536 or more is bridged by dummy entries (column = the
+// earlier column + 65,535) and rows are padded to whole steps with delta 0;
+// both carry the value -0.0, which no stored entry has (a stored -0.0 becomes
+// +0.0).  A row whose sum is NaN is summed again without them, so that an
+// infinite or NaN element of x that the row does not list stays out of its sum.
+//
+// What bounds it: the bytes of the stream, (2 + value) per position.  Dummies
+// and padding add 8% (A) and 14% (A^T) on the 3-D mid matrix, 9% and 16% on
+// the 12 GB class.  Measured and not kept: a half step (4 entries per lane) at
+// a row's end, 4% / 7% of padding but rows that start inside a 128-byte line
+// (mid, FP32 / FP16 values: 0.442 / 0.361 ms per iteration against 0.431 /
+// 0.313).  The lane sums (two chains per lane, even and odd elements) are
+// reduced by a fixed xor tree: deterministic.
 #include "kernels.cuh"
 
 #include <algorithm>
@@ -69,8 +76,82 @@ struct Val8<__nv_bfloat16> {
     }
 };
 
+// The value of dummies and padding.
+template <typename V>
+__device__ __forceinline__ V pad_value() {
+    V v;
+    *reinterpret_cast<uint16_t*>(&v) = 0x8000u;
+    return v;
+}
+template <>
+__device__ __forceinline__ float pad_value<float>() { return -0.0f; }
+
+// A row's sum again, in the same order, without the dummies and the padding, by
+// one thread: for rows whose sum is NaN (see the head of the file).
+template <typename V, int LPR>
+__device__ __noinline__ float d16_row_real(const uint64_t* __restrict__ dvptr, const uint32_t* __restrict__ dbase,
+                                           const uint16_t* __restrict__ d16, const V* __restrict__ dval,
+                                           const float* __restrict__ x, uint32_t row) {
+    const uint64_t v0 = dvptr[row], v1 = dvptr[row + 1];
+    float sum[LPR];
+    for (int l = 0; l < LPR; ++l) {
+        uint32_t col = dbase[row];
+        float acc[2] = {0.f, 0.f};
+        for (uint64_t v = v0 + l; v < v1; v += LPR)
+            for (int j = 0; j < 8; ++j) {
+                col += d16[8 * v + j];
+                const float a = (float)dval[8 * v + j];
+                if (__float_as_uint(a) != 0x80000000u) acc[j & 1] = fmaf(a, __ldg(x + col), acc[j & 1]);
+            }
+        sum[l] = acc[0] + acc[1];
+    }
+    for (int o = LPR / 2; o > 0; o >>= 1)
+        for (int l = 0; l < o; ++l) sum[l] += sum[l + o];
+    return sum[0];
+}
+
+// N steps of a lane: loads, columns, gathers, FMAs (even elements into acc0,
+// odd ones into acc1).  dp, vp: the lane's delta and value vector of the first.
+template <typename V, int LPR, int N>
+__device__ __forceinline__ void d16_steps(const uint4* dp, const V* vp, const float* __restrict__ x, uint32_t& prev,
+                                          float& acc0, float& acc1) {
+    uint4 dw[N];
+    float a[N][8];
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+        dw[u] = ld_stream(dp + u * LPR);
+        Val8<V>::load(vp, (uint64_t)u * LPR, a[u]);
+    }
+    uint32_t col[N][8];
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+        const uint32_t w[4] = {dw[u].x, dw[u].y, dw[u].z, dw[u].w};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            prev += (w[j >> 1] >> (16 * (j & 1))) & 0xFFFFu;
+            col[u][j] = prev;
+        }
+    }
+    float gx[N][8];
+#pragma unroll
+    for (int u = 0; u < N; ++u)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) gx[u][j] = __ldg(x + col[u][j]);
+#pragma unroll
+    for (int u = 0; u < N; ++u)
+#pragma unroll
+        for (int j = 0; j < 8; j += 2) {
+            acc0 = fmaf(a[u][j], gx[u][j], acc0);
+            acc1 = fmaf(a[u][j + 1], gx[u][j + 1], acc1);
+        }
+}
+
+// Blocks per SM, measured on the 3-D mid / 12 GB-class matrix, ms per iteration
+// with U = 1 and U = 2: FP32 values 5 blocks (48 registers) 0.431, 0.433 / 2.83,
+// 2.90, 8 and 6 blocks 0.472, 0.438 / 3.77, 2.99; FP16 values 8 and 6 blocks (32
+// and 40 registers) 0.313, 0.316 / 2.14, 2.04, 5 blocks 0.335, 0.337 / 2.08, 2.09.
 template <typename V, int EPI, int LPR, int U>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, sizeof(V) == 4 ? 5 : U == 2 ? 6 : 8)
 k_csr_d16(const uint64_t* __restrict__ dvptr, const uint32_t* __restrict__ dbase, const uint16_t* __restrict__ d16,
           const V* __restrict__ dval, const float* __restrict__ x, uint32_t nrows, const int32_t* __restrict__ g,
           float* __restrict__ out, float* __restrict__ fwproj, float* __restrict__ f, const float* __restrict__ norm) {
@@ -79,11 +160,12 @@ k_csr_d16(const uint64_t* __restrict__ dvptr, const uint32_t* __restrict__ dbase
     const bool live = row < nrows;
     const uint64_t v0 = live ? dvptr[row] : 0, v1 = live ? dvptr[row + 1] : 0;
     const uint32_t nsteps = (uint32_t)((v1 - v0) / LPR);
-    const uint4* dv = reinterpret_cast<const uint4*>(d16);
+    const uint4* dp = reinterpret_cast<const uint4*>(d16) + v0;
+    const V* vp = dval + 8 * v0;
     if (live && gl == 0 && v1 > v0) {
         // the row's vectors into L2 ahead of the loads (whole 16-byte vectors)
-        const uint64_t lo = reinterpret_cast<uint64_t>(dv + v0), nb = 16 * (v1 - v0);
-        const uint64_t lv = reinterpret_cast<uint64_t>(dval) + 8 * sizeof(V) * v0, nv = 8 * sizeof(V) * (v1 - v0);
+        const uint64_t lo = reinterpret_cast<uint64_t>(dp), nb = 16 * (v1 - v0);
+        const uint64_t lv = reinterpret_cast<uint64_t>(vp), nv = 8 * sizeof(V) * (v1 - v0);
         for (uint64_t q = 0; q < nb; q += 65536)
             asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(lo + q),
                          "r"((uint32_t)(nb - q < 65536 ? nb - q : 65536)) : "memory");
@@ -92,45 +174,21 @@ k_csr_d16(const uint64_t* __restrict__ dvptr, const uint32_t* __restrict__ dbase
                          "r"((uint32_t)(nv - q < 65536 ? nv - q : 65536)) : "memory");
     }
     uint32_t prev = live ? dbase[row] : 0u;  // column of this lane's previous element
-    float acc = 0.f;
-    for (uint32_t k = 0; k < nsteps; k += U) {
-        uint4 dw[U];
-        float a[U][8];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (k + u < nsteps) {
-                const uint64_t v = v0 + (uint64_t)(k + u) * LPR + gl;
-                dw[u] = ld_stream(dv + v);
-                Val8<V>::load(dval, v, a[u]);
-            } else {
-                dw[u] = make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) a[u][j] = 0.f;
-            }
-        }
-        uint32_t col[U][8];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const uint32_t w[4] = {dw[u].x, dw[u].y, dw[u].z, dw[u].w};
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                prev += (w[j >> 1] >> (16 * (j & 1))) & 0xFFFFu;
-                col[u][j] = prev;
-            }
-        }
-        float gx[U][8];
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) gx[u][j] = (k + u < nsteps) ? __ldg(x + col[u][j]) : 0.f;
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) acc = fmaf(a[u][j], gx[u][j], acc);
+    float acc0 = 0.f, acc1 = 0.f;
+    dp += gl;
+    vp += 8 * gl;
+    uint32_t k = 0;
+    for (; k + U <= nsteps; k += U) {
+        d16_steps<V, LPR, U>(dp, vp, x, prev, acc0, acc1);
+        dp += U * LPR;
+        vp += U * 8 * LPR;
     }
+    if (U == 2 && k < nsteps) d16_steps<V, LPR, 1>(dp, vp, x, prev, acc0, acc1);
+    float acc = acc0 + acc1;
 #pragma unroll
     for (int o = LPR / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o, LPR);
     if (live && gl == 0) {
+        if (isnan(acc)) acc = d16_row_real<V, LPR>(dvptr, dbase, d16, dval, x, row);
         if (EPI == (int)Epi::Correl) {
             out[row] = (acc != 0.0f) ? __fdiv_rn((float)g[row], acc) : 0.0f;
             if (fwproj) fwproj[row] = acc;
@@ -158,68 +216,94 @@ __global__ void k_d16_check(const uint64_t* __restrict__ rowptr, const uint32_t*
     }
 }
 
-// Walks row r's positions: a dummy wherever the next column is 65,536 or more
-// past the column L positions earlier.  emit(p, delta, e) for every position
-// (e = entry index, or ~0 for a dummy); returns the positions used.
-template <int L, class Emit>
-__device__ __forceinline__ uint64_t d16_walk(const uint32_t* __restrict__ col, uint64_t s, uint64_t t, Emit&& emit) {
-    if (s == t) return 0;
-    uint32_t ring[L];
-#pragma unroll
-    for (int i = 0; i < L; ++i) ring[i] = col[s];
-    uint64_t p = 0;
-    for (uint64_t e = s; e < t;) {
-        uint32_t earlier = ring[0];
-#pragma unroll
-        for (int i = 1; i < L; ++i)
-            if ((p % L) == (uint64_t)i) earlier = ring[i];
-        const uint32_t c = col[e];
-        uint32_t now, d;
-        uint64_t ent;
-        if (c - earlier >= 65536u) {
-            now = earlier + 65535u;
-            d = 65535u;
-            ent = ~0ull;
-        } else {
-            now = c;
-            d = c - earlier;
-            ent = e;
-            ++e;
-        }
-        emit(p, d, ent);
-#pragma unroll
-        for (int i = 0; i < L; ++i)
-            if ((p % L) == (uint64_t)i) ring[i] = now;
-        ++p;
-    }
-    return p;
-}
-
-// Vectors per row (positions rounded up to whole steps of 8·L).  One thread per row.
+// One slice (L consecutive positions, one per lane) of a row's walk by its
+// group of L lanes: lane i's position takes the next entry unless its column
+// lies 65,536 or more past `ring`, the column L positions earlier, when it
+// takes a dummy.  e = next entry on entry and on return; ent = the lane's
+// entry, ~0 for a dummy or padding; returns the lane's delta.
 template <int L>
-__global__ void k_d16_count(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ col, uint32_t rows,
-                            uint32_t* __restrict__ nvec) {
-    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x) {
-        const uint64_t n = d16_walk<L>(col, rowptr[r], rowptr[r + 1], [](uint64_t, uint32_t, uint64_t) {});
-        nvec[r] = (uint32_t)((n + 8 * L - 1) / (8 * L) * L);
+__device__ __forceinline__ uint32_t d16_slice(const uint32_t* __restrict__ col, uint64_t t, uint64_t& e, uint32_t& ring,
+                                              uint64_t& ent, unsigned mask, int gl) {
+    const bool have = e + gl < t;
+    const uint32_t c = have ? col[e + gl] : ring;
+    if (!__any_sync(mask, c - ring >= 65536u)) {
+        const uint32_t d = c - ring;
+        ent = have ? e + gl : ~0ull;
+        ring = c;
+        e += L;
+        return d;
     }
+    uint32_t d = 0;
+    ent = ~0ull;
+#pragma unroll 1
+    for (int i = 0; i < L; ++i) {
+        const uint32_t r = __shfl_sync(mask, ring, i, L);
+        if (e >= t) break;
+        const uint32_t ci = col[e];
+        const bool dummy = ci - r >= 65536u;
+        if (gl == i) {
+            d = dummy ? 65535u : ci - r;
+            ent = dummy ? ~0ull : e;
+            ring = r + d;
+        }
+        if (!dummy) ++e;
+    }
+    return d;
 }
 
-// Deltas and values at their positions (the arrays are zeroed beforehand,
-// which is the padding).  One thread per row.
+__device__ __forceinline__ unsigned group_mask(int L) { return ((1u << L) - 1u) << ((threadIdx.x & 31) & ~(L - 1)); }
+
+// Vectors per row (positions rounded up to whole steps of 8·L).  L lanes per row.
+template <int L>
+__global__ void __launch_bounds__(256)
+k_d16_count(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ col, uint32_t rows,
+            uint32_t* __restrict__ nvec) {
+    const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) / L;
+    const int gl = threadIdx.x % L;
+    if (r >= rows) return;  // whole group
+    const unsigned mask = group_mask(L);
+    uint64_t e = rowptr[r], ent;
+    const uint64_t t = rowptr[r + 1];
+    uint32_t n = 0, ring = e < t ? col[e] : 0u;
+    for (; e < t; ++n) d16_slice<L>(col, t, e, ring, ent, mask, gl);
+    if (gl == 0) nvec[r] = (n + 7) / 8 * L;
+}
+
+// Deltas and values at their positions, padding included.  L lanes per row; a
+// lane collects its 8 elements of a step in shared memory and writes them as
+// 16-byte vectors (both copies of the mid matrix: 5 ms, against 45 ms with one
+// thread per row and one store per entry).
 template <typename V, int L>
-__global__ void k_d16_fill(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ col,
-                           const V* __restrict__ val, uint32_t rows, const uint64_t* __restrict__ dvptr,
-                           uint32_t* __restrict__ dbase, uint16_t* __restrict__ d16, V* __restrict__ dval) {
-    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x) {
-        const uint64_t s = rowptr[r], t = rowptr[r + 1], v0 = dvptr[r];
-        dbase[r] = s < t ? col[s] : 0u;
-        d16_walk<L>(col, s, t, [&](uint64_t p, uint32_t d, uint64_t e) {
-            // position p: step p / (8L), lane p % L, element (p / L) % 8
-            const uint64_t v = v0 + (p / (8 * L)) * L + p % L, q = 8 * v + (p / L) % 8;
-            d16[q] = (uint16_t)d;
-            if (e != ~0ull) dval[q] = val[e];
-        });
+__global__ void __launch_bounds__(256)
+k_d16_fill(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ col, const V* __restrict__ val,
+           uint32_t rows, const uint64_t* __restrict__ dvptr, uint32_t* __restrict__ dbase,
+           uint16_t* __restrict__ d16, V* __restrict__ dval) {
+    __shared__ __align__(16) uint16_t sd[256][8];
+    __shared__ __align__(16) V sv[256][8];
+    const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) / L;
+    const int gl = threadIdx.x % L;
+    if (r >= rows) return;  // whole group
+    const unsigned mask = group_mask(L);
+    uint64_t e = rowptr[r];
+    const uint64_t t = rowptr[r + 1], v1 = dvptr[r + 1];
+    uint32_t ring = e < t ? col[e] : 0u;
+    if (gl == 0) dbase[r] = ring;
+    uint16_t* md = sd[threadIdx.x];
+    V* mv = sv[threadIdx.x];
+    for (uint64_t v = dvptr[r]; v < v1; v += L) {
+        for (int j = 0; j < 8; ++j) {
+            uint64_t ent = ~0ull;
+            uint32_t d = 0;
+            if (e < t) d = d16_slice<L>(col, t, e, ring, ent, mask, gl);
+            V a = pad_value<V>();
+            if (ent != ~0ull) a = (float)val[ent] == 0.0f ? (V)0.0f : val[ent];
+            md[j] = (uint16_t)d;
+            mv[j] = a;
+        }
+        reinterpret_cast<uint4*>(d16)[v + gl] = *reinterpret_cast<const uint4*>(md);
+#pragma unroll
+        for (int i = 0; i < (int)sizeof(V) / 2; ++i)
+            reinterpret_cast<uint4*>(dval + 8 * (v + gl))[i] = reinterpret_cast<const uint4*>(mv)[i];
     }
 }
 
@@ -227,18 +311,16 @@ unsigned grid_rows(uint32_t rows) {
     return std::max(1u, std::min<unsigned>(ceil_div_u((uint64_t)rows * 32, 256), 152u * 32u));
 }
 
-unsigned grid_threads(uint32_t rows) {
-    return std::max(1u, std::min<unsigned>(ceil_div_u(rows, 128), 152u * 32u));
-}
+unsigned grid_groups(uint32_t rows, int lanes) { return ceil_div_u((uint64_t)rows * lanes, 256); }
 
 template <typename V>
 void d16_fill(DevCsr& op, const uint32_t* idx, const void* val, cudaStream_t s) {
     if (op.d16_lanes == 4)
-        k_d16_fill<V, 4><<<grid_threads(op.nrows), 128, 0, s>>>(op.rowptr, idx, static_cast<const V*>(val), op.nrows,
-                                                                op.dvptr, op.dbase, op.d16, static_cast<V*>(op.dval));
+        k_d16_fill<V, 4><<<grid_groups(op.nrows, 4), 256, 0, s>>>(op.rowptr, idx, static_cast<const V*>(val), op.nrows,
+                                                                  op.dvptr, op.dbase, op.d16, static_cast<V*>(op.dval));
     else
-        k_d16_fill<V, 8><<<grid_threads(op.nrows), 128, 0, s>>>(op.rowptr, idx, static_cast<const V*>(val), op.nrows,
-                                                                op.dvptr, op.dbase, op.d16, static_cast<V*>(op.dval));
+        k_d16_fill<V, 8><<<grid_groups(op.nrows, 8), 256, 0, s>>>(op.rowptr, idx, static_cast<const V*>(val), op.nrows,
+                                                                  op.dvptr, op.dbase, op.d16, static_cast<V*>(op.dval));
     MLEM_LAUNCHED();
 }
 
@@ -280,9 +362,9 @@ void sorted_copy(const DevCsr& op, uint32_t*& idx, void*& val, cudaStream_t s) {
 
 template <typename V, int EPI, int LPR, int U>
 void d16_launch(const DevCsr& op, const float* x, const EpiArgs& e, L2Window win, cudaStream_t s) {
-    launch_ex(k_csr_d16<V, EPI, LPR, U>, dim3(ceil_div_u((uint64_t)op.nrows * LPR, 256)), dim3(256), 0, s, win,
-              op.dvptr, op.dbase, op.d16, static_cast<const V*>(op.dval), x, op.nrows, e.g, e.out, e.fwproj, e.f,
-              e.norm);
+    launch_ex(k_csr_d16<V, EPI, LPR, U>, dim3(grid_groups(op.nrows, LPR)), dim3(256), 0, s, win, op.dvptr, op.dbase,
+              op.d16, static_cast<const V*>(op.dval), x, op.nrows, e.g, e.out, e.fwproj,
+              e.f, e.norm);
 }
 
 template <typename V, int EPI>
@@ -307,39 +389,54 @@ void d16_dispatch(const DevCsr& op, const float* x, const EpiArgs& e, int unroll
 
 }  // namespace
 
-void build_d16(DevCsr& op, cudaStream_t s) {
+void free_d16(DevCsr& op) {
+    cudaFree(op.dvptr);
+    cudaFree(op.dbase);
+    cudaFree(op.d16);
+    cudaFree(op.dval);
+    op.dvptr = nullptr;
+    op.dbase = nullptr;
+    op.d16 = nullptr;
+    op.dval = nullptr;
+    op.dvec = 0;
+    op.d16_lanes = 0;
+}
+
+bool build_d16(DevCsr& op, bool sort_rows, cudaStream_t s) {
     const uint64_t R = std::max<uint32_t>(op.nrows, 1);
-    // 4 lanes per row for short rows, 8 for long ones (the padding to whole
-    // steps of 8 L entries costs less than 10% either way)
-    op.d16_lanes = op.nrows && op.nnz / op.nrows >= 256 ? 8 : 4;
+    // 8 lanes per row cover more neighbouring columns per gather, 4 pad short
+    // rows less (steps of 64 or 32 entries)
+    const int lanes = op.nrows && op.nnz / op.nrows >= kD16LongRow ? 8 : 4;
     // deltas need every row in ascending column order
     const uint32_t* idx = op.idx;
     const void* val = op.val;
     uint32_t* sidx = nullptr;
     void* sval = nullptr;
+    uint32_t* nvec = nullptr;
     int* flag = nullptr;
     int unsorted = 0;
-    MLEM_CUDA(cudaMallocAsync(&flag, sizeof(int), s));
-    MLEM_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), s));
-    if (op.nrows) {
-        k_d16_check<<<grid_rows(op.nrows), 256, 0, s>>>(op.rowptr, op.idx, op.nrows, flag);
-        MLEM_LAUNCHED();
-    }
-    MLEM_CUDA(cudaMemcpyAsync(&unsorted, flag, sizeof(int), cudaMemcpyDeviceToHost, s));
-    MLEM_CUDA(cudaFreeAsync(flag, s));
-    MLEM_CUDA(cudaStreamSynchronize(s));
-    if (unsorted) {
-        sorted_copy(op, sidx, sval, s);
-        idx = sidx;
-        val = sval;
-    }
-    uint32_t* nvec = nullptr;
     try {
+        MLEM_CUDA(cudaMallocAsync(&flag, sizeof(int), s));
+        MLEM_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), s));
+        if (op.nrows) {
+            k_d16_check<<<grid_rows(op.nrows), 256, 0, s>>>(op.rowptr, op.idx, op.nrows, flag);
+            MLEM_LAUNCHED();
+        }
+        MLEM_CUDA(cudaMemcpyAsync(&unsorted, flag, sizeof(int), cudaMemcpyDeviceToHost, s));
+        MLEM_CUDA(cudaFreeAsync(flag, s));
+        MLEM_CUDA(cudaStreamSynchronize(s));
+        if (unsorted && !sort_rows) return false;
+        if (unsorted) {
+            sorted_copy(op, sidx, sval, s);
+            idx = sidx;
+            val = sval;
+        }
+        op.d16_lanes = lanes;
         MLEM_CUDA(cudaMallocAsync(&nvec, sizeof(uint32_t) * R, s));
         MLEM_CUDA(cudaMalloc(&op.dvptr, sizeof(uint64_t) * (R + 1)));
         if (op.nrows) {
-            if (op.d16_lanes == 4) k_d16_count<4><<<grid_threads(op.nrows), 128, 0, s>>>(op.rowptr, idx, op.nrows, nvec);
-            else k_d16_count<8><<<grid_threads(op.nrows), 128, 0, s>>>(op.rowptr, idx, op.nrows, nvec);
+            if (lanes == 4) k_d16_count<4><<<grid_groups(op.nrows, 4), 256, 0, s>>>(op.rowptr, idx, op.nrows, nvec);
+            else k_d16_count<8><<<grid_groups(op.nrows, 8), 256, 0, s>>>(op.rowptr, idx, op.nrows, nvec);
             MLEM_LAUNCHED();
         }
         scan_counts_u64(nvec, op.dvptr, op.nrows, s);
@@ -351,8 +448,6 @@ void build_d16(DevCsr& op, cudaStream_t s) {
         MLEM_CUDA(cudaMalloc(&op.dbase, sizeof(uint32_t) * R));
         MLEM_CUDA(cudaMalloc(&op.d16, sizeof(uint16_t) * slots));
         MLEM_CUDA(cudaMalloc(&op.dval, val_bytes(op.vt) * slots));
-        MLEM_CUDA(cudaMemsetAsync(op.d16, 0, sizeof(uint16_t) * slots, s));
-        MLEM_CUDA(cudaMemsetAsync(op.dval, 0, val_bytes(op.vt) * slots, s));
         if (op.nrows) {
             switch (op.vt) {
                 case MLEM_VAL_F32: d16_fill<float>(op, idx, val, s); break;
@@ -366,11 +461,13 @@ void build_d16(DevCsr& op, cudaStream_t s) {
         cudaFree(nvec);
         cudaFree(sidx);
         cudaFree(sval);
+        free_d16(op);
         throw;
     }
     cudaFree(nvec);
     cudaFree(sidx);
     cudaFree(sval);
+    return true;
 }
 
 void launch_csr_d16(const DevCsr& op, const float* x, const EpiArgs& epi, int unroll, L2Window win, cudaStream_t s) {

@@ -86,7 +86,9 @@ typedef struct {
                                    earlier in its row, plus its value; ~2.2 B of index per
                                    nonzero instead of 4, dummies and padding included) for the
                                    csr-vector projections (kernel D16, an autotuner candidate);
-                                   with FP16 values the fastest form for a stored matrix */
+                                   with FP16 values the fastest form for a stored matrix.
+                                   0: the copy is not part of the handle, but the autotuner may
+                                   make one of its own (see MLEM_KERNEL_AUTO) */
     uint32_t interleave;        /* 1: also keep a lane-interleaved copy (16-byte loads whose
                                    gathers cover consecutive columns) for the projections */
     uint32_t layout;            /* mlem_layout: device order of rows and columns */
@@ -236,7 +238,11 @@ typedef enum {
     MLEM_KERNEL_DIRECT = 0,
     MLEM_KERNEL_TMA = 1,
     MLEM_KERNEL_PERSISTENT = 2,
-    MLEM_KERNEL_AUTO = 3, /* autotuned per matrix operand (lanes per row, vectors in flight, variant) */
+    MLEM_KERNEL_AUTO = 3, /* autotuned per matrix operand (lanes per row, vectors in flight, variant).
+                             An operand larger than L2 with ascending columns in every row also gets
+                             a delta-coded copy (the D16 form, ~1.1 * nnz * (2 + value) bytes) on its
+                             first AUTO run if that fits a quarter of the free memory; it is kept
+                             where it is the fastest and counts in mlem_matrix_info.device_bytes */
     MLEM_KERNEL_D16 = 4,  /* delta-coded indices (matrix created with compress_indices = 1) */
     MLEM_KERNEL_ILV = 5,  /* lane-interleaved copy (matrix created with interleave = 1) */
     MLEM_KERNEL_ORDERED = 6, /* DIRECT with rows in locality order (generated matrices:

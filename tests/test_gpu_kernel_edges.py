@@ -9,6 +9,8 @@ stored in 16 bits are rounded to their type before the FP64 sum).
 """
 from __future__ import annotations
 
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -73,4 +75,90 @@ def test_fused_pass_repeated_columns(pkg, O, lanes, unroll):
     m = pkg.Matrix.from_csr(*A, cols, norm=norm, build_transpose=False)
     got = m.run(g, 8, f0=f0, bp_mode=pkg.BP_FUSED, kernel=pkg.KERNEL_DIRECT, lanes=lanes, unroll=unroll)
     assert O.rel_l2(got, O.mlem_f64(A, g, norm, f0, 8)) < 1e-5
+    m.close()
+
+
+def d16_rows(seed, cols, long_rows):
+    """Ascending rows whose columns jump by more than 65,535 (once, twice, in a
+    row's first entries, back to back), repeat, and end at and around the steps of
+    8 entries per lane; mean length on the wanted side of 128."""
+    rng = np.random.default_rng(seed)
+    lens = [n for n in LENS if n <= (4099 if long_rows else 129)] * (6 if long_rows else 40)
+    rows = []
+    for i, n in enumerate(lens):
+        c = np.sort(rng.integers(0, cols if i % 3 else 3000, n))
+        if n > 12 and i % 4 == 0:
+            c[n // 2:] = np.minimum(c[n // 2:] + 200_000, cols - 1)
+            c = np.sort(c)
+        rows.append(c)
+    rp = np.zeros(len(rows) + 1, np.uint64)
+    rp[1:] = np.cumsum([len(c) for c in rows])
+    col = np.concatenate(rows).astype(np.uint32)
+    val = rng.uniform(0.05, 1.0, len(col)).astype(np.float32)
+    val[::97] = -0.0
+    return rng, rp, col, val
+
+
+@pytest.mark.parametrize("vt", [0, 1, 2])
+@pytest.mark.parametrize("long_rows", [True, False])
+@pytest.mark.parametrize("unroll", [1, 2])
+def test_delta_coded_projection(pkg, cuda, vt, long_rows, unroll):
+    """Delta-coded rows of A and of its transpose against FP64, and against the
+    csr-vector kernel where x holds infinities and NaN: an element outside a row
+    must not reach its sum through the dummies or the padding."""
+    cols = 600_000
+    rng, rp, col, val = d16_rows(31, cols, long_rows)
+    rows = len(rp) - 1
+    rid = np.repeat(np.arange(rows), np.diff(rp.astype(np.int64)))
+    v = stored(cuda, val, vt)
+    m = pkg.Matrix.from_csr(rp, col, val, cols, value_type=vt, compress=True)
+    assert m.d16["lanes"] == (8 if long_rows else 4)
+    x = rng.uniform(0.5, 1.5, cols).astype(np.float32)
+    r = rng.uniform(0.5, 1.5, rows).astype(np.float32)
+    g = cuda.zeros(rows, dtype=cuda.int32, device="cuda")
+
+    def project(x, r, **kw):
+        dx, dr = cuda.from_numpy(x).cuda(), cuda.from_numpy(r).cuda()
+        ratio, fp, bp = cuda.empty(rows, device="cuda"), cuda.empty(rows, device="cuda"), cuda.empty(cols, device="cuda")
+        m.forward_project(dx.data_ptr(), g.data_ptr(), ratio.data_ptr(), fp.data_ptr(), **kw)
+        m.back_project(dr.data_ptr(), bp.data_ptr(), **kw)
+        cuda.cuda.synchronize()
+        return fp.cpu().numpy(), bp.cpu().numpy()
+
+    fp, bp = project(x, r, kernel=pkg.KERNEL_D16, unroll=unroll)
+    want = np.bincount(rid, weights=v * x[col].astype(np.float64), minlength=rows)
+    assert np.all(np.abs(fp - want) <= (np.bincount(rid, minlength=rows) + 2) * 2.0**-24 * want)
+    want = np.bincount(col, weights=v * r[rid].astype(np.float64), minlength=cols)
+    assert np.all(np.abs(bp - want) <= (np.bincount(col, minlength=cols) + 2) * 2.0**-24 * want)
+    x[rng.choice(cols, 4000, replace=False)] = np.inf
+    x[rng.choice(cols, 4000, replace=False)] = np.nan
+    r[rng.choice(rows, 8, replace=False)] = -np.inf
+    for a, b in zip(project(x, r, kernel=pkg.KERNEL_D16, unroll=unroll), project(x, r, kernel=pkg.KERNEL_DIRECT)):
+        np.testing.assert_array_equal(np.isnan(a), np.isnan(b))
+        np.testing.assert_array_equal(a[np.isinf(b)], b[np.isinf(b)])
+        np.testing.assert_array_equal(np.isfinite(a), np.isfinite(b))
+    m.close()
+
+
+def test_tuned_copy_stays_private(pkg, cuda):
+    """A handle that the tuner gave a delta-coded copy of its own still reports
+    none and still refuses the kernel that needs compress_indices; its image
+    stays within the FP32 tolerance of the csr-vector kernel's."""
+    rng = np.random.default_rng(5)
+    rows, cols, n = 40_000, 50_000, 450  # 18 M nonzeros: 144 MB, more than L2
+    start = rng.integers(0, cols - 2 * n, rows)
+    col = (start[:, None] + np.arange(0, 2 * n, 2)[None, :]).astype(np.uint32).ravel()
+    rp = (np.arange(rows + 1) * n).astype(np.uint64)
+    val = rng.uniform(0.05, 1.0, col.size).astype(np.float32)
+    g = rng.poisson(50.0, rows).astype(np.int32)
+    m = pkg.Matrix.from_csr(rp, col, val, cols)
+    direct = m.run(g, 5, kernel=pkg.KERNEL_DIRECT)
+    auto = m.run(g, 5)
+    assert np.linalg.norm(auto - direct) <= 1e-5 * np.linalg.norm(direct)
+    np.testing.assert_array_equal(m.run(g, 5), auto)
+    with pytest.raises(pkg.MlemError, match="compress_indices"):
+        m.run(g, 1, kernel=pkg.KERNEL_D16)
+    info = pkg.MatrixInfo()
+    pkg.load_library().mlem_matrix_get_info(m.handle, C.byref(info))
+    assert (info.d16_slots, info.d16_slots_t, info.d16_lanes, info.d16_lanes_t) == (0, 0, 0, 0)
     m.close()
