@@ -5,10 +5,9 @@
 //
 // The merged list (row ends ∪ nonzeros) is cut into tiles whose start
 // coordinates come from the reference search.  Library matrices use
-// row-parallel tiles (k_merge_rows): a tile spans at least the stretch one
-// 1024-thread block of the reference covers (1024 * secsize items) and about
-// 32 average rows; its rows are shared out to 16-lane groups that read their
-// part of the row with 16-byte vector loads.  Caller-owned arrays (the
+// row-parallel tiles (k_merge_rows): a tile spans at least secsize items per
+// thread and about 32 average rows; its rows are shared out to 8- or 16-lane
+// groups that read their part of the row with 16-byte vector loads.  Caller-owned arrays (the
 // allocation-free entry point) use the per-thread form (k_merge_tile): thread
 // t consumes secsize items from diagonal t*secsize, the tile's products are
 // staged in shared memory and the per-thread carries are combined with a
@@ -257,63 +256,75 @@ __global__ void k_merge_fixup(const uint32_t* __restrict__ ti, const float* __re
     }
 }
 
-// Row-parallel tile: the tile is the same stretch of the merge path as above
-// (row ends and nonzeros from the reference search), but its rows are shared
-// out to the CTA's warps.  A warp sums its row's part of the tile with
-// 16-byte vector loads (the operand's arrays are padded and 16-byte aligned)
-// and a fixed xor reduction; rows that end inside the tile get their
-// epilogue here, the tile's first row (which began in an earlier tile) goes
-// to head[k] and the row still open at the tile's end to carry[k], for the
-// same fix-up kernel.  Deterministic.
+// Row-parallel tile: a stretch of the merge path (row ends and nonzeros from
+// the reference search) whose rows are shared out to the CTA's lane groups.
+// The CTA first lists the rows that have entries in the tile, 128 rows per
+// round, and writes the result of the empty ones there and then; a group sums
+// its row's part of the tile with 16-byte vector loads (the operand's arrays
+// are padded and 16-byte aligned) and a fixed xor reduction.  Rows that end
+// inside the tile get their epilogue here, the tile's first row (which began in
+// an earlier tile) goes to head[k] and the row still open at the tile's end to
+// carry[k], for the same fix-up kernel.  Deterministic.
+//
+// Why the list: a tile of empty rows (voxels that no LOR crosses, detector
+// pairs beside the grid) holds thousands of them, and taken one by one by 16
+// groups they kept one CTA busy after all others were done: the kernel's SMs
+// were active 52% of its time on the 3-D mid matrix in natural order.  Forward
+// / back projection of it 0.367 / 0.583 -> 0.352 / 0.371 ms, of an odd scanner in
+// bfloat16 0.390 / 0.193 -> 0.206 / 0.204 ms.  128 threads, so that a CTA waits
+// for fewer unlucky groups (mid, locality layout, per iteration: 0.680 ms, 256
+// threads 0.701).  Measured and not kept: warps that each stream an equal
+// stretch of nonzeros whatever their rows (0.477 / 0.652 ms: neighbouring rows
+// no longer run side by side and share fewer cache lines), cached loads of the
+// matrix (7% slower).
+constexpr uint32_t kRowsT = 128;  // threads per CTA
+
 template <typename V, int LPR, int U>
-__device__ __forceinline__ float group_part_dot(const uint32_t* __restrict__ idx, const V* __restrict__ val,
-                                                const float* __restrict__ x, uint64_t s, uint64_t t, int sub) {
-    const uint4* idx4 = reinterpret_cast<const uint4*>(idx);
-    const uint64_t v1 = (t + 3) >> 2;
+__device__ __forceinline__ float group_part_dot(const uint4* __restrict__ idx4, const V* __restrict__ val,
+                                                const float* __restrict__ x, uint32_t s, uint32_t t, int sub) {
+    // s, t: first and last entry + 1, relative to a multiple of 4 that idx4 and val start at
+    const uint32_t v1 = (t + 3) >> 2;
     float acc = 0.f;
     // U = 2: two vectors per lane in flight; the FMAs still run in the lane's
     // vector order, so the sums are those of one vector at a time
-    uint64_t v = (s >> 2) + sub;
-    if constexpr (U == 2)
-    for (; v + LPR < v1; v += 2 * LPR) {
+    uint32_t v = (s >> 2) + sub;
+    for (; U == 2 && v + LPR < v1; v += 2 * LPR) {
         const uint4 c0 = ld_stream(idx4 + v), c1 = ld_stream(idx4 + v + LPR);
         float a0[4], a1[4];
         Val4<V>::load(val, v, a0);
         Val4<V>::load(val, v + LPR, a1);
         const uint32_t cs0[4] = {c0.x, c0.y, c0.z, c0.w}, cs1[4] = {c1.x, c1.y, c1.z, c1.w};
-        // element 4v+k lies in [s, t) unless it is a masked head or tail element
-        const uint32_t lo = (uint32_t)(s > 4 * v ? s - 4 * v : 0);
-        const uint32_t hi1 = (uint32_t)(t - 4 * (v + LPR));  // the second vector starts past the head
+        const uint32_t e0 = 4 * v, e1 = 4 * (v + LPR);  // the second vector starts past the head
         float g0[4], g1[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) g0[k] = (k >= (int)lo) ? __ldg(x + cs0[k]) : 0.f;
+        for (int k = 0; k < 4; ++k) g0[k] = (e0 + k >= s) ? __ldg(x + cs0[k]) : 0.f;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) g1[k] = (k < (int)hi1) ? __ldg(x + cs1[k]) : 0.f;
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-            if (k >= (int)lo) acc = fmaf(a0[k], g0[k], acc);
+        for (int k = 0; k < 4; ++k) g1[k] = (e1 + k < t) ? __ldg(x + cs1[k]) : 0.f;
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            if (k < (int)hi1) acc = fmaf(a1[k], g1[k], acc);
+            if (e0 + k >= s) acc = fmaf(a0[k], g0[k], acc);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (e1 + k < t) acc = fmaf(a1[k], g1[k], acc);
     }
     for (; v < v1; v += LPR) {
         const uint4 c = ld_stream(idx4 + v);
         float a[4];
         Val4<V>::load(val, v, a);
         const uint32_t cs[4] = {c.x, c.y, c.z, c.w};
-        const uint32_t lo = (uint32_t)(s > 4 * v ? s - 4 * v : 0), hi = (uint32_t)(t - 4 * v);
+        const uint32_t e = 4 * v;
         float g[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) g[k] = (k >= (int)lo && k < (int)hi) ? __ldg(x + cs[k]) : 0.f;
+        for (int k = 0; k < 4; ++k) g[k] = (e + k >= s && e + k < t) ? __ldg(x + cs[k]) : 0.f;
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            if (k >= (int)lo && k < (int)hi) acc = fmaf(a[k], g[k], acc);
+            if (e + k >= s && e + k < t) acc = fmaf(a[k], g[k], acc);
     }
     return acc;
 }
 
 template <typename V, int LPR, int U>
-__global__ void __launch_bounds__(256, U == 1 ? 8 : 6)
+__global__ void __launch_bounds__(kRowsT, U == 1 ? 16 : 12)
 k_merge_rows(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ idx, const V* __restrict__ val,
              const float* __restrict__ x, uint32_t rows, const uint32_t* __restrict__ ti,
              const uint64_t* __restrict__ tj, float* __restrict__ carry, uint32_t* __restrict__ carry_row,
@@ -322,29 +333,56 @@ k_merge_rows(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ i
     const uint32_t I0 = ti[k], I1 = ti[k + 1];
     const uint64_t J0 = tj[k], J1 = tj[k + 1];
     const uint32_t nrow_l = I1 - I0;  // rows that end inside the tile
-    constexpr uint32_t NG = 256 / LPR;  // lane groups of the CTA
-    const uint32_t grp = threadIdx.x / LPR;
+    constexpr uint32_t NG = kRowsT / LPR;  // lane groups of the CTA
+    __shared__ uint32_t s_i[kRowsT], s_beg[kRowsT], s_end[kRowsT], s_cnt[kRowsT / 32];
+    const uint32_t grp = threadIdx.x / LPR, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sub = threadIdx.x & (LPR - 1);
-    const unsigned mask = LPR == 32 ? 0xffffffffu : (((1u << LPR) - 1u) << ((threadIdx.x & 31) & ~(LPR - 1)));
-    for (uint32_t i = grp; i <= nrow_l; i += NG) {
-        const uint32_t r = I0 + i;
-        float acc = 0.f;
-        if (r < rows) {
-            uint64_t s = rowptr[r], t = rowptr[r + 1];
+    const unsigned mask = LPR == 32 ? 0xffffffffu : (((1u << LPR) - 1u) << (lane & ~(LPR - 1)));
+    const uint64_t base = J0 & ~3ull;
+    const uint4* idx4 = reinterpret_cast<const uint4*>(idx + base);
+    const V* vb = val + base;
+    for (uint32_t c0 = 0; c0 <= nrow_l; c0 += kRowsT) {
+        const uint32_t i = c0 + threadIdx.x, r = I0 + i;
+        uint64_t s = J0, t = J0;
+        if (i <= nrow_l && r < rows) {
+            s = rowptr[r];
+            t = rowptr[r + 1];
             s = s < J0 ? J0 : s;
             t = t > J1 ? J1 : t;
-            if (s < t) acc = group_part_dot<V, LPR, U>(idx, val, x, s, t, sub);
         }
+        const bool keep = i <= nrow_l && (s < t || i == 0 || i == nrow_l);
+        if (i <= nrow_l && !keep) epi(r, 0.f);
+        const unsigned kept = __ballot_sync(0xffffffffu, keep);
+        if (c0) __syncthreads();  // the list of the previous rows is used up
+        if (lane == 0) s_cnt[w] = __popc(kept);
+        __syncthreads();
+        uint32_t n = 0, at = __popc(kept & ((1u << lane) - 1u));
 #pragma unroll
-        for (int o = LPR / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(mask, acc, o);
-        if (sub == 0) {
-            if (i == nrow_l) {  // still open at the tile's end (or past the last row)
-                carry[k] = acc;
-                carry_row[k] = r;
-            } else if (i == 0) {
-                head[k] = acc;  // began in an earlier tile: the fix-up adds their carries
-            } else {
-                epi(r, acc);
+        for (uint32_t q = 0; q < kRowsT / 32; ++q) {
+            if (q == w) at += n;
+            n += s_cnt[q];
+        }
+        if (keep) {
+            s_i[at] = i;
+            s_beg[at] = (uint32_t)(s - base);
+            s_end[at] = (uint32_t)((t > s ? t : s) - base);
+        }
+        __syncthreads();
+        for (uint32_t j = grp; j < n; j += NG) {
+            const uint32_t ii = s_i[j];
+            const uint32_t s0 = s_beg[j], t0 = s_end[j];
+            float acc = s0 < t0 ? group_part_dot<V, LPR, U>(idx4, vb, x, s0, t0, sub) : 0.f;
+#pragma unroll
+            for (int o = LPR / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(mask, acc, o);
+            if (sub == 0) {
+                if (ii == nrow_l) {  // still open at the tile's end (or past the last row)
+                    carry[k] = acc;
+                    carry_row[k] = I0 + ii;
+                } else if (ii == 0) {
+                    head[k] = acc;  // began in an earlier tile: the fix-up adds their carries
+                } else {
+                    epi(I0 + ii, acc);
+                }
             }
         }
     }
@@ -353,12 +391,17 @@ k_merge_rows(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ i
 template <typename V>
 void merge_launch_t(const DevCsr& op, const MergePlan& p, const float* x, const EpiDev& e,
                     L2Window win, cudaStream_t s) {
-    if (p.rows_kernel && p.rows_u == 2)
-        launch_ex(k_merge_rows<V, 16, 2>, dim3((unsigned)p.ntiles), dim3(256), 0, s, win, op.rowptr, op.idx,
+    auto rows = [&](auto kern) {
+        launch_ex(kern, dim3((unsigned)p.ntiles), dim3(kRowsT), 0, s, win, op.rowptr, op.idx,
                   static_cast<const V*>(op.val), x, op.nrows, p.tile_i, p.tile_j, p.carry, p.carry_row, p.head, e);
-    else if (p.rows_kernel)
-        launch_ex(k_merge_rows<V, 16, 1>, dim3((unsigned)p.ntiles), dim3(256), 0, s, win, op.rowptr, op.idx,
-                  static_cast<const V*>(op.val), x, op.nrows, p.tile_i, p.tile_j, p.carry, p.carry_row, p.head, e);
+    };
+    if (p.rows_kernel && p.lanes == 16) {
+        if (p.rows_u == 2) rows(k_merge_rows<V, 16, 2>);
+        else rows(k_merge_rows<V, 16, 1>);
+    } else if (p.rows_kernel) {
+        if (p.rows_u == 2) rows(k_merge_rows<V, 8, 2>);
+        else rows(k_merge_rows<V, 8, 1>);
+    }
     else
         launch_ex(k_merge_tile<V>, dim3((unsigned)p.ntiles), dim3(p.threads), p.smem, s, win,
                   op.rowptr, op.idx, static_cast<const V*>(op.val), x, op.nrows, p.secsize,
@@ -399,15 +442,20 @@ void merge_plan_build(const DevCsr& op, uint32_t secsize, MergePlan& plan, cudaS
                  "merge section size must be in 1..512");
     plan.release();
     plan.secsize = secsize;
-    // Row-parallel tiles of the merge path, 256 threads: at least the stretch
-    // one 1024-thread block of the reference covers (1024 * secsize items),
-    // and enough items for about 32 average rows so that the CTA's 8 warps
-    // share the tile's rows evenly; at most 65536 items.
+    // Row-parallel tiles of the merge path: at least secsize items per thread,
+    // and enough items for about 32 average rows so that the CTA's groups share
+    // the tile's rows evenly (fewer, down to 8, where the tiles would not fill
+    // 152 SMs x 16 CTAs: 2-D ring 19 us per iteration with 8, 33 with 32); at
+    // most 65536 items.  8 lanes take a row of a mean below 96, 16 the longer ones
+    // (mean 38: 0.080 against 0.104 ms; mean 313: 0.363 against 0.352).
     plan.rows_kernel = true;
-    plan.threads = 256;
+    plan.threads = kRowsT;
+    plan.lanes = op.nrows && op.nnz / op.nrows < 96 ? 8 : 16;
     const uint64_t items = (uint64_t)op.nrows + op.nnz;
     const uint64_t per_row = op.nrows ? (items + op.nrows - 1) / op.nrows : 1;
-    const uint64_t TS = std::min<uint64_t>(std::max<uint64_t>(1024ull * secsize, 32 * per_row), 65536ull);
+    const uint64_t rows_per_tile = std::min<uint64_t>(std::max<uint64_t>(op.nrows / (152ull * 16), 8), 32);
+    const uint64_t TS =
+        std::min<uint64_t>(std::max<uint64_t>((uint64_t)kRowsT * secsize, rows_per_tile * per_row), 65536ull);
     plan.ntiles = (items + TS - 1) / TS;
     MLEM_REQUIRE(plan.ntiles < (1ull << 31), MLEM_EUNSUPPORTED, "merge path: too many tiles");
     plan.smem = 0;

@@ -340,7 +340,7 @@ const MergePlan& merge_plan(mlem_matrix* m, bool transposed, uint32_t secsize) {
     merge_plan_build(op, secsize, p, s);
     MLEM_CUDA(cudaStreamSynchronize(s));
     if (p.rows_kernel && op.nnz) {
-        // one or two vectors per lane in flight in the row kernel (6 or 8 blocks
+        // one or two vectors per lane in flight in the row kernel (16 or 12 blocks
         // per SM), timed with a Raw epilogue on an image of ones; same sums
         float *x = nullptr, *y = nullptr;
         cudaEvent_t e0 = nullptr, e1 = nullptr;

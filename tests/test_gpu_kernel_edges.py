@@ -162,3 +162,47 @@ def test_tuned_copy_stays_private(pkg, cuda):
     pkg.load_library().mlem_matrix_get_info(m.handle, C.byref(info))
     assert (info.d16_slots, info.d16_slots_t, info.d16_lanes, info.d16_lanes_t) == (0, 0, 0, 0)
     m.close()
+
+
+@pytest.mark.parametrize("vt", [0, 1, 2])
+@pytest.mark.parametrize("secsize", [1, 5, 64, 512])
+@pytest.mark.parametrize("long_rows", [True, False])
+def test_merge_tiles_with_empty_runs(pkg, cuda, vt, secsize, long_rows):
+    """Merge-path projections of rows on both sides of the 8 / 16 lane choice, with
+    runs of empty rows longer than a tile at the start, inside and at the end, and
+    rows longer than several tiles next to them."""
+    cols = 4999
+    rng, rp, col, val = edge_csr(41, cols, False)
+    lens = np.diff(rp.astype(np.int64))
+    if not long_rows:  # many short rows bring the mean below 96
+        short = rng.integers(0, 40, 4000)
+        lens, col = np.concatenate([lens, short]), np.concatenate([col, rng.integers(0, cols, short.sum())])
+    big = np.array([30_000, 1, 200_000 if secsize < 512 else 70_000])
+    lens = np.concatenate([np.zeros(700, int), lens, np.zeros(9000, int), big, np.zeros(300, int)])
+    col = np.concatenate([col, rng.integers(0, cols, big.sum())]).astype(np.uint32)
+    if long_rows:
+        lens = lens[lens > 0]  # no empty rows at all: a mean above 96
+        lens = np.concatenate([[0], lens, [0, 0]])
+    rows = len(lens)
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.uint64)
+    val = rng.uniform(0.05, 1.0, len(col)).astype(np.float32)
+    assert (len(col) // rows >= 96) == long_rows
+    rid = np.repeat(np.arange(rows), lens)
+    v = stored(cuda, val, vt)
+    x = rng.uniform(0.5, 1.5, cols).astype(np.float32)
+    r = rng.uniform(0.5, 1.5, rows).astype(np.float32)
+    g = rng.integers(0, 50, rows).astype(np.int32)
+    m = pkg.Matrix.from_csr(rp, col, val, cols, value_type=vt)
+    dx, dr, dg = (cuda.from_numpy(a).cuda() for a in (x, r, g))
+    ratio, fp, bp = (cuda.full((n,), -1.0, device="cuda") for n in (rows, rows, cols))
+    kw = dict(spmv=pkg.SPMV_MERGE, secsize_fp=secsize, secsize_bp=secsize)
+    m.forward_project(dx.data_ptr(), dg.data_ptr(), ratio.data_ptr(), fp.data_ptr(), **kw)
+    m.back_project(dr.data_ptr(), bp.data_ptr(), **kw)
+    cuda.cuda.synchronize()
+    fp, bp, ratio = fp.cpu().numpy(), bp.cpu().numpy(), ratio.cpu().numpy()
+    want = np.bincount(rid, weights=v * x[col].astype(np.float64), minlength=rows)
+    assert np.all(np.abs(fp - want) <= (lens + 2) * 2.0**-24 * want)
+    np.testing.assert_array_equal(ratio, np.where(fp != 0, g.astype(np.float32) / np.where(fp != 0, fp, 1), 0))
+    want = np.bincount(col, weights=v * r[rid].astype(np.float64), minlength=cols)
+    assert np.all(np.abs(bp - want) <= (np.bincount(col, minlength=cols) + 2) * 2.0**-24 * want)
+    m.close()
