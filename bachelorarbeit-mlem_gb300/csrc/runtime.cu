@@ -166,6 +166,10 @@ static bool permuted(const mlem_matrix* m) { return m->lor_of || m->vox_of; }
 int scatter_lanes(mlem_matrix* m) {
     if (m->scatter_lanes) return m->scatter_lanes;
     const DevCsr& A = m->A;
+    if (m->one_call) {  // not worth timing: the pick is the fastest on the 3-D matrices measured
+        m->scatter_unroll = 4;
+        return m->scatter_lanes = std::max(8, pick_lanes(A.nnz, A.nrows));
+    }
     cudaStream_t s = m->stream;
     float *r = nullptr, *bp = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -476,17 +480,26 @@ static bool may_copy_d16(const mlem_matrix* m, const DevCsr& op) {
     return stream > (uint64_t)l2 && copy <= avail / 4;
 }
 
-// Times every candidate configuration on the operand itself (Raw epilogue
-// into a scratch vector, x = 1) and keeps the fastest.  Runs once per
-// operand, outside any stream capture.
+// Times the candidate configurations on the operand itself (Raw epilogue into
+// a scratch vector, constant x) and keeps the fastest.  A candidate that its
+// first launch shows to be a quarter slower than the best so far gets no
+// further ones.  Runs once per operand, outside any stream capture.  A handle
+// made for one call tries the plain kernel with three lane counts only: the
+// other forms are within a few percent of it, and timing them all takes longer
+// than 100 iterations (30 M nonzeros: 12.2 ms for both operands; 1.0 ms so).
 static void tune_projection(mlem_matrix* m, bool transposed) {
     if (m->tuned[transposed]) return;
     DevCsr& op = transposed ? m->AT : m->A;
     cudaStream_t s = m->stream;
     std::vector<ProjCfg> cand;
     const int base = pick_lanes(op.nnz, op.nrows);
+    const bool brief = m->one_call != 0;
     for (int lanes : {base / 2, base, base * 2})
         if (lanes >= 4 && lanes <= 32) {
+            if (brief) {
+                cand.push_back(ProjCfg{MLEM_KERNEL_DIRECT, lanes, 2, 0.f, false, false});
+                continue;
+            }
             for (int u : {1, 2, 4}) cand.push_back(ProjCfg{MLEM_KERNEL_DIRECT, lanes, u, 0.f, false, false});
             if (lanes >= 16)
                 for (int u : {1, 2})
@@ -495,16 +508,18 @@ static void tune_projection(mlem_matrix* m, bool transposed) {
                             if ((ord || pipe) && (!ord || op.order))
                                 cand.push_back(ProjCfg{MLEM_KERNEL_DIRECT, lanes, u, 0.f, ord, pipe});
         }
-    if (base >= 16) cand.push_back(ProjCfg{MLEM_KERNEL_PERSISTENT, base, 1, 0.f, false, false});
-    cand.push_back(ProjCfg{MLEM_KERNEL_TMA, 32, 2, 0.f});
-    if (op.d16) d16_cands(op, cand);
-    if (op.idx_ilv)
-        for (int u : {1, 2, 4}) cand.push_back(ProjCfg{MLEM_KERNEL_ILV, 32, u, 0.f});
-    if (m->sym.fp_rowptr)
-        for (int u : {2, 4, 8})
-            for (bool grouped : {false, true}) cand.push_back(ProjCfg{MLEM_KERNEL_SYM, 32, u, 0.f, grouped, false});
-    prepare_csrvec_pipe(op.vt);
-    prepare_csr_tma(op.vt);
+    if (!brief) {
+        if (base >= 16) cand.push_back(ProjCfg{MLEM_KERNEL_PERSISTENT, base, 1, 0.f, false, false});
+        cand.push_back(ProjCfg{MLEM_KERNEL_TMA, 32, 2, 0.f});
+        if (op.d16) d16_cands(op, cand);
+        if (op.idx_ilv)
+            for (int u : {1, 2, 4}) cand.push_back(ProjCfg{MLEM_KERNEL_ILV, 32, u, 0.f});
+        if (m->sym.fp_rowptr)
+            for (int u : {2, 4, 8})
+                for (bool grouped : {false, true}) cand.push_back(ProjCfg{MLEM_KERNEL_SYM, 32, u, 0.f, grouped, false});
+        prepare_csrvec_pipe(op.vt);
+        prepare_csr_tma(op.vt);
+    }
     ensure_workspace(m);
     float *x = nullptr, *y = nullptr;
     MLEM_CUDA(cudaMalloc(&x, sizeof(float) * std::max<uint32_t>(op.ncols, 1)));
@@ -515,21 +530,25 @@ static void tune_projection(mlem_matrix* m, bool transposed) {
     ProjCfg best;
     best.ms = 1e30f;
     try {
-        std::vector<float> ones(std::max<uint32_t>(op.ncols, 1), 1.0f);
-        MLEM_CUDA(cudaMemcpyAsync(x, ones.data(), sizeof(float) * ones.size(), cudaMemcpyHostToDevice, s));
+        // every byte 0x3f: x = 0.747
+        MLEM_CUDA(cudaMemsetAsync(x, 0x3f, sizeof(float) * std::max<uint32_t>(op.ncols, 1), s));
         EpiArgs e;
         e.kind = Epi::Raw;
         e.out = y;
-        const int reps = op.nnz > (50ull << 20) ? 2 : 4;
-        auto time = [&](ProjCfg& c) {
-            launch_cfg(m, op, x, e, c, {}, s);  // warm-up
+        const int reps = brief ? 1 : op.nnz > (50ull << 20) ? 2 : op.nnz > (4ull << 20) ? 4 : 16;
+        auto launches = [&](const ProjCfg& c, int n) {  // milliseconds of one launch, the mean of n
             MLEM_CUDA(cudaEventRecord(e0, s));
-            for (int r = 0; r < reps; ++r) launch_cfg(m, op, x, e, c, {}, s);
+            for (int r = 0; r < n; ++r) launch_cfg(m, op, x, e, c, {}, s);
             MLEM_CUDA(cudaEventRecord(e1, s));
             MLEM_CUDA(cudaEventSynchronize(e1));
             float ms = 0.f;
             MLEM_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-            c.ms = ms / reps;
+            return ms / n;
+        };
+        auto time = [&](ProjCfg& c) {
+            launch_cfg(m, op, x, e, c, {}, s);  // warm-up
+            c.ms = launches(c, 1);
+            if (reps > 1 && c.ms < 1.25f * best.ms) c.ms = launches(c, reps);
             if (c.ms < best.ms) best = c;
         };
         for (ProjCfg& c : cand) time(c);
@@ -879,7 +898,10 @@ static void postprocess_matrix(mlem_matrix* m, const mlem_matrix_opts& o) {
         if (m->has_t) build_ilv(m->AT, s);
     }
     MLEM_CUDA(cudaMalloc(&m->norm, sizeof(float) * std::max<uint32_t>(A.ncols, 1)));
-    m->norm_host.resize(A.ncols);
+    // the host copy and its running sum serve the getter and the reference
+    // initial value; a handle made for one call is given its image and norm
+    const bool host_norm = !m->one_call;
+    if (host_norm) m->norm_host.resize(A.ncols);
     if (o.norm) {
         // given in natural column order
         if (m->vox_of && A.ncols) {
@@ -892,7 +914,7 @@ static void postprocess_matrix(mlem_matrix* m, const mlem_matrix_opts& o) {
         } else {
             MLEM_CUDA(cudaMemcpyAsync(m->norm, o.norm, sizeof(float) * A.ncols, cudaMemcpyHostToDevice, s));
         }
-        std::copy(o.norm, o.norm + A.ncols, m->norm_host.begin());
+        if (host_norm) std::copy(o.norm, o.norm + A.ncols, m->norm_host.begin());
     } else {
         if (m->has_t) colsum_from_transpose(m->AT, m->norm, s);
         else colsum_scatter(A, m->norm, s);
@@ -1101,6 +1123,46 @@ void mlem_run_opts_default(mlem_run_opts* o) {
     o->loglik_rel_tol = 0.0;
 }
 
+namespace mlem {
+// one_call: iterations of the only run the handle is made for (0: a caller's
+// handle); it must come with its sensitivity image.
+static mlem_matrix* create_matrix(const mlem_csr_host* csr, const mlem_matrix_opts& o, uint32_t one_call) {
+    check_host_csr(csr);
+    DeviceGuard dg(o.device);
+    mlem_matrix* m = new_matrix(o);
+    m->one_call = one_call;
+    try {
+        upload_csr(csr, m->A, m->stream);
+        if (o.symmetry) {
+            MLEM_REQUIRE(o.layout == MLEM_LAYOUT_NATURAL, MLEM_EUNSUPPORTED,
+                         "symmetry keeps the natural layout (the symmetric operands are compact already)");
+            MLEM_REQUIRE(o.grid_nx == o.grid_ny, MLEM_EUNSUPPORTED, "symmetry needs a square voxel grid");
+            DevCsr hat;
+            try {
+                build_symmetric_checked(*csr, m->A, o.grid_nx, o.grid_nz, o.sym_det_per_ring, o.sym_rings, hat,
+                                        m->AT, m->sym, m->stream);
+            } catch (...) {
+                free_csr(hat);
+                throw;
+            }
+            free_csr(hat);  // equal to the caller's matrix, which stays
+            m->has_t = true;
+            postprocess_matrix(m, o);
+            lower_symmetric_values(m->sym, o.value_type, m->stream);
+            sym_set_norm(m->sym, m->norm, m->stream);
+            MLEM_CUDA(cudaStreamSynchronize(m->stream));
+        } else {
+            maybe_apply_layout(m, o, o.grid_nx, o.grid_ny, o.grid_nz, {});
+            postprocess_matrix(m, o);
+        }
+    } catch (...) {
+        destroy_matrix(m);
+        throw;
+    }
+    return m;
+}
+}  // namespace mlem
+
 mlem_status mlem_matrix_create(const mlem_csr_host* csr, const mlem_matrix_opts* opts, mlem_matrix** out) {
     return guarded([&] {
         MLEM_REQUIRE(out != nullptr, MLEM_EINVAL, "out is NULL");
@@ -1108,38 +1170,7 @@ mlem_status mlem_matrix_create(const mlem_csr_host* csr, const mlem_matrix_opts*
         mlem_matrix_opts o;
         mlem_matrix_opts_default(&o);
         if (opts) o = *opts;
-        check_host_csr(csr);
-        DeviceGuard dg(o.device);
-        mlem_matrix* m = new_matrix(o);
-        try {
-            upload_csr(csr, m->A, m->stream);
-            if (o.symmetry) {
-                MLEM_REQUIRE(o.layout == MLEM_LAYOUT_NATURAL, MLEM_EUNSUPPORTED,
-                             "symmetry keeps the natural layout (the symmetric operands are compact already)");
-                MLEM_REQUIRE(o.grid_nx == o.grid_ny, MLEM_EUNSUPPORTED, "symmetry needs a square voxel grid");
-                DevCsr hat;
-                try {
-                    build_symmetric_checked(*csr, m->A, o.grid_nx, o.grid_nz, o.sym_det_per_ring, o.sym_rings, hat,
-                                            m->AT, m->sym, m->stream);
-                } catch (...) {
-                    free_csr(hat);
-                    throw;
-                }
-                free_csr(hat);  // equal to the caller's matrix, which stays
-                m->has_t = true;
-                postprocess_matrix(m, o);
-                lower_symmetric_values(m->sym, o.value_type, m->stream);
-                sym_set_norm(m->sym, m->norm, m->stream);
-                MLEM_CUDA(cudaStreamSynchronize(m->stream));
-            } else {
-                maybe_apply_layout(m, o, o.grid_nx, o.grid_ny, o.grid_nz, {});
-                postprocess_matrix(m, o);
-            }
-        } catch (...) {
-            destroy_matrix(m);
-            throw;
-        }
-        *out = m;
+        *out = create_matrix(csr, o, 0);
     });
 }
 
@@ -1655,10 +1686,7 @@ mlem_status mlem_reconstruct(const uint64_t* csr_rows, const uint32_t* csr_cols,
         mo.norm = norm;
         const bool host_t = using_trans == 0 && csr_rows_trans && (nnzs == 0 || (csr_cols_trans && csr_vals_trans));
         mo.build_transpose = (using_trans == 0 && !host_t) ? 1 : 0;
-        mlem_matrix* m = nullptr;
-        mlem_status st = mlem_matrix_create(&c, &mo, &m);
-        if (st != MLEM_OK) fail(st, get_error());
-        m->one_call = iterations;
+        mlem_matrix* m = create_matrix(&c, mo, std::max<uint32_t>(iterations, 1));
         try {
             if (host_t) {
                 // the caller supplied Aᵀ (as main.cu:100-105 does): upload it as is
@@ -1675,7 +1703,10 @@ mlem_status mlem_reconstruct(const uint64_t* csr_rows, const uint32_t* csr_cols,
             o.bp_mode = using_trans ? MLEM_BP_SCATTER : MLEM_BP_TRANS;
             o.secsize_fp = secsize_fp;
             o.secsize_bp = secsize_bp;
-            st = mlem_run(m, g, f, iterations, &o, result_f, nullptr, nullptr);
+            // two graphs (8 iterations and 1) cost 0.8 ms to capture and
+            // instantiate, an eagerly launched iteration 6 us of host time
+            o.use_graph = iterations >= 200;
+            const mlem_status st = mlem_run(m, g, f, iterations, &o, result_f, nullptr, nullptr);
             if (st != MLEM_OK) fail(st, get_error());
         } catch (...) {
             destroy_matrix(m);
