@@ -73,6 +73,28 @@ __device__ __forceinline__ uint4 ld_stream_u4(const uint4* p) { return __ldcs(p)
 __device__ __forceinline__ uint2 ld_stream_u2(const uint2* p) { return __ldcs(p); }
 __device__ __forceinline__ float4 ld_stream_f4(const float4* p) { return __ldcs(p); }
 
+// Programmatic dependent launch (EpiArgs::overlap): a kernel launched so may
+// start while its predecessor in the stream drains.  Before grid_wait it
+// touches nothing but arrays that no kernel of a run writes (the operand's row
+// offsets, indices and values); after it, everything the predecessors wrote is
+// visible.  Every block of such a kernel calls grid_wait, so that a grid never
+// ends before its predecessor.  Vectors that a predecessor may have written
+// are read with ld_after (a plain load: the read-only path, ld.global.nc, is
+// for data that is constant for the kernel's whole lifetime, which begins
+// before the wait).
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ float ld_after(const float* p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ int32_t ld_after(const int32_t* p) {
+    int32_t v;
+    asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+
 __device__ __forceinline__ uint64_t globaltimer_ns() {
     uint64_t t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));

@@ -30,6 +30,12 @@ struct EpiArgs {
     float* fwproj = nullptr;      // Correl: optional copy of the projection
     float* f = nullptr;           // Update: image, updated in place
     const float* norm = nullptr;  // Update
+    // csr-vector (DIRECT) and D16 kernels: launched so that they may start while
+    // the previous kernel of the stream drains.  Set inside an MLEM loop: 8.15 ->
+    // 7.34 us per iteration on the 2-D ring, 43.9 -> 43.2 us with 6 M nonzeros,
+    // 4.26 -> 4.20 ms on the 3-D mid matrix; a single projection only pays for the
+    // attribute (0.4 us of host time).
+    bool overlap = false;
     // symmetry-compressed kernels only: also write the results in orbit
     // order (Correl: ratio into SymOps::orb_r; Update: image into orb_x), and
     // take the input's orbit array as current instead of gathering it
@@ -346,28 +352,40 @@ extern size_t g_max_window_bytes;
 
 // Launch through cudaLaunchKernelEx so the L2 access-policy window travels
 // with the launch (and into a CUDA graph node when captured).
+// overlap: for kernels that call grid_wait (common.cuh), which may then start
+// before their predecessor in the stream has ended.
 template <typename... KArgs, typename... Args>
-inline void launch_ex(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                      cudaStream_t s, L2Window win, Args... args) {
+inline void launch_attrs(bool overlap, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                         cudaStream_t s, L2Window win, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     unsigned n = 0;
     if (win.bytes && g_max_window_bytes) {
-        attr[0].id = cudaLaunchAttributeAccessPolicyWindow;
-        attr[0].val.accessPolicyWindow.base_ptr = const_cast<void*>(win.ptr);
-        attr[0].val.accessPolicyWindow.num_bytes = win.bytes < g_max_window_bytes ? win.bytes : g_max_window_bytes;
-        attr[0].val.accessPolicyWindow.hitRatio = 1.0f;
-        attr[0].val.accessPolicyWindow.hitProp = cudaAccessPropertyPersisting;
-        attr[0].val.accessPolicyWindow.missProp = cudaAccessPropertyStreaming;
-        n = 1;
+        attr[n].id = cudaLaunchAttributeAccessPolicyWindow;
+        attr[n].val.accessPolicyWindow.base_ptr = const_cast<void*>(win.ptr);
+        attr[n].val.accessPolicyWindow.num_bytes = win.bytes < g_max_window_bytes ? win.bytes : g_max_window_bytes;
+        attr[n].val.accessPolicyWindow.hitRatio = 1.0f;
+        attr[n].val.accessPolicyWindow.hitProp = cudaAccessPropertyPersisting;
+        attr[n].val.accessPolicyWindow.missProp = cudaAccessPropertyStreaming;
+        ++n;
+    }
+    if (overlap) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n].val.programmaticStreamSerializationAllowed = 1;
+        ++n;
     }
     cfg.attrs = attr;
     cfg.numAttrs = n;
     MLEM_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...));
     count_launch();
+}
+template <typename... KArgs, typename... Args>
+inline void launch_ex(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, L2Window win,
+                      Args... args) {
+    launch_attrs(false, kernel, grid, block, smem, s, win, args...);
 }
 }  // namespace mlem

@@ -483,7 +483,7 @@ static bool may_copy_d16(const mlem_matrix* m, const DevCsr& op) {
 // Times the candidate configurations on the operand itself (Raw epilogue into
 // a scratch vector, constant x) and keeps the fastest.  A candidate that its
 // first launch shows to be a quarter slower than the best so far gets no
-// further ones.  Runs once per operand, outside any stream capture.  A handle
+// further ones; short kernels are timed from a graph.  Runs once per operand, outside any stream capture.  A handle
 // made for one call tries the plain kernel with three lane counts only: the
 // other forms are within a few percent of it, and timing them all takes longer
 // than 100 iterations (30 M nonzeros: 12.2 ms for both operands; 1.0 ms so).
@@ -535,7 +535,8 @@ static void tune_projection(mlem_matrix* m, bool transposed) {
         EpiArgs e;
         e.kind = Epi::Raw;
         e.out = y;
-        const int reps = brief ? 1 : op.nnz > (50ull << 20) ? 2 : op.nnz > (4ull << 20) ? 4 : 16;
+        const int reps = brief ? 1 : op.nnz > (50ull << 20) ? 2 : 4;
+        constexpr uint64_t kShort = 4ull << 20;  // nonzeros; a projection of fewer takes under 10 us
         auto launches = [&](const ProjCfg& c, int n) {  // milliseconds of one launch, the mean of n
             MLEM_CUDA(cudaEventRecord(e0, s));
             for (int r = 0; r < n; ++r) launch_cfg(m, op, x, e, c, {}, s);
@@ -545,10 +546,46 @@ static void tune_projection(mlem_matrix* m, bool transposed) {
             MLEM_CUDA(cudaEventElapsedTime(&ms, e0, e1));
             return ms / n;
         };
+        // the same from a graph, as the MLEM loop replays it: launched one by one,
+        // kernels of a few microseconds all take the launch rate's 6
+        auto replayed = [&](const ProjCfg& c, int n) {
+            cudaGraph_t graph = nullptr;
+            cudaGraphExec_t exec = nullptr;
+            const uint64_t l0 = g_launches.load();
+            MLEM_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+            try {
+                EpiArgs ov = e;
+                ov.overlap = true;
+                for (int r = 0; r < n; ++r) launch_cfg(m, op, x, ov, c, {}, s);
+            } catch (...) {
+                cudaStreamEndCapture(s, &graph);
+                if (graph) cudaGraphDestroy(graph);
+                throw;
+            }
+            MLEM_CUDA(cudaStreamEndCapture(s, &graph));
+            g_launches.fetch_sub(g_launches.load() - l0);
+            const cudaError_t made = cudaGraphInstantiate(&exec, graph, 0);
+            cudaGraphDestroy(graph);
+            MLEM_CUDA(made);
+            float ms = 0.f;
+            cudaError_t err = cudaSuccess;
+            for (int r = 0; r < 3 && err == cudaSuccess; ++r) {  // the first two warm up
+                cudaEventRecord(e0, s);
+                err = cudaGraphLaunch(exec, s);
+                cudaEventRecord(e1, s);
+                if (err == cudaSuccess) err = cudaEventSynchronize(e1);
+            }
+            if (err == cudaSuccess) err = cudaEventElapsedTime(&ms, e0, e1);
+            cudaGraphExecDestroy(exec);
+            MLEM_CUDA(err);
+            count_launch(3 * n);
+            return ms / n;
+        };
         auto time = [&](ProjCfg& c) {
             launch_cfg(m, op, x, e, c, {}, s);  // warm-up
             c.ms = launches(c, 1);
-            if (reps > 1 && c.ms < 1.25f * best.ms) c.ms = launches(c, reps);
+            if (!brief && op.nnz <= kShort) c.ms = replayed(c, 16);
+            else if (reps > 1 && c.ms < 1.25f * best.ms) c.ms = launches(c, reps);
             if (c.ms < best.ms) best = c;
         };
         for (ProjCfg& c : cand) time(c);
@@ -707,6 +744,7 @@ void enqueue_iteration(mlem_matrix* m, const mlem_run_opts& o, cudaStream_t s, d
     } else {
         EpiArgs fe;
         fe.kind = Epi::Correl;
+        fe.overlap = true;
         fe.g = w.g;
         fe.out = w.ratio;
         fe.fwproj = want_ll ? w.fwproj : nullptr;
@@ -724,6 +762,7 @@ void enqueue_iteration(mlem_matrix* m, const mlem_run_opts& o, cudaStream_t s, d
         if (o.bp_mode == MLEM_BP_TRANS) {
             EpiArgs be;
             be.kind = Epi::Update;
+            be.overlap = true;
             be.f = w.f;
             be.norm = m->norm;
             if (sym_fused) {
@@ -812,7 +851,10 @@ static uint32_t run_iterations(mlem_matrix* m, const mlem_run_opts& o, uint32_t 
         }
         return iters;
     }
-    constexpr uint32_t kChunk = 8;
+    // 32 iterations per graph and one graph of what is left (at most 32 graphs
+    // per set of options): 50 iterations of the 2-D ring take two launches; as
+    // six graphs of 8 and two of 1 they took 3% longer
+    constexpr uint32_t kChunk = 32;
     auto get_graph = [&](uint32_t chunk) -> cudaGraphExec_t {
         RunKey key{(int)o.spmv, (int)o.bp_mode, (int)o.secsize_fp, (int)o.secsize_bp, (int)o.l2_window,
                    (int)chunk, (int)(o.kernel | o.lanes << 8 | o.unroll << 16 | o.row_order << 24 | o.pipeline << 25)};
@@ -861,7 +903,7 @@ static uint32_t run_iterations(mlem_matrix* m, const mlem_run_opts& o, uint32_t 
         }
     };
     if (full) replay(kChunk, full);
-    if (rest) replay(1, rest);
+    if (rest) replay(rest, 1);
     return iters;
 }
 
@@ -1703,8 +1745,8 @@ mlem_status mlem_reconstruct(const uint64_t* csr_rows, const uint32_t* csr_cols,
             o.bp_mode = using_trans ? MLEM_BP_SCATTER : MLEM_BP_TRANS;
             o.secsize_fp = secsize_fp;
             o.secsize_bp = secsize_bp;
-            // two graphs (8 iterations and 1) cost 0.8 ms to capture and
-            // instantiate, an eagerly launched iteration 6 us of host time
+            // graphs of 32 iterations cost 0.8 ms to capture and instantiate,
+            // an eagerly launched iteration 6 us of host time
             o.use_graph = iterations >= 200;
             const mlem_status st = mlem_run(m, g, f, iterations, &o, result_f, nullptr, nullptr);
             if (st != MLEM_OK) fail(st, get_error());

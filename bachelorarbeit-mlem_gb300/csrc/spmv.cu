@@ -37,13 +37,20 @@ struct Vec4 {
     }
 };
 
+// AFTER: the kernel may be launched ahead of its predecessor's end (common.cuh).
+template <bool AFTER>
+__device__ __forceinline__ float load_x(const float* p) {
+    return AFTER ? ld_after(p) : __ldg(p);
+}
+
 // Gathers for one 4-element vector (masked), then the FMAs in element order.
+template <bool AFTER = false>
 __device__ __forceinline__ void gather4(const uint4& c, uint64_t base, uint64_t s, uint64_t t,
                                         const float* __restrict__ x, float g[4]) {
-    g[0] = in_row(base + 0, s, t) ? __ldg(x + c.x) : 0.f;
-    g[1] = in_row(base + 1, s, t) ? __ldg(x + c.y) : 0.f;
-    g[2] = in_row(base + 2, s, t) ? __ldg(x + c.z) : 0.f;
-    g[3] = in_row(base + 3, s, t) ? __ldg(x + c.w) : 0.f;
+    g[0] = in_row(base + 0, s, t) ? load_x<AFTER>(x + c.x) : 0.f;
+    g[1] = in_row(base + 1, s, t) ? load_x<AFTER>(x + c.y) : 0.f;
+    g[2] = in_row(base + 2, s, t) ? load_x<AFTER>(x + c.z) : 0.f;
+    g[3] = in_row(base + 3, s, t) ? load_x<AFTER>(x + c.w) : 0.f;
 }
 
 __device__ __forceinline__ float fma4(float acc, const float a[4], const float g[4], uint64_t base,
@@ -56,7 +63,7 @@ __device__ __forceinline__ float fma4(float acc, const float a[4], const float g
 
 // Dot product of row [s, t) with x by one lane of an LPR-lane group; U
 // vectors of 4 elements are loaded before their gathers are consumed.
-template <typename V, int LPR, int U = 2>
+template <typename V, int LPR, int U = 2, bool AFTER = false>
 __device__ __forceinline__ float lane_dot(const uint32_t* __restrict__ idx, const V* __restrict__ val,
                                           const float* __restrict__ x, uint64_t s, uint64_t t, int sub) {
     const uint4* idx4 = reinterpret_cast<const uint4*>(idx);
@@ -69,7 +76,7 @@ __device__ __forceinline__ float lane_dot(const uint32_t* __restrict__ idx, cons
         for (int q = 0; q < U; ++q) p[q].load(idx4, val, v + q * LPR);
         float gq[U][4];
 #pragma unroll
-        for (int q = 0; q < U; ++q) gather4(p[q].c, (v + q * LPR) << 2, s, t, x, gq[q]);
+        for (int q = 0; q < U; ++q) gather4<AFTER>(p[q].c, (v + q * LPR) << 2, s, t, x, gq[q]);
 #pragma unroll
         for (int q = 0; q < U; ++q) acc = fma4(acc, p[q].a, gq[q], (v + q * LPR) << 2, s, t);
     }
@@ -77,7 +84,7 @@ __device__ __forceinline__ float lane_dot(const uint32_t* __restrict__ idx, cons
         Vec4<V> p;
         p.load(idx4, val, v);
         float gp[4];
-        gather4(p.c, v << 2, s, t, x, gp);
+        gather4<AFTER>(p.c, v << 2, s, t, x, gp);
         acc = fma4(acc, p.a, gp, v << 2, s, t);
     }
     return acc;
@@ -97,7 +104,7 @@ __device__ __forceinline__ void load_step(Vec4<V> (&p)[U], const uint4* __restri
 // loaded before the gathers of the current step, so the index/value stream
 // stays in flight while the gathers wait.  Same per-lane order of additions
 // as lane_dot (bit-identical results).
-template <typename V, int LPR, int U>
+template <typename V, int LPR, int U, bool AFTER = false>
 __device__ __forceinline__ float lane_dot_pipe(const uint32_t* __restrict__ idx, const V* __restrict__ val,
                                                const float* __restrict__ x, uint64_t s, uint64_t t, int sub) {
     const uint4* idx4 = reinterpret_cast<const uint4*>(idx);
@@ -114,7 +121,7 @@ __device__ __forceinline__ float lane_dot_pipe(const uint32_t* __restrict__ idx,
 #pragma unroll
         for (int q = 0; q < U; ++q) {
             const uint64_t v = b + sub + (uint64_t)q * LPR;
-            if (v < v1) gather4(cur[q].c, v << 2, s, t, x, gq[q]);
+            if (v < v1) gather4<AFTER>(cur[q].c, v << 2, s, t, x, gq[q]);
         }
 #pragma unroll
         for (int q = 0; q < U; ++q) {
@@ -137,19 +144,17 @@ __device__ __forceinline__ float group_sum(float acc) {
 }
 
 // Epilogues (executed by the group leader only).
-__device__ __forceinline__ void epi_correl(uint32_t r, float sum, const int32_t* __restrict__ g,
-                                           float* __restrict__ ratio, float* __restrict__ fwproj) {
+__device__ __forceinline__ void epi_correl(uint32_t r, float sum, int32_t g, float* __restrict__ ratio,
+                                           float* __restrict__ fwproj) {
     // calcCorrel (kernel.cu:17-18): ratio stays 0 where the projection is 0.
-    ratio[r] = (sum != 0.0f) ? __fdiv_rn((float)g[r], sum) : 0.0f;
+    ratio[r] = (sum != 0.0f) ? __fdiv_rn((float)g, sum) : 0.0f;
     if (fwproj) fwproj[r] = sum;
 }
 
-__device__ __forceinline__ void epi_update(uint32_t c, float sum, float* __restrict__ f,
-                                           const float* __restrict__ norm) {
+__device__ __forceinline__ float epi_update(float f, float sum, float n) {
     // calcUpdate (kernel.cu:34-37): f * bp / norm, evaluated left to right.
-    const float t = __fmul_rn(f[c], sum);
-    const float n = norm[c];
-    f[c] = (n == 0.0f) ? t : __fdiv_rn(t, n);
+    const float t = __fmul_rn(f, sum);
+    return (n == 0.0f) ? t : __fdiv_rn(t, n);
 }
 
 template <typename V, int LPR, int EPI, int U, bool ORD, bool PIPE>
@@ -161,17 +166,23 @@ k_csrvec(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ idx,
     const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t k = gt / LPR;
     const int sub = threadIdx.x & (LPR - 1);
+    grid_release();
     float acc = 0.f;
     uint32_t row = k;
+    uint64_t s = 0, t = 0;
     if (k < nrows) {
         if (ORD) row = __ldg(order + k);
-        const uint64_t s = rowptr[row], t = rowptr[row + 1];
-        acc = PIPE ? lane_dot_pipe<V, LPR, U>(idx, val, x, s, t, sub) : lane_dot<V, LPR, U>(idx, val, x, s, t, sub);
+        s = rowptr[row];
+        t = rowptr[row + 1];
     }
+    grid_wait();
+    if (k < nrows)
+        acc = PIPE ? lane_dot_pipe<V, LPR, U, true>(idx, val, x, s, t, sub)
+                   : lane_dot<V, LPR, U, true>(idx, val, x, s, t, sub);
     acc = group_sum<LPR>(acc);
     if (sub == 0 && k < nrows) {
-        if (EPI == (int)Epi::Correl) epi_correl(row, acc, g, out, fwproj);
-        else if (EPI == (int)Epi::Update) epi_update(row, acc, f, norm);
+        if (EPI == (int)Epi::Correl) epi_correl(row, acc, ld_after(g + row), out, fwproj);
+        else if (EPI == (int)Epi::Update) f[row] = epi_update(ld_after(f + row), acc, norm[row]);
         else out[row] = acc;
     }
 }
@@ -239,8 +250,8 @@ k_csrvec_pipe(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ 
         if (last) {
             acc = group_sum_masked<LPR>(acc, mask);
             if (sub == 0) {
-                if (EPI == (int)Epi::Correl) epi_correl(row, acc, g, out, fwproj);
-                else if (EPI == (int)Epi::Update) epi_update(row, acc, f, norm);
+                if (EPI == (int)Epi::Correl) epi_correl(row, acc, g[row], out, fwproj);
+                else if (EPI == (int)Epi::Update) f[row] = epi_update(f[row], acc, norm[row]);
                 else out[row] = acc;
             }
             acc = 0.f;
@@ -424,18 +435,12 @@ k_fused_rescan(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__
     scatter_row<V, LPR, 4>(idx, val, s, t, sub, r, bp);
 }
 
-// calcUpdate (kernel.cu:34-37) for the scatter forms: f * bp / norm, left to right.
-__device__ __forceinline__ float update_one(float f, float b, float nn) {
-    const float t = __fmul_rn(f, b);
-    return (nn == 0.0f) ? t : __fdiv_rn(t, nn);
-}
-
 __global__ void k_update_zero(float* __restrict__ f, float* __restrict__ bp,
                               const float* __restrict__ norm, uint32_t n) {
     for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
         const float b = bp[c];
         bp[c] = 0.0f;
-        f[c] = update_one(f[c], b, norm[c]);
+        f[c] = epi_update(f[c], b, norm[c]);
     }
 }
 
@@ -452,14 +457,14 @@ __global__ void k_update_zero4(float* __restrict__ f, float* __restrict__ bp, co
         const float4 x = f4[c];
         const float4 nn = __ldg(m4 + c);
         b4[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-        f4[c] = make_float4(update_one(x.x, b.x, nn.x), update_one(x.y, b.y, nn.y), update_one(x.z, b.z, nn.z),
-                            update_one(x.w, b.w, nn.w));
+        f4[c] = make_float4(epi_update(x.x, b.x, nn.x), epi_update(x.y, b.y, nn.y), epi_update(x.z, b.z, nn.z),
+                            epi_update(x.w, b.w, nn.w));
     }
     if (blockIdx.x == 0 && threadIdx.x < (n & 3u)) {
         const uint32_t c = (n4 << 2) + threadIdx.x;
         const float b = bp[c];
         bp[c] = 0.0f;
-        f[c] = update_one(f[c], b, norm[c]);
+        f[c] = epi_update(f[c], b, norm[c]);
     }
 }
 
@@ -506,17 +511,17 @@ void csrvec_dispatch_epi(const DevCsr& op, const float* x, const EpiArgs& e, L2W
     const uint32_t* ord = op.order;
     switch (e.kind) {
         case Epi::Correl:
-            launch_ex(k_csrvec<V, LPR, (int)Epi::Correl, U, ORD, PIPE>, grid, block, 0, s, win, op.rowptr, op.idx,
-                      val, x, op.nrows, e.g, e.out, e.fwproj, (float*)nullptr, (const float*)nullptr, ord);
+            launch_attrs(e.overlap, k_csrvec<V, LPR, (int)Epi::Correl, U, ORD, PIPE>, grid, block, 0, s, win,
+                         op.rowptr, op.idx, val, x, op.nrows, e.g, e.out, e.fwproj, (float*)nullptr, (const float*)nullptr, ord);
             break;
         case Epi::Update:
-            launch_ex(k_csrvec<V, LPR, (int)Epi::Update, U, ORD, PIPE>, grid, block, 0, s, win, op.rowptr, op.idx,
-                      val, x, op.nrows, (const int32_t*)nullptr, (float*)nullptr, (float*)nullptr,
+            launch_attrs(e.overlap, k_csrvec<V, LPR, (int)Epi::Update, U, ORD, PIPE>, grid, block, 0, s, win,
+                         op.rowptr, op.idx, val, x, op.nrows, (const int32_t*)nullptr, (float*)nullptr, (float*)nullptr,
                       e.f, e.norm, ord);
             break;
         default:
-            launch_ex(k_csrvec<V, LPR, (int)Epi::Raw, U, ORD, PIPE>, grid, block, 0, s, win, op.rowptr, op.idx,
-                      val, x, op.nrows, (const int32_t*)nullptr, e.out, (float*)nullptr,
+            launch_attrs(e.overlap, k_csrvec<V, LPR, (int)Epi::Raw, U, ORD, PIPE>, grid, block, 0, s, win,
+                         op.rowptr, op.idx, val, x, op.nrows, (const int32_t*)nullptr, e.out, (float*)nullptr,
                       (float*)nullptr, (const float*)nullptr, ord);
     }
 }

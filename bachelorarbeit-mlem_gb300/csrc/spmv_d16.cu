@@ -101,7 +101,7 @@ __device__ __noinline__ float d16_row_real(const uint64_t* __restrict__ dvptr, c
             for (int j = 0; j < 8; ++j) {
                 col += d16[8 * v + j];
                 const float a = (float)dval[8 * v + j];
-                if (__float_as_uint(a) != 0x80000000u) acc[j & 1] = fmaf(a, __ldg(x + col), acc[j & 1]);
+                if (__float_as_uint(a) != 0x80000000u) acc[j & 1] = fmaf(a, ld_after(x + col), acc[j & 1]);
             }
         sum[l] = acc[0] + acc[1];
     }
@@ -136,7 +136,7 @@ __device__ __forceinline__ void d16_steps(const uint4* dp, const V* vp, const fl
 #pragma unroll
     for (int u = 0; u < N; ++u)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) gx[u][j] = __ldg(x + col[u][j]);
+        for (int j = 0; j < 8; ++j) gx[u][j] = ld_after(x + col[u][j]);
 #pragma unroll
     for (int u = 0; u < N; ++u)
 #pragma unroll
@@ -155,6 +155,7 @@ __global__ void __launch_bounds__(256, sizeof(V) == 4 ? 5 : U == 2 ? 6 : 8)
 k_csr_d16(const uint64_t* __restrict__ dvptr, const uint32_t* __restrict__ dbase, const uint16_t* __restrict__ d16,
           const V* __restrict__ dval, const float* __restrict__ x, uint32_t nrows, const int32_t* __restrict__ g,
           float* __restrict__ out, float* __restrict__ fwproj, float* __restrict__ f, const float* __restrict__ norm) {
+    grid_release();
     const uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) / LPR;
     const uint32_t gl = threadIdx.x % LPR;
     const bool live = row < nrows;
@@ -177,6 +178,7 @@ k_csr_d16(const uint64_t* __restrict__ dvptr, const uint32_t* __restrict__ dbase
     float acc0 = 0.f, acc1 = 0.f;
     dp += gl;
     vp += 8 * gl;
+    grid_wait();
     uint32_t k = 0;
     for (; k + U <= nsteps; k += U) {
         d16_steps<V, LPR, U>(dp, vp, x, prev, acc0, acc1);
@@ -190,7 +192,7 @@ k_csr_d16(const uint64_t* __restrict__ dvptr, const uint32_t* __restrict__ dbase
     if (live && gl == 0) {
         if (isnan(acc)) acc = d16_row_real<V, LPR>(dvptr, dbase, d16, dval, x, row);
         if (EPI == (int)Epi::Correl) {
-            out[row] = (acc != 0.0f) ? __fdiv_rn((float)g[row], acc) : 0.0f;
+            out[row] = (acc != 0.0f) ? __fdiv_rn((float)ld_after(g + row), acc) : 0.0f;
             if (fwproj) fwproj[row] = acc;
         } else if (EPI == (int)Epi::Update) {
             const float tt = __fmul_rn(f[row], acc);
@@ -362,7 +364,7 @@ void sorted_copy(const DevCsr& op, uint32_t*& idx, void*& val, cudaStream_t s) {
 
 template <typename V, int EPI, int LPR, int U>
 void d16_launch(const DevCsr& op, const float* x, const EpiArgs& e, L2Window win, cudaStream_t s) {
-    launch_ex(k_csr_d16<V, EPI, LPR, U>, dim3(grid_groups(op.nrows, LPR)), dim3(256), 0, s, win, op.dvptr, op.dbase,
+    launch_attrs(e.overlap, k_csr_d16<V, EPI, LPR, U>, dim3(grid_groups(op.nrows, LPR)), dim3(256), 0, s, win, op.dvptr, op.dbase,
               op.d16, static_cast<const V*>(op.dval), x, op.nrows, e.g, e.out, e.fwproj,
               e.f, e.norm);
 }
