@@ -40,21 +40,55 @@ __device__ __forceinline__ float4 load_state(const float* p) {
 
 template <typename V, int W, bool NC = true>
 __device__ __forceinline__ void batch_rows(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ idx,
-                                           const V* __restrict__ val, const float* x, uint32_t BT,
+                                           const V* __restrict__ val, const float* x, uint32_t BT, uint32_t na,
                                            uint32_t row, bool ok, int lane, float4& acc) {
     constexpr int LPN = W / 4;  // lanes per nonzero
     constexpr int E = 32 / W;   // entries per lane per 32-entry chunk
-    const int sl = lane % W, chain = sl / LPN, q4 = (sl % LPN) * 4, seg0 = lane - sl;
+    const int sl = lane % W, chain = sl / LPN, seg0 = lane - sl;
+    const uint32_t q4 = (sl % LPN) * 4;
+    // lanes of slots that are not read repeat those of slot 0 (no bytes of their own)
+    const float* xq = x + (q4 < na ? q4 : 0);
     uint64_t s = 0, t = 0;
     if (ok) {
         s = rowptr[row];
         t = rowptr[row + 1];
     }
-    // the warp runs as many chunks as its longest row needs (shuffles stay converged)
-    uint32_t chunks = (uint32_t)((t - s + 31) >> 5);
+    // the warp runs as many chunks as its longest row needs (shuffles stay
+    // converged); from 16 slots on without checks as long as its shortest row is
+    // not used up (3-D mid matrix, FP32, both projections: 16 slots 2.71 -> 2.61
+    // ms, 32 slots 4.23 -> 4.03; with fewer slots, several entries per lane, the
+    // second loop's registers cost more than the checks)
+    uint32_t chunks = (uint32_t)((t - s + 31) >> 5), whole = W >= 16 ? (uint32_t)((t - s) >> 5) : 0;
 #pragma unroll
-    for (int o = W; o < 32; o <<= 1) chunks = max(chunks, __shfl_xor_sync(0xffffffffu, chunks, o));
-    for (uint32_t ch = 0; ch < chunks; ++ch) {
+    for (int o = W; o < 32; o <<= 1) {
+        chunks = max(chunks, __shfl_xor_sync(0xffffffffu, chunks, o));
+        if (W >= 16) whole = min(whole, __shfl_xor_sync(0xffffffffu, whole, o));
+    }
+    const uint32_t* ip = idx + s + sl;
+    const V* vp = val + s + sl;
+    for (uint32_t ch = 0; ch < whole; ++ch) {
+        uint32_t c[E];
+        float v[E];
+#pragma unroll
+        for (int i = 0; i < E; ++i) {
+            c[i] = ld_stream(ip + i * W);
+            v[i] = Val4<V>::one(vp, i * W);
+        }
+        ip += 32;
+        vp += 32;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int src = seg0 + chain + (4 * q) % W;
+            const uint32_t ck = __shfl_sync(0xffffffffu, c[(4 * q) / W], src);
+            const float vk = __shfl_sync(0xffffffffu, v[(4 * q) / W], src);
+            const float4 xv = load_state<NC>(xq + (uint64_t)ck * BT);
+            acc.x = fmaf(vk, xv.x, acc.x);
+            acc.y = fmaf(vk, xv.y, acc.y);
+            acc.z = fmaf(vk, xv.z, acc.z);
+            acc.w = fmaf(vk, xv.w, acc.w);
+        }
+    }
+    for (uint32_t ch = whole; ch < chunks; ++ch) {
         const uint64_t base = s + 32ull * ch;
         // entry base + sl + i*W sits in slot i of lane sl
         uint32_t c[E];
@@ -81,7 +115,7 @@ __device__ __forceinline__ void batch_rows(const uint64_t* __restrict__ rowptr, 
             const uint32_t ck = __shfl_sync(0xffffffffu, c[(4 * q) / W], src);
             const float vk = __shfl_sync(0xffffffffu, v[(4 * q) / W], src);
             if (4 * q < r) {
-                const float4 xv = load_state<NC>(x + (uint64_t)ck * BT + q4);
+                const float4 xv = load_state<NC>(xq + (uint64_t)ck * BT);
                 acc.x = fmaf(vk, xv.x, acc.x);
                 acc.y = fmaf(vk, xv.y, acc.y);
                 acc.z = fmaf(vk, xv.z, acc.z);
@@ -108,9 +142,9 @@ __device__ __forceinline__ float update1(float f, float acc, float n) {
 
 // ratio[row*BT + b] = g/(A f)_b for the first W slots.
 template <typename V, int W>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, W >= 16 ? 6 : W == 8 ? 5 : 4)
 k_batch_fp(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ idx,
-           const V* __restrict__ val, const float* __restrict__ f, uint32_t rows, uint32_t BT,
+           const V* __restrict__ val, const float* __restrict__ f, uint32_t rows, uint32_t BT, uint32_t na,
            const int32_t* __restrict__ g, float* __restrict__ ratio) {
     const int lane = threadIdx.x & 31;
     const uint64_t first = ((blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5) * (32 / W);
@@ -118,9 +152,9 @@ k_batch_fp(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ idx
     const uint64_t row = first + lane / W;
     const bool ok = row < rows;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    batch_rows<V, W>(rowptr, idx, val, f, BT, (uint32_t)row, ok, lane, acc);
+    batch_rows<V, W>(rowptr, idx, val, f, BT, na, (uint32_t)row, ok, lane, acc);
     const int sl = lane % W;
-    if (ok && sl < W / 4) {
+    if (ok && sl < W / 4 && (uint32_t)sl * 4 < na) {
         const uint64_t o = row * BT + sl * 4;
         const int4 gg = *reinterpret_cast<const int4*>(g + o);
         *reinterpret_cast<float4*>(ratio + o) =
@@ -130,9 +164,9 @@ k_batch_fp(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ idx
 
 // f[c*BT + b] = f·(Aᵀ ratio)_b / norm[c] for the slots b < W with iterations left.
 template <typename V, int W>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, W >= 16 ? 6 : W == 8 ? 5 : 4)
 k_batch_bp(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ idx,
-           const V* __restrict__ val, const float* __restrict__ ratio, uint32_t cols, uint32_t BT,
+           const V* __restrict__ val, const float* __restrict__ ratio, uint32_t cols, uint32_t BT, uint32_t na,
            const float* __restrict__ norm, const uint32_t* __restrict__ remaining,
            float* __restrict__ f) {
     const int lane = threadIdx.x & 31;
@@ -141,9 +175,9 @@ k_batch_bp(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ idx
     const uint64_t c = first + lane / W;
     const bool ok = c < cols;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    batch_rows<V, W>(rowptr, idx, val, ratio, BT, (uint32_t)c, ok, lane, acc);
+    batch_rows<V, W>(rowptr, idx, val, ratio, BT, na, (uint32_t)c, ok, lane, acc);
     const int sl = lane % W;
-    if (ok && sl < W / 4) {
+    if (ok && sl < W / 4 && (uint32_t)sl * 4 < na) {
         const uint64_t o = c * BT + sl * 4;
         const uint4 rem = *reinterpret_cast<const uint4*>(remaining + sl * 4);
         const float n = norm[c];
@@ -220,7 +254,7 @@ __global__ void __launch_bounds__(256, W == 32 ? 8 : 6)
 k_batch_loop(const uint64_t* __restrict__ rp, const uint32_t* __restrict__ ix, const V* __restrict__ vl,
              uint32_t rows, const uint64_t* __restrict__ rpT, const uint32_t* __restrict__ ixT,
              const V* __restrict__ vlT, uint32_t cols, const float* __restrict__ norm, uint32_t BT,
-             const int32_t* __restrict__ g, float* f, float* ratio, uint32_t* remaining, uint32_t steps,
+             uint32_t na, const int32_t* __restrict__ g, float* f, float* ratio, uint32_t* remaining, uint32_t steps,
              unsigned* count, int* err) {
     constexpr uint32_t RPW = 32 / W;  // rows per warp
     const int lane = threadIdx.x & 31, sl = lane % W;
@@ -233,8 +267,8 @@ k_batch_loop(const uint64_t* __restrict__ rp, const uint32_t* __restrict__ ix, c
             const uint32_t row = first + lane / W;
             const bool ok = row < rows;
             float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-            batch_rows<V, W, false>(rp, ix, vl, f, BT, row, ok, lane, acc);
-            if (ok && sl < W / 4) {
+            batch_rows<V, W, false>(rp, ix, vl, f, BT, na, row, ok, lane, acc);
+            if (ok && sl < W / 4 && (uint32_t)sl * 4 < na) {
                 const uint64_t o = (uint64_t)row * BT + sl * 4;
                 const int4 gg = *reinterpret_cast<const int4*>(g + o);
                 *reinterpret_cast<float4*>(ratio + o) = make_float4(correl1(gg.x, acc.x), correl1(gg.y, acc.y),
@@ -246,8 +280,8 @@ k_batch_loop(const uint64_t* __restrict__ rp, const uint32_t* __restrict__ ix, c
             const uint32_t c = first + lane / W;
             const bool ok = c < cols;
             float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-            batch_rows<V, W, false>(rpT, ixT, vlT, ratio, BT, c, ok, lane, acc);
-            if (ok && sl < W / 4) {
+            batch_rows<V, W, false>(rpT, ixT, vlT, ratio, BT, na, c, ok, lane, acc);
+            if (ok && sl < W / 4 && (uint32_t)sl * 4 < na) {
                 const uint64_t o = (uint64_t)c * BT + sl * 4;
                 const uint4 rem = *reinterpret_cast<const uint4*>(remaining + sl * 4);
                 const float n = norm[c];
@@ -269,13 +303,13 @@ k_batch_loop(const uint64_t* __restrict__ rp, const uint32_t* __restrict__ ix, c
 template <int W, typename V>
 void fp_w(const DevCsr& A, const BatchArgs& b, L2Window win, cudaStream_t s) {
     launch_ex(k_batch_fp<V, W>, dim3(ceil_div_u((uint64_t)A.nrows * W, 256)), dim3(256), 0, s, win, A.rowptr,
-              A.idx, static_cast<const V*>(A.val), (const float*)b.f, A.nrows, b.tile, b.g, b.ratio);
+              A.idx, static_cast<const V*>(A.val), (const float*)b.f, A.nrows, b.tile, b.slots(), b.g, b.ratio);
 }
 
 template <int W, typename V>
 void bp_w(const DevCsr& AT, const float* norm, const BatchArgs& b, L2Window win, cudaStream_t s) {
     launch_ex(k_batch_bp<V, W>, dim3(ceil_div_u((uint64_t)AT.nrows * W, 256)), dim3(256), 0, s, win, AT.rowptr,
-              AT.idx, static_cast<const V*>(AT.val), (const float*)b.ratio, AT.nrows, b.tile, norm,
+              AT.idx, static_cast<const V*>(AT.val), (const float*)b.ratio, AT.nrows, b.tile, b.slots(), norm,
               (const uint32_t*)b.remaining, b.f);
 }
 
@@ -398,7 +432,7 @@ void loop_w(const DevCsr& A, const DevCsr& AT, const float* norm, const BatchArg
     MLEM_CUDA(cudaLaunchKernelEx(&cfg, kern, (const uint64_t*)A.rowptr, (const uint32_t*)A.idx,
                                  static_cast<const V*>(A.val), A.nrows, (const uint64_t*)AT.rowptr,
                                  (const uint32_t*)AT.idx, static_cast<const V*>(AT.val), AT.nrows, norm, b.tile,
-                                 b.g, b.f, b.ratio, b.remaining, steps, count, err));
+                                 b.slots(), b.g, b.f, b.ratio, b.remaining, steps, count, err));
     count_launch();
 }
 

@@ -309,6 +309,8 @@ struct BatchArgs {
         while (w < a) w <<= 1;
         return w;
     }
+    // slots whose state the projections read and write: `active` rounded up to 4
+    uint32_t slots() const { return (std::min(active ? active : tile, tile) + 3) / 4 * 4; }
 };
 // Slots the projections cover for `active` leading slots in a tile (4..tile).
 inline uint32_t batch_width(uint32_t tile, uint32_t active) {

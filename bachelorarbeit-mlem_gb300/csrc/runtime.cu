@@ -789,7 +789,9 @@ float reference_initial_value(const mlem_matrix* m, const int32_t* g) {
     // main.cu:83-97: FP32 running sum of norm in column order (kept with the
     // matrix), integer sum of g
     int64_t sum_g = 0;
-    for (uint32_t i = 0; i < m->A.nrows; ++i) sum_g += g[i];
+    const uint32_t n = m->A.nrows;
+#pragma omp simd reduction(+ : sum_g)
+    for (uint32_t i = 0; i < n; ++i) sum_g += g[i];
     return (float)sum_g / m->norm_sum;
 }
 

@@ -85,8 +85,8 @@ struct BatchState {
     float* stage_f = nullptr;    // [cols] contiguous staging
     unsigned* bar = nullptr;     // barrier word of the persistent form
     int* err = nullptr;          // set by the persistent form when a barrier wait ran out
-    cudaGraphExec_t graph[4] = {};  // one iteration per projection width 4/8/16/32
-    uint64_t graph_nodes[4] = {};
+    cudaGraphExec_t graph[8] = {};  // one iteration for 4, 8, .. 32 slots
+    uint64_t graph_nodes[8] = {};
     uint64_t bytes = 0;
     void alloc(uint32_t rows, uint32_t cols, uint32_t tile, bool scatter);
     void release();
@@ -135,6 +135,7 @@ struct mlem_matrix {
     mlem::Workspace ws;
     std::map<uint32_t, mlem::MergePlan> plan_A, plan_AT;
     uint32_t batch_tile = 0;          // autotuned batch tile (0 = not yet)
+    float batch_ms[3][8] = {};        // and the iteration times behind it: tile 8 / 16 / 32, slots 4 .. 32 by 4
     uint32_t batch_form = 0;          // autotuned batch form: 1 graphs, 2 persistent (0 = not yet)
     int scatter_lanes = 0;            // autotuned lanes per row of the scatter back projection (0 = not yet)
     int scatter_unroll = 4;           // and its entries per lane in flight

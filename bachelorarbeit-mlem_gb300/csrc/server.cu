@@ -25,6 +25,7 @@
 #include <cmath>
 #include <cstring>
 #include <deque>
+#include <limits>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -96,8 +97,8 @@ static void batch_step(mlem_matrix* m, BatchState& b, cudaStream_t s, bool use_g
         enqueue_batch_iteration(m, b, s, active);
         return;
     }
-    const uint32_t w = m->has_t ? batch_width(b.tile, active) : b.tile;  // the scatter form covers the tile
-    const int gi = w == 4 ? 0 : w == 8 ? 1 : w == 16 ? 2 : 3;
+    const uint32_t w = m->has_t ? b.args(active).slots() : b.tile;  // the scatter form covers the tile
+    const int gi = (int)(w / 4) - 1;
     if (!b.graph[gi]) {
         cudaStream_t cs = nullptr;
         MLEM_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
@@ -124,7 +125,9 @@ static void batch_step(mlem_matrix* m, BatchState& b, cudaStream_t s, bool use_g
     count_launch(b.graph_nodes[gi]);
 }
 
-// Picks the batch tile with the highest images*iterations per second.
+// Times one iteration of every batch tile at each of its projection widths and
+// keeps the tile with the highest images*iterations per second (the server's
+// choice; a batch whose counts are known picks by pool_cost).
 static uint32_t autotune_tile(mlem_matrix* m, cudaStream_t s) {
     if (m->batch_tile) return m->batch_tile;
     const uint32_t rows = m->A.nrows, cols = m->A.ncols;
@@ -133,7 +136,8 @@ static uint32_t autotune_tile(mlem_matrix* m, cudaStream_t s) {
     cudaEvent_t e0, e1;
     MLEM_CUDA(cudaEventCreate(&e0));
     MLEM_CUDA(cudaEventCreate(&e1));
-    for (uint32_t bt : {8u, 16u, 32u}) {
+    for (int ti = 0; ti < 3; ++ti) {
+        const uint32_t bt = 8u << ti;
         BatchState b;
         try {
             b.alloc(rows, cols, bt, !m->has_t);
@@ -148,13 +152,16 @@ static uint32_t autotune_tile(mlem_matrix* m, cudaStream_t s) {
         std::vector<int32_t> cnt((uint64_t)std::max(rows, 1u) * bt, 1);
         MLEM_CUDA(cudaMemcpyAsync(b.f, ones.data(), sizeof(float) * ones.size(), cudaMemcpyHostToDevice, s));
         MLEM_CUDA(cudaMemcpyAsync(b.g, cnt.data(), sizeof(int32_t) * cnt.size(), cudaMemcpyHostToDevice, s));
-        enqueue_batch_iteration(m, b, s, bt);  // warm-up
-        MLEM_CUDA(cudaEventRecord(e0, s));
-        for (int q = 0; q < 3; ++q) enqueue_batch_iteration(m, b, s, bt);
-        MLEM_CUDA(cudaEventRecord(e1, s));
-        MLEM_CUDA(cudaEventSynchronize(e1));
         float ms = 0.f;
-        cudaEventElapsedTime(&ms, e0, e1);
+        for (uint32_t w = m->has_t ? 4 : bt; w <= bt; w *= 2) {
+            enqueue_batch_iteration(m, b, s, w);  // warm-up
+            MLEM_CUDA(cudaEventRecord(e0, s));
+            for (int q = 0; q < 2; ++q) enqueue_batch_iteration(m, b, s, w);
+            MLEM_CUDA(cudaEventRecord(e1, s));
+            MLEM_CUDA(cudaEventSynchronize(e1));
+            cudaEventElapsedTime(&ms, e0, e1);
+            for (uint32_t c = m->has_t ? w / 8 : 0; c < w / 4; ++c) m->batch_ms[ti][c] = ms / 2;
+        }
         const double rate = bt / std::max(1e-6, (double)ms);
         if (rate > best_rate) {
             best_rate = rate;
@@ -167,6 +174,32 @@ static uint32_t autotune_tile(mlem_matrix* m, cudaStream_t s) {
     cudaEventDestroy(e1);
     m->batch_tile = best;
     return best;
+}
+
+// Milliseconds of iterations that a pool of `tile` slots takes for instances
+// entering with these counts, from the measured iteration times (a tile whose
+// state did not fit has none: infinite).
+static double pool_cost(const mlem_matrix* m, uint32_t tile, const std::vector<uint64_t>& counts) {
+    const float* ms = m->batch_ms[tile == 8 ? 0 : tile == 16 ? 1 : 2];
+    if (!(ms[0] > 0.f)) return std::numeric_limits<double>::infinity();
+    std::vector<uint64_t> end(tile, 0);  // step at which a slot is free (0: never taken)
+    size_t next = 0;
+    uint64_t step = 0;
+    double cost = 0.0;
+    while (true) {
+        uint32_t act = 0;
+        uint64_t until = ~0ull;
+        for (uint32_t b = 0; b < tile; ++b) {
+            while (end[b] <= step && next < counts.size()) end[b] = step + counts[next++];
+            if (end[b] > step) {
+                act = b + 1;
+                until = std::min(until, end[b]);
+            }
+        }
+        if (act == 0) return cost;
+        cost += (double)(until - step) * ms[(act + 3) / 4 - 1];
+        step = until;
+    }
 }
 
 // Picks the faster form at the matrix's tile: per-iteration launches or the
@@ -507,15 +540,32 @@ mlem_status mlem_batch_run(mlem_matrix* m, uint32_t count, const int32_t* g, con
         DeviceGuard dg(m->device);
         cudaStream_t s = m->stream;
         const uint32_t rows = m->A.nrows, cols = m->A.ncols;
-        const uint32_t tile = o.tile ? o.tile : autotune_tile(m, s);
-        const bool persistent = (o.form ? o.form : autotune_form(m, tile, s)) == 2;
-        std::unique_lock<std::mutex> plk(persistent_lock(m->device), std::defer_lock);
-        if (persistent) plk.lock();
         std::vector<uint32_t> order(count);
         std::iota(order.begin(), order.end(), 0u);
         if (o.order_by_iterations)
             std::stable_sort(order.begin(), order.end(),
                              [&](uint32_t a, uint32_t b) { return iterations[a] > iterations[b]; });
+        uint32_t tile = o.tile;
+        if (!tile) {
+            // by the cost of this pool, not by the rate of a full tile: 24 instances
+            // of uneven counts on the 3-D mid matrix take 48.9 ms of iterations in 16
+            // slots (refilled) and 56.9 in 32 (a quarter of them never used)
+            autotune_tile(m, s);
+            std::vector<uint64_t> counts;
+            for (uint32_t i : order) counts.push_back(iterations[i]);
+            double best = std::numeric_limits<double>::infinity();
+            tile = m->batch_tile;
+            for (uint32_t t : {8u, 16u, 32u}) {
+                const double c = pool_cost(m, t, counts);
+                if (c < best) {
+                    best = c;
+                    tile = t;
+                }
+            }
+        }
+        const bool persistent = (o.form ? o.form : autotune_form(m, tile, s)) == 2;
+        std::unique_lock<std::mutex> plk(persistent_lock(m->device), std::defer_lock);
+        if (persistent) plk.lock();
         BatchState bs;
         bs.alloc(rows, cols, tile, !m->has_t);
         uint64_t h2d = 0, d2h = 0, iters_total = 0;
@@ -556,7 +606,7 @@ mlem_status mlem_batch_run(mlem_matrix* m, uint32_t count, const int32_t* g, con
         auto admit = [&](uint32_t b) {
             const uint32_t i = order[next++];
             const int32_t* gi = g + (uint64_t)i * rows;
-            if (pinned) {
+            if (pinned && step > 0) {  // nothing runs yet at step 0: a direct copy has nothing to drain
                 const uint32_t j = ring_g++ % kRing;
                 if (ev_g[j]) MLEM_CUDA(cudaEventSynchronize(ev_g[j]));
                 else MLEM_CUDA(cudaEventCreateWithFlags(&ev_g[j], cudaEventDisableTiming));

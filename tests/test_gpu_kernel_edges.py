@@ -206,3 +206,29 @@ def test_merge_tiles_with_empty_runs(pkg, cuda, vt, secsize, long_rows):
     want = np.bincount(col, weights=v * r[rid].astype(np.float64), minlength=cols)
     assert np.all(np.abs(bp - want) <= (np.bincount(col, minlength=cols) + 2) * 2.0**-24 * want)
     m.close()
+
+
+@pytest.mark.parametrize("vt", [0, 1])
+def test_batch_slots_and_row_lengths(pkg, O, cuda, vt):
+    """Batches that leave slots of every width unused, on rows around the 32 entries
+    of a chunk: the same bits in every tile and count, alone and together, and the
+    FP64 oracle's image (the batched tolerance, 1e-5 relative L2)."""
+    cols = 4999
+    rng, rp, col, val = edge_csr(51, cols, False)
+    v = stored(cuda, val, vt).astype(np.float32)
+    x = rng.uniform(0.0, 1.0, (5, cols))
+    G = np.stack([rng.poisson(O.project_f64(rp, col, v, xi) * 20.0) for xi in x]).astype(np.int32)
+    m = pkg.Matrix.from_csr(rp, col, val, cols, value_type=vt)
+    norm = O.colsum(rp, col, v, cols, f64=True)
+    its = [3, 5, 2, 4, 5]
+    alone = [m.batch_run(G[k:k + 1], its[k:k + 1])[0] for k in range(5)]
+    for k in range(5):
+        f0 = np.full(cols, m.initial_value(G[k]), np.float32)
+        assert O.rel_l2(alone[k], O.mlem_f64((rp, col, v), G[k], norm, f0, its[k])) < 1e-5
+    for count in (1, 4, 5, 9, 13, 20, 24, 29, 33):
+        which = np.arange(count) % 5
+        for tile in (0, 8, 16, 32):
+            out = m.batch_run(G[which], [its[k] for k in which], tile=tile)
+            for b, k in enumerate(which):
+                np.testing.assert_array_equal(out[b], alone[k], err_msg=f"count {count} tile {tile} instance {b}")
+    m.close()
