@@ -232,3 +232,21 @@ def test_batch_slots_and_row_lengths(pkg, O, cuda, vt):
             for b, k in enumerate(which):
                 np.testing.assert_array_equal(out[b], alone[k], err_msg=f"count {count} tile {tile} instance {b}")
     m.close()
+
+
+@pytest.mark.parametrize("cols", [1, 31, 33, 256, 257, 8192, 8193, 65_537, 2_000_000])
+@pytest.mark.parametrize("nnz", [1, 4095, 4097, 70_001])
+def test_transpose_pass_shapes(pkg, cols, nnz):
+    """The stable counting sort on both sides of the number of its passes, of a full
+    digit and of a tile of 4,096 elements: bit-exact."""
+    rng = np.random.default_rng(61)
+    rows = 37
+    lens = rng.multinomial(nnz, np.ones(rows) / rows)
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.uint64)
+    col = rng.integers(0, cols, nnz).astype(np.uint32)
+    val = rng.standard_normal(nnz).astype(np.float32)
+    cp, ri, v = pkg.transpose(rp, col, val, cols)
+    order = np.argsort(col, kind="stable")
+    np.testing.assert_array_equal(cp, np.concatenate([[0], np.cumsum(np.bincount(col, minlength=cols))]).astype(np.uint64))
+    np.testing.assert_array_equal(ri, np.repeat(np.arange(rows, dtype=np.uint32), lens)[order])
+    np.testing.assert_array_equal(v.view(np.uint32), val[order].view(np.uint32))
