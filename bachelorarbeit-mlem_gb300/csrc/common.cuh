@@ -95,6 +95,12 @@ __device__ __forceinline__ int32_t ld_after(const int32_t* p) {
     return v;
 }
 
+__device__ __forceinline__ uint32_t ld_after(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+
 __device__ __forceinline__ uint64_t globaltimer_ns() {
     uint64_t t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));

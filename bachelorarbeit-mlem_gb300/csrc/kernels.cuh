@@ -30,7 +30,7 @@ struct EpiArgs {
     float* fwproj = nullptr;      // Correl: optional copy of the projection
     float* f = nullptr;           // Update: image, updated in place
     const float* norm = nullptr;  // Update
-    // csr-vector (DIRECT) and D16 kernels: launched so that they may start while
+    // csr-vector (DIRECT), D16 and merge-path row kernels: launched so that they may start while
     // the previous kernel of the stream drains.  Set inside an MLEM loop: 8.15 ->
     // 7.34 us per iteration on the 2-D ring, 43.9 -> 43.2 us with 6 M nonzeros,
     // 4.26 -> 4.20 ms on the 3-D mid matrix; a single projection only pays for the
@@ -178,13 +178,15 @@ struct MergePlan {
     // true: the row-parallel tile kernel (library-owned, padded operands);
     // false: the per-thread walk over shared-memory products (any arrays)
     bool rows_kernel = false;
+    bool whole = false;          // row kernel: tiles of whole rows, no carries and no fix-up launch
     int lanes = 16;              // row kernel: lanes per row (8 or 16)
     int rows_u = 1;              // row kernel: vectors per lane in flight (1: 16 blocks per SM, 2: 12)
     void release();
 };
 // Builds the tile partition of `op` for a section size (device allocations).
 void merge_plan_build(const DevCsr& op, uint32_t secsize, MergePlan& plan, cudaStream_t s);
-// Merge-path product with deterministic carry fix-up (2 launches).
+// Merge-path product: one launch where the plan's tiles hold whole rows, else
+// two (deterministic carry fix-up).
 void launch_merge_spmv(const DevCsr& op, const MergePlan& plan, const float* x,
                        const EpiArgs& epi, L2Window win, cudaStream_t s);
 

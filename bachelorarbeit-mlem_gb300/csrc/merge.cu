@@ -14,9 +14,9 @@
 // segmented scan in a fixed order.  Both apply the fused epilogue
 // (correlation or update) to rows that end inside the tile and leave the
 // first row of every tile to a small fix-up kernel that adds the carries of
-// earlier tiles in tile order.  The reference instead adds every row fragment
-// with a global atomicAdd (order nondeterministic); results here are
-// deterministic.
+// earlier tiles in tile order (tiles of whole rows need none).  The reference
+// instead adds every row fragment with a global atomicAdd (order
+// nondeterministic); results here are deterministic.
 #include "kernels.cuh"
 
 #include <algorithm>
@@ -65,8 +65,9 @@ __global__ void k_search_ref(const uint64_t* __restrict__ rowptr, uint32_t rows,
 }
 
 // Tile start coordinates at diagonals k*T*S; the end of the path is (rows, nnz).
+// whole: a tile starts with the row that its diagonal falls into.
 __global__ void k_tile_coords(const uint64_t* __restrict__ rowptr, uint32_t rows, uint64_t nnz,
-                              uint64_t tile_items, uint64_t ntiles, uint32_t* __restrict__ ti,
+                              uint64_t tile_items, uint64_t ntiles, bool whole, uint32_t* __restrict__ ti,
                               uint64_t* __restrict__ tj) {
     for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k <= ntiles;
          k += (uint64_t)gridDim.x * blockDim.x) {
@@ -78,7 +79,7 @@ __global__ void k_tile_coords(const uint64_t* __restrict__ rowptr, uint32_t rows
             int64_t i, j;
             search_ref(rowptr, rows, (int64_t)d, i, j);
             ti[k] = (uint32_t)i;
-            tj[k] = (uint64_t)j;
+            tj[k] = whole ? rowptr[i] : (uint64_t)j;
         }
     }
 }
@@ -236,22 +237,25 @@ k_merge_tile(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ i
 
 // Rows that end in tile k but started earlier: sum of carries of the earlier
 // tiles that ended inside the row (in tile order), plus the tile's head.
-__global__ void k_merge_fixup(const uint32_t* __restrict__ ti, const float* __restrict__ carry,
-                              const uint32_t* __restrict__ carry_row,
-                              const float* __restrict__ head, uint64_t ntiles, EpiDev epi) {
+__global__ void k_merge_fixup(const uint32_t* __restrict__ ti, const float* carry, const uint32_t* carry_row,
+                              const float* head, uint64_t ntiles, EpiDev epi) {
+    grid_release();
+    grid_wait();
     for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < ntiles;
          k += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t I0 = ti[k], I1 = ti[k + 1];
         if (I1 == I0) continue;  // the tile's first row does not end here
         int64_t q = (int64_t)k - 1;
-        while (q >= 0 && carry_row[q] == I0) --q;
+        while (q >= 0 && ld_after(carry_row + q) == I0) --q;
         float tot = 0.f;
         bool any = false;
         for (uint64_t p = (uint64_t)(q + 1); p < k; ++p) {
-            tot = any ? tot + carry[p] : carry[p];
+            const float c = ld_after(carry + p);
+            tot = any ? tot + c : c;
             any = true;
         }
-        tot = any ? tot + head[k] : head[k];
+        const float h = ld_after(head + k);
+        tot = any ? tot + h : h;
         epi(I0, tot);
     }
 }
@@ -264,7 +268,8 @@ __global__ void k_merge_fixup(const uint32_t* __restrict__ ti, const float* __re
 // are padded and 16-byte aligned) and a fixed xor reduction.  Rows that end
 // inside the tile get their epilogue here, the tile's first row (which began in
 // an earlier tile) goes to head[k] and the row still open at the tile's end to
-// carry[k], for the same fix-up kernel.  Deterministic.
+// carry[k], for the same fix-up kernel.  WHOLE: tiles of whole rows
+// (merge_plan_build), every row gets its epilogue here.  Deterministic.
 //
 // Why the list: a tile of empty rows (voxels that no LOR crosses, detector
 // pairs beside the grid) holds thousands of them, and taken one by one by 16
@@ -297,9 +302,9 @@ __device__ __forceinline__ float group_part_dot(const uint4* __restrict__ idx4, 
         const uint32_t e0 = 4 * v, e1 = 4 * (v + LPR);  // the second vector starts past the head
         float g0[4], g1[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) g0[k] = (e0 + k >= s) ? __ldg(x + cs0[k]) : 0.f;
+        for (int k = 0; k < 4; ++k) g0[k] = (e0 + k >= s) ? ld_after(x + cs0[k]) : 0.f;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) g1[k] = (e1 + k < t) ? __ldg(x + cs1[k]) : 0.f;
+        for (int k = 0; k < 4; ++k) g1[k] = (e1 + k < t) ? ld_after(x + cs1[k]) : 0.f;
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (e0 + k >= s) acc = fmaf(a0[k], g0[k], acc);
@@ -315,7 +320,7 @@ __device__ __forceinline__ float group_part_dot(const uint4* __restrict__ idx4, 
         const uint32_t e = 4 * v;
         float g[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) g[k] = (e + k >= s && e + k < t) ? __ldg(x + cs[k]) : 0.f;
+        for (int k = 0; k < 4; ++k) g[k] = (e + k >= s && e + k < t) ? ld_after(x + cs[k]) : 0.f;
 #pragma unroll
         for (int k = 0; k < 4; ++k)
             if (e + k >= s && e + k < t) acc = fmaf(a[k], g[k], acc);
@@ -323,16 +328,18 @@ __device__ __forceinline__ float group_part_dot(const uint4* __restrict__ idx4, 
     return acc;
 }
 
-template <typename V, int LPR, int U>
+template <typename V, int LPR, int U, bool WHOLE>
 __global__ void __launch_bounds__(kRowsT, U == 1 ? 16 : 12)
 k_merge_rows(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ idx, const V* __restrict__ val,
              const float* __restrict__ x, uint32_t rows, const uint32_t* __restrict__ ti,
              const uint64_t* __restrict__ tj, float* __restrict__ carry, uint32_t* __restrict__ carry_row,
              float* __restrict__ head, EpiDev epi) {
+    grid_release();
     const uint64_t k = blockIdx.x;
     const uint32_t I0 = ti[k], I1 = ti[k + 1];
     const uint64_t J0 = tj[k], J1 = tj[k + 1];
-    const uint32_t nrow_l = I1 - I0;  // rows that end inside the tile
+    const uint32_t nrow_l = I1 - I0;           // rows that end inside the tile
+    const uint32_t n_row = nrow_l + !WHOLE;    // rows with a part in it
     constexpr uint32_t NG = kRowsT / LPR;  // lane groups of the CTA
     __shared__ uint32_t s_i[kRowsT], s_beg[kRowsT], s_end[kRowsT], s_cnt[kRowsT / 32];
     const uint32_t grp = threadIdx.x / LPR, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -341,17 +348,21 @@ k_merge_rows(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ i
     const uint64_t base = J0 & ~3ull;
     const uint4* idx4 = reinterpret_cast<const uint4*>(idx + base);
     const V* vb = val + base;
-    for (uint32_t c0 = 0; c0 <= nrow_l; c0 += kRowsT) {
+    if (n_row == 0) grid_wait();  // every block waits before it ends
+    for (uint32_t c0 = 0; c0 < n_row; c0 += kRowsT) {
         const uint32_t i = c0 + threadIdx.x, r = I0 + i;
         uint64_t s = J0, t = J0;
-        if (i <= nrow_l && r < rows) {
+        if (i < n_row && r < rows) {
             s = rowptr[r];
             t = rowptr[r + 1];
-            s = s < J0 ? J0 : s;
-            t = t > J1 ? J1 : t;
+            if (!WHOLE) {
+                s = s < J0 ? J0 : s;
+                t = t > J1 ? J1 : t;
+            }
         }
-        const bool keep = i <= nrow_l && (s < t || i == 0 || i == nrow_l);
-        if (i <= nrow_l && !keep) epi(r, 0.f);
+        if (c0 == 0) grid_wait();
+        const bool keep = i < n_row && (s < t || (!WHOLE && (i == 0 || i == nrow_l)));
+        if (i < n_row && !keep) epi(r, 0.f);
         const unsigned kept = __ballot_sync(0xffffffffu, keep);
         if (c0) __syncthreads();  // the list of the previous rows is used up
         if (lane == 0) s_cnt[w] = __popc(kept);
@@ -375,7 +386,9 @@ k_merge_rows(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ i
 #pragma unroll
             for (int o = LPR / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(mask, acc, o);
             if (sub == 0) {
-                if (ii == nrow_l) {  // still open at the tile's end (or past the last row)
+                if (WHOLE) {
+                    epi(I0 + ii, acc);
+                } else if (ii == nrow_l) {  // still open at the tile's end (or past the last row)
                     carry[k] = acc;
                     carry_row[k] = I0 + ii;
                 } else if (ii == 0) {
@@ -389,26 +402,28 @@ k_merge_rows(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ i
 }
 
 template <typename V>
-void merge_launch_t(const DevCsr& op, const MergePlan& p, const float* x, const EpiDev& e,
+void merge_launch_t(const DevCsr& op, const MergePlan& p, const float* x, const EpiDev& e, bool overlap,
                     L2Window win, cudaStream_t s) {
     auto rows = [&](auto kern) {
-        launch_ex(kern, dim3((unsigned)p.ntiles), dim3(kRowsT), 0, s, win, op.rowptr, op.idx,
-                  static_cast<const V*>(op.val), x, op.nrows, p.tile_i, p.tile_j, p.carry, p.carry_row, p.head, e);
+        launch_attrs(overlap, kern, dim3((unsigned)p.ntiles), dim3(kRowsT), 0, s, win, op.rowptr, op.idx,
+                     static_cast<const V*>(op.val), x, op.nrows, p.tile_i, p.tile_j, p.carry, p.carry_row, p.head, e);
     };
-    if (p.rows_kernel && p.lanes == 16) {
-        if (p.rows_u == 2) rows(k_merge_rows<V, 16, 2>);
-        else rows(k_merge_rows<V, 16, 1>);
-    } else if (p.rows_kernel) {
-        if (p.rows_u == 2) rows(k_merge_rows<V, 8, 2>);
-        else rows(k_merge_rows<V, 8, 1>);
+    if (p.whole) {
+        if (p.lanes == 16) rows(p.rows_u == 2 ? k_merge_rows<V, 16, 2, true> : k_merge_rows<V, 16, 1, true>);
+        else rows(p.rows_u == 2 ? k_merge_rows<V, 8, 2, true> : k_merge_rows<V, 8, 1, true>);
+        return;
     }
-    else
+    if (p.rows_kernel) {
+        if (p.lanes == 16) rows(p.rows_u == 2 ? k_merge_rows<V, 16, 2, false> : k_merge_rows<V, 16, 1, false>);
+        else rows(p.rows_u == 2 ? k_merge_rows<V, 8, 2, false> : k_merge_rows<V, 8, 1, false>);
+    } else {
         launch_ex(k_merge_tile<V>, dim3((unsigned)p.ntiles), dim3(p.threads), p.smem, s, win,
                   op.rowptr, op.idx, static_cast<const V*>(op.val), x, op.nrows, p.secsize,
                   p.tile_i, p.tile_j, p.carry, p.carry_row, p.head, e);
+    }
     const unsigned fg = std::max(1u, std::min<unsigned>(ceil_div_u(p.ntiles, 256), 152u * 8u));
-    launch_ex(k_merge_fixup, dim3(fg), dim3(256), 0, s, L2Window{}, p.tile_i, p.carry,
-              p.carry_row, p.head, p.ntiles, e);
+    launch_attrs(overlap, k_merge_fixup, dim3(fg), dim3(256), 0, s, L2Window{}, p.tile_i, p.carry,
+                 p.carry_row, p.head, p.ntiles, e);
 }
 
 }  // namespace
@@ -445,7 +460,8 @@ void merge_plan_build(const DevCsr& op, uint32_t secsize, MergePlan& plan, cudaS
     // Row-parallel tiles of the merge path: at least secsize items per thread,
     // and enough items for about 32 average rows so that the CTA's groups share
     // the tile's rows evenly (fewer, down to 8, where the tiles would not fill
-    // 152 SMs x 16 CTAs: 2-D ring 19 us per iteration with 8, 33 with 32); at
+    // 152 SMs x 16 CTAs: with tiles of shared rows the 2-D ring took 19 us per
+    // iteration with 8, 33 with 32); at
     // most 65536 items.  8 lanes take a row of a mean below 96, 16 the longer ones
     // (mean 38: 0.080 against 0.104 ms; mean 313: 0.363 against 0.352).
     plan.rows_kernel = true;
@@ -456,6 +472,15 @@ void merge_plan_build(const DevCsr& op, uint32_t secsize, MergePlan& plan, cudaS
     const uint64_t rows_per_tile = std::min<uint64_t>(std::max<uint64_t>(op.nrows / (152ull * 16), 8), 32);
     const uint64_t TS =
         std::min<uint64_t>(std::max<uint64_t>((uint64_t)kRowsT * secsize, rows_per_tile * per_row), 65536ull);
+    // Whole rows per tile where no row is longer than a tile's items: a tile then
+    // starts with a row, holds at most two tiles' items, and neither carries nor
+    // the fix-up launch are needed; no lane group walks more than it may in a
+    // tile of shared rows.  A longer row is shared out to several tiles.  Per
+    // iteration, with and without whole rows (the latter without overlapped
+    // launches, EpiArgs::overlap): 1,770 short rows 6.9 / 14.5 us, 2-D ring 10.8 /
+    // 16.9 us, 6 M nonzeros 66.7 / 79.6 us, 3-D mid matrix 0.677 / 0.729 ms
+    // (locality layout 0.603 / 0.682 ms).
+    plan.whole = op.max_row <= TS;
     plan.ntiles = (items + TS - 1) / TS;
     MLEM_REQUIRE(plan.ntiles < (1ull << 31), MLEM_EUNSUPPORTED, "merge path: too many tiles");
     plan.smem = 0;
@@ -489,7 +514,7 @@ void merge_plan_build(const DevCsr& op, uint32_t secsize, MergePlan& plan, cudaS
         }
     }
     const unsigned grid = std::max(1u, std::min<unsigned>(ceil_div_u(plan.ntiles + 1, 256), 152u * 16u));
-    k_tile_coords<<<grid, 256, 0, s>>>(op.rowptr, op.nrows, op.nnz, TS, plan.ntiles, plan.tile_i,
+    k_tile_coords<<<grid, 256, 0, s>>>(op.rowptr, op.nrows, op.nnz, TS, plan.ntiles, plan.whole, plan.tile_i,
                                        plan.tile_j);
     MLEM_LAUNCHED();
 }
@@ -499,9 +524,9 @@ void launch_merge_spmv(const DevCsr& op, const MergePlan& plan, const float* x, 
     if (plan.ntiles == 0) return;
     EpiDev e{(int)epi.kind, epi.g, epi.out, epi.fwproj, epi.f, epi.norm};
     switch (op.vt) {
-        case MLEM_VAL_F32: merge_launch_t<float>(op, plan, x, e, win, s); break;
-        case MLEM_VAL_F16: merge_launch_t<__half>(op, plan, x, e, win, s); break;
-        default: merge_launch_t<__nv_bfloat16>(op, plan, x, e, win, s);
+        case MLEM_VAL_F32: merge_launch_t<float>(op, plan, x, e, epi.overlap, win, s); break;
+        case MLEM_VAL_F16: merge_launch_t<__half>(op, plan, x, e, epi.overlap, win, s); break;
+        default: merge_launch_t<__nv_bfloat16>(op, plan, x, e, epi.overlap, win, s);
     }
 }
 
@@ -631,7 +656,7 @@ extern "C" mlem_status mlem_forward_project_merge_noalloc(const uint64_t* rowptr
         p.head = reinterpret_cast<float*>(base + off);
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         const unsigned grid = std::max(1u, std::min<unsigned>(ceil_div_u(ntiles + 1, 256), 152u * 16u));
-        k_tile_coords<<<grid, 256, 0, s>>>(rowptr_dev, rows, nnz, TS, ntiles, p.tile_i, p.tile_j);
+        k_tile_coords<<<grid, 256, 0, s>>>(rowptr_dev, rows, nnz, TS, ntiles, false, p.tile_i, p.tile_j);
         MLEM_LAUNCHED();
         DevCsr A;
         A.nrows = rows;

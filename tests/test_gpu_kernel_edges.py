@@ -208,6 +208,44 @@ def test_merge_tiles_with_empty_runs(pkg, cuda, vt, secsize, long_rows):
     m.close()
 
 
+@pytest.mark.parametrize("vt", [0, 1, 2])
+@pytest.mark.parametrize("mean", [20, 150])
+@pytest.mark.parametrize("longest", [1, 640, 641, 1300])
+def test_merge_tiles_of_whole_rows(pkg, cuda, vt, mean, longest):
+    """Longest rows around the items of a tile (128 threads x 5 items, or 8 mean rows),
+    where the merge-path tiles change from whole rows to shared ones, beside tiles
+    that hold no row end: single products and an image of 40 iterations."""
+    rng, cols = np.random.default_rng(longest + mean), 3001
+    lens = rng.integers(0, 2 * mean, 3000)
+    lens[rng.random(3000) < 0.2] = 0
+    lens = np.minimum(lens, longest)
+    lens[[0, 77, 78, 79, 2999]] = longest
+    col = rng.integers(0, cols, lens.sum()).astype(np.uint32)
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.uint64)
+    val = rng.uniform(0.05, 1.0, len(col)).astype(np.float32)
+    rid, v = np.repeat(np.arange(3000), lens), stored(cuda, val, vt)
+    x = rng.uniform(0.5, 1.5, cols).astype(np.float32)
+    g = rng.integers(0, 50, 3000).astype(np.int32)
+    m = pkg.Matrix.from_csr(rp, col, val, cols, value_type=vt)
+    dx, dg = cuda.from_numpy(x).cuda(), cuda.from_numpy(g).cuda()
+    ratio, fp, bp = (cuda.full((n,), -1.0, device="cuda") for n in (3000, 3000, cols))
+    m.forward_project(dx.data_ptr(), dg.data_ptr(), ratio.data_ptr(), fp.data_ptr(), spmv=pkg.SPMV_MERGE)
+    m.back_project(ratio.data_ptr(), bp.data_ptr(), spmv=pkg.SPMV_MERGE)
+    fp, bp, ratio = fp.cpu().numpy(), bp.cpu().numpy(), ratio.cpu().numpy()
+    want = np.bincount(rid, weights=v * x[col].astype(np.float64), minlength=3000)
+    assert np.all(np.abs(fp - want) <= (lens + 2) * 2.0**-24 * want)
+    want = np.bincount(col, weights=v * ratio[rid].astype(np.float64), minlength=cols)
+    assert np.all(np.abs(bp - want) <= (np.bincount(col, minlength=cols) + 2) * 2.0**-24 * want)
+    # an iteration's relative rounding error is at most the two sums' (lens + column
+    # entries) plus 5 operations; iterations with positive weights do not amplify it
+    # beyond their sum, here with a factor of 4 to spare for the ratio's share
+    f = {k: m.run(g, 40, x, spmv=k) for k in (pkg.SPMV_MERGE, pkg.SPMV_CSR_VECTOR)}
+    a, b = (np.asarray(q, np.float64) for q in f.values())
+    per = int(lens.max()) + int(np.bincount(col, minlength=cols).max()) + 5
+    assert np.linalg.norm(a - b) <= 4 * 40 * per * 2.0**-24 * np.linalg.norm(b)
+    m.close()
+
+
 @pytest.mark.parametrize("vt", [0, 1])
 def test_batch_slots_and_row_lengths(pkg, O, cuda, vt):
     """Batches that leave slots of every width unused, on rows around the 32 entries
