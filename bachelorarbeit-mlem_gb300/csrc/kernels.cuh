@@ -192,6 +192,8 @@ void launch_merge_spmv(const DevCsr& op, const MergePlan& plan, const float* x,
 
 // ------------------------------------------------------------- transpose.cu
 // Stable counting sort by column of A (f32 values) -> Aᵀ with u32 row ids.
+// Zeroes the entries of idx and val past nnz (16-byte loads may touch them).
+void zero_padding(const DevCsr& c, cudaStream_t s);
 void transpose_device(const DevCsr& A, DevCsr& AT, cudaStream_t s);
 // norm[c] = (float) Σ (double) val over column c.
 void colsum_from_transpose(const DevCsr& AT, float* norm, cudaStream_t s);

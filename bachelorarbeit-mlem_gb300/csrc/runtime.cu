@@ -1085,8 +1085,7 @@ static void upload_csr(const mlem_csr_host* c, DevCsr& A, cudaStream_t s) {
     MLEM_CUDA(cudaMalloc(&A.rowptr, sizeof(uint64_t) * ((uint64_t)c->rows + 1)));
     MLEM_CUDA(cudaMalloc(&A.idx, sizeof(uint32_t) * padded(c->nnz)));
     MLEM_CUDA(cudaMalloc(&A.val, sizeof(float) * padded(c->nnz)));
-    MLEM_CUDA(cudaMemsetAsync(A.idx, 0, sizeof(uint32_t) * padded(c->nnz), s));
-    MLEM_CUDA(cudaMemsetAsync(A.val, 0, sizeof(float) * padded(c->nnz), s));
+    zero_padding(A, s);
     MLEM_CUDA(cudaMemcpyAsync(A.rowptr, c->rowptr, sizeof(uint64_t) * ((uint64_t)c->rows + 1),
                               cudaMemcpyHostToDevice, s));
     if (c->nnz) {

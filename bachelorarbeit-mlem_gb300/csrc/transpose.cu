@@ -8,11 +8,10 @@
 //
 // Here the same permutation is produced by a stable LSD radix sort on the
 // GPU: key = column index (8-bit digits, as many passes as the column count
-// needs), payload = (row id, value bits).  Each pass is a per-tile digit
+// needs), row id and value as payloads.  Each pass is a per-tile digit
 // histogram, an exclusive scan over (digit, tile) and a scatter in which every
-// warp ranks its elements chunk by chunk with __match_any_sync, so equal
-// digits keep their input order (stable).  The column pointer is a count +
-// exclusive scan.  The result is bit-identical to the reference transpose.
+// warp ranks its elements chunk by chunk, so equal digits keep their input
+// order (stable).  The column pointer is a count + exclusive scan.  The result is bit-identical to the reference transpose.
 #include "kernels.cuh"
 
 #include <algorithm>
@@ -142,16 +141,14 @@ __global__ void k_col_count(const uint32_t* __restrict__ col, uint64_t nnz, uint
         atomicAdd(cnt + col[e], 1u);
 }
 
-// payload[e] = row(e) | value_bits(e) << 32, one warp per row.
-__global__ void k_row_payload(const uint64_t* __restrict__ rowptr, const float* __restrict__ val,
-                              uint32_t rows, uint64_t* __restrict__ pay) {
+// row_of[e] = row of entry e, one warp per row.
+__global__ void k_row_of(const uint64_t* __restrict__ rowptr, uint32_t rows, uint32_t* __restrict__ row_of) {
     const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
     for (uint32_t r = wid; r < rows; r += nw) {
         const uint64_t s = rowptr[r], t = rowptr[r + 1];
-        for (uint64_t e = s + lane; e < t; e += 32)
-            pay[e] = (uint64_t)r | ((uint64_t)__float_as_uint(val[e]) << 32);
+        for (uint64_t e = s + lane; e < t; e += 32) row_of[e] = r;
     }
 }
 
@@ -171,22 +168,25 @@ __global__ void __launch_bounds__(kRsT) k_radix_hist(const uint32_t* __restrict_
     hist[(uint64_t)threadIdx.x * ntiles + blockIdx.x] = cnt[threadIdx.x];
 }
 
-// Stable scatter of one radix pass.  Warp w of the tile owns elements
-// [tile + w*512, +512) and ranks them 32 at a time in order.  The ranked keys,
-// then the payloads, pass through shared memory so that consecutive threads
-// write consecutive elements of a digit's run: written straight from their
-// input order, 32 lanes hit up to 32 sectors with 4 or 8 bytes each, which is
-// what the pass spent its time on (208 M elements, 256 digits: 6.2 -> 2.5 ms; the
-// last of three passes over 784,000 columns has 12 digits and long runs either
-// way: 1.2 -> 1.8 ms, and a straight form kept for it gained nothing in sum).
-// Digits of 7 bits in three passes were no faster.
+// Stable scatter of one radix pass over digits of `bits` bits (keys, rows and
+// values in three arrays).  Warp w of the tile owns elements [tile + w*512,
+// +512) and ranks them 32 at a time in order: the lanes of equal digit are the
+// intersection of one ballot per digit bit.  The ranked keys, rows and values
+// pass through shared memory so that consecutive threads write consecutive
+// elements of a digit's run (written straight from their input order, 32 lanes
+// hit up to 32 sectors with 4 or 8 bytes each: 208 M elements, 256 digits 6.2
+// against 2.5 ms).  With ballots instead of __match_any_sync, and rows and
+// values apart, so that the output arrays hold them between passes:
+// mlem_matrix_create of the 3-D mid matrix (208 M nonzeros, three passes) 32.5
+// -> 26.8 ms, a one-call reconstruction of 30 M nonzeros 9.65 -> 8.64 ms.
+// Digits of 7 bits in three passes were no faster (at 2.5 ms a pass).
 template <bool LAST>
-__global__ void __launch_bounds__(kRsT)
-k_radix_scatter(const uint32_t* __restrict__ keys_in, const uint64_t* __restrict__ pay_in,
-                uint64_t n, int shift, const uint32_t* __restrict__ offs, uint64_t ntiles,
-                uint32_t* __restrict__ keys_out, uint64_t* __restrict__ pay_out,
-                uint32_t* __restrict__ row_out, float* __restrict__ val_out) {
-    __shared__ uint64_t buf[kRsTile];  // keys, then payloads, in rank order
+__global__ void __launch_bounds__(kRsT, 4)
+k_radix_scatter(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ row_in,
+                const uint32_t* __restrict__ val_in, uint64_t n, int shift, int bits,
+                const uint32_t* __restrict__ offs, uint64_t ntiles, uint32_t* __restrict__ keys_out,
+                uint32_t* __restrict__ row_out, uint32_t* __restrict__ val_out) {
+    __shared__ uint32_t buf[kRsTile];  // keys, then rows, then values, in rank order
     __shared__ uint32_t wcnt[kRsWarps][256];
     __shared__ uint32_t goff[256];  // output position of a digit's run less its first rank
     __shared__ uint32_t sh[8];
@@ -195,38 +195,39 @@ k_radix_scatter(const uint32_t* __restrict__ keys_in, const uint64_t* __restrict
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned lt_mask = (1u << lane) - 1u;
     const uint64_t tile = blockIdx.x * (uint64_t)kRsTile;
-    const uint64_t base = tile + (uint64_t)w * (32 * kRsIpt);
     const uint32_t here = (uint32_t)(n - tile < (uint64_t)kRsTile ? n - tile : (uint64_t)kRsTile);
+    const uint32_t first = w * (32 * kRsIpt) + lane;  // this thread's elements: tile + first + 32 c
+    keys_in += tile;
+    row_in += tile;
+    val_in += tile;
     uint32_t key[kRsIpt];
     uint32_t pos[kRsIpt];
 #pragma unroll
-    for (int c = 0; c < kRsIpt; ++c) {
-        const uint64_t e = base + c * 32 + lane;
-        key[c] = e < n ? keys_in[e] : 0u;
-    }
+    for (int c = 0; c < kRsIpt; ++c) key[c] = first + 32 * c < here ? keys_in[first + 32 * c] : 0u;
 #pragma unroll
     for (int c = 0; c < kRsIpt; ++c) {
-        const uint64_t e = base + c * 32 + lane;
-        const bool valid = e < n;
-        const unsigned vm = __ballot_sync(0xffffffffu, valid);
+        const bool valid = first + 32 * c < here;
         const uint32_t d = (key[c] >> shift) & 255u;
-        unsigned peers = 0, cnt = 0;
-        if (valid) {
-            peers = __match_any_sync(vm, d);
-            cnt = wcnt[w][d];
-            pos[c] = cnt + __popc(peers & lt_mask);
+        unsigned peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+            if (b >= bits) break;  // uniform
+            const unsigned set = __ballot_sync(0xffffffffu, (d >> b) & 1u);
+            peers &= (d >> b) & 1u ? set : ~set;
         }
+        const unsigned cnt = wcnt[w][d];
+        pos[c] = cnt + __popc(peers & lt_mask);
         __syncwarp();
         if (valid && (peers & lt_mask) == 0) wcnt[w][d] = cnt + __popc(peers);
         __syncwarp();
     }
     __syncthreads();
     {  // ranks: exclusive prefix over digits, then per digit over the warps in order
-        uint32_t total = 0, first;
+        uint32_t total = 0, start;
         for (int q = 0; q < kRsWarps; ++q) total += wcnt[q][threadIdx.x];
-        block_excl_scan<uint32_t>(total, first, sh);
-        goff[threadIdx.x] = offs[(uint64_t)threadIdx.x * ntiles + blockIdx.x] - first;
-        uint32_t run = first;
+        block_excl_scan<uint32_t>(total, start, sh);
+        goff[threadIdx.x] = offs[(uint64_t)threadIdx.x * ntiles + blockIdx.x] - start;
+        uint32_t run = start;
         for (int q = 0; q < kRsWarps; ++q) {
             const uint32_t c = wcnt[q][threadIdx.x];
             wcnt[q][threadIdx.x] = run;
@@ -234,12 +235,11 @@ k_radix_scatter(const uint32_t* __restrict__ keys_in, const uint64_t* __restrict
         }
     }
     __syncthreads();
-    uint32_t* kbuf = reinterpret_cast<uint32_t*>(buf);
 #pragma unroll
     for (int c = 0; c < kRsIpt; ++c) {
-        if (base + c * 32 + lane < n) {
+        if (first + 32 * c < here) {
             pos[c] += wcnt[w][(key[c] >> shift) & 255u];
-            kbuf[pos[c]] = key[c];
+            buf[pos[c]] = key[c];
         }
     }
     __syncthreads();
@@ -248,31 +248,28 @@ k_radix_scatter(const uint32_t* __restrict__ keys_in, const uint64_t* __restrict
     for (int c = 0; c < kRsIpt; ++c) {
         const uint32_t r = c * kRsT + threadIdx.x;
         if (r < here) {
-            const uint32_t k = kbuf[r];
+            const uint32_t k = buf[r];
             out[c] = goff[(k >> shift) & 255u] + r;
             if (!LAST) keys_out[out[c]] = k;
         }
     }
-    __syncthreads();
+    auto pass = [&](const uint32_t* __restrict__ in, uint32_t* __restrict__ dst) {
+        uint32_t x[kRsIpt];
 #pragma unroll
-    for (int c = 0; c < kRsIpt; ++c) {
-        const uint64_t e = base + c * 32 + lane;
-        if (e < n) buf[pos[c]] = pay_in[e];
-    }
-    __syncthreads();
+        for (int c = 0; c < kRsIpt; ++c) x[c] = first + 32 * c < here ? in[first + 32 * c] : 0u;
+        __syncthreads();  // buf is free
 #pragma unroll
-    for (int c = 0; c < kRsIpt; ++c) {
-        const uint32_t r = c * kRsT + threadIdx.x;
-        if (r < here) {
-            const uint64_t p = buf[r];
-            if (LAST) {
-                row_out[out[c]] = (uint32_t)p;
-                val_out[out[c]] = __uint_as_float((uint32_t)(p >> 32));
-            } else {
-                pay_out[out[c]] = p;
-            }
+        for (int c = 0; c < kRsIpt; ++c)
+            if (first + 32 * c < here) buf[pos[c]] = x[c];
+        __syncthreads();
+#pragma unroll
+        for (int c = 0; c < kRsIpt; ++c) {
+            const uint32_t r = c * kRsT + threadIdx.x;
+            if (r < here) dst[out[c]] = buf[r];
         }
-    }
+    };
+    pass(row_in, row_out);
+    pass(val_in, val_out);
 }
 
 // norm[c] = Σ val over row c of Aᵀ, FP64, lane-strided then xor tree.
@@ -373,6 +370,13 @@ void scan_counts_u64(const uint32_t* in, uint64_t* out, uint64_t n, cudaStream_t
     scan_exclusive<uint32_t, uint64_t>(in, out, n, out + n, s);
 }
 
+void zero_padding(const DevCsr& c, cudaStream_t s) {
+    const uint64_t n = c.nnz, pad = padded(n) - n;
+    if (pad == 0) return;
+    MLEM_CUDA(cudaMemsetAsync(c.idx + n, 0, sizeof(uint32_t) * pad, s));
+    MLEM_CUDA(cudaMemsetAsync(static_cast<unsigned char*>(c.val) + n * val_bytes(c.vt), 0, pad * val_bytes(c.vt), s));
+}
+
 void transpose_device(const DevCsr& A, DevCsr& AT, cudaStream_t s) {
     MLEM_REQUIRE(A.vt == MLEM_VAL_F32, MLEM_EINVAL, "transpose expects f32 values");
     MLEM_REQUIRE(A.nnz < (1ull << 32), MLEM_EUNSUPPORTED, "transpose: nnz must be < 2^32");
@@ -384,8 +388,7 @@ void transpose_device(const DevCsr& A, DevCsr& AT, cudaStream_t s) {
     MLEM_CUDA(cudaMalloc(&AT.rowptr, sizeof(uint64_t) * ((uint64_t)AT.nrows + 1)));
     MLEM_CUDA(cudaMalloc(&AT.idx, sizeof(uint32_t) * padded(n)));
     MLEM_CUDA(cudaMalloc(&AT.val, sizeof(float) * padded(n)));
-    MLEM_CUDA(cudaMemsetAsync(AT.idx, 0, sizeof(uint32_t) * padded(n), s));
-    MLEM_CUDA(cudaMemsetAsync(AT.val, 0, sizeof(float) * padded(n), s));
+    zero_padding(AT, s);
 
     // column pointer: count + exclusive scan (cscColPtr of sptrans.h:455-463)
     uint32_t* cnt = nullptr;
@@ -404,45 +407,46 @@ void transpose_device(const DevCsr& A, DevCsr& AT, cudaStream_t s) {
     const int passes = std::max(1, (bits + 7) / 8);
     const uint64_t ntiles = (n + kRsTile - 1) / kRsTile;
 
-    uint32_t *kb[2] = {nullptr, nullptr}, *hist = nullptr, *offs = nullptr;
-    uint64_t* pb[2] = {nullptr, nullptr};
-    for (int q = 0; q < 2; ++q) {
-        MLEM_CUDA(cudaMallocAsync(&kb[q], sizeof(uint32_t) * n, s));
-        MLEM_CUDA(cudaMallocAsync(&pb[q], sizeof(uint64_t) * n, s));
-    }
-    MLEM_CUDA(cudaMallocAsync(&hist, sizeof(uint32_t) * 256 * ntiles, s));
-    MLEM_CUDA(cudaMallocAsync(&offs, sizeof(uint32_t) * 256 * ntiles, s));
+    // Keys move between two buffers, rows and values between a temporary and the
+    // output, so that the last pass writes the output; the rows start in the
+    // one of these that the first pass does not write, the values in A.  16
+    // bytes of temporaries per nonzero (24 with packed payloads), which a
+    // one-call reconstruction pays for at allocation and release.
+    uint32_t *kb[2] = {nullptr, nullptr}, *tr = nullptr, *tv = nullptr, *hist = nullptr, *offs = nullptr;
+    auto alloc = [&](uint32_t*& p, uint64_t words) { MLEM_CUDA(cudaMallocAsync(&p, sizeof(uint32_t) * words, s)); };
+    for (int q = 0; q < std::min(passes - 1, 2); ++q) alloc(kb[q], n);
+    alloc(tr, n);
+    if (passes > 1) alloc(tv, n);
+    alloc(hist, 256 * ntiles);
+    alloc(offs, 256 * ntiles);
 
-    k_row_payload<<<grid_for((uint64_t)A.nrows * 32, 256, 152u * 32u), 256, 0, s>>>(
-        A.rowptr, static_cast<const float*>(A.val), A.nrows, pb[0]);
+    uint32_t* rows[2] = {AT.idx, tr};  // by passes left, even or odd
+    uint32_t* vals[2] = {static_cast<uint32_t*>(AT.val), tv};
+    uint32_t* row_of = rows[passes & 1];
+    k_row_of<<<grid_for((uint64_t)A.nrows * 32, 256, 152u * 32u), 256, 0, s>>>(A.rowptr, A.nrows, row_of);
     MLEM_LAUNCHED();
 
-    const uint32_t* kin = A.idx;
-    int cur = 0;
+    const uint32_t *kin = A.idx, *rin = row_of, *vin = static_cast<const uint32_t*>(A.val);
     for (int p = 0; p < passes; ++p) {
-        const int shift = 8 * p;
-        const bool last = (p == passes - 1);
+        const int shift = 8 * p, left = passes - 1 - p;
         k_radix_hist<<<(unsigned)ntiles, kRsT, 0, s>>>(kin, n, shift, hist, ntiles);
         MLEM_LAUNCHED();
         scan_exclusive<uint32_t, uint32_t>(hist, offs, 256 * ntiles, (uint32_t*)nullptr, s);
-        if (last) {
-            k_radix_scatter<true><<<(unsigned)ntiles, kRsT, 0, s>>>(
-                kin, pb[cur], n, shift, offs, ntiles, nullptr, nullptr, AT.idx,
-                static_cast<float*>(AT.val));
-        } else {
-            k_radix_scatter<false><<<(unsigned)ntiles, kRsT, 0, s>>>(
-                kin, pb[cur], n, shift, offs, ntiles, kb[cur ^ 1], pb[cur ^ 1], nullptr, nullptr);
-        }
+        const int width = std::min(8, bits - shift);
+        uint32_t *ro = rows[left & 1], *vo = vals[left & 1], *ko = kb[p & 1];
+        if (left)
+            k_radix_scatter<false><<<(unsigned)ntiles, kRsT, 0, s>>>(kin, rin, vin, n, shift, width, offs, ntiles, ko,
+                                                                     ro, vo);
+        else
+            k_radix_scatter<true><<<(unsigned)ntiles, kRsT, 0, s>>>(kin, rin, vin, n, shift, width, offs, ntiles,
+                                                                    nullptr, ro, vo);
         MLEM_LAUNCHED();
-        kin = kb[cur ^ 1];
-        cur ^= 1;
+        kin = ko;
+        rin = ro;
+        vin = vo;
     }
-    for (int q = 0; q < 2; ++q) {
-        MLEM_CUDA(cudaFreeAsync(kb[q], s));
-        MLEM_CUDA(cudaFreeAsync(pb[q], s));
-    }
-    MLEM_CUDA(cudaFreeAsync(hist, s));
-    MLEM_CUDA(cudaFreeAsync(offs, s));
+    for (uint32_t* p : {kb[0], kb[1], tr, tv, hist, offs})
+        if (p) MLEM_CUDA(cudaFreeAsync(p, s));
     AT.max_row = max_row_length(AT.rowptr, AT.nrows, s);
 }
 

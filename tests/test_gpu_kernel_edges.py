@@ -288,3 +288,21 @@ def test_transpose_pass_shapes(pkg, cols, nnz):
     np.testing.assert_array_equal(cp, np.concatenate([[0], np.cumsum(np.bincount(col, minlength=cols))]).astype(np.uint64))
     np.testing.assert_array_equal(ri, np.repeat(np.arange(rows, dtype=np.uint32), lens)[order])
     np.testing.assert_array_equal(v.view(np.uint32), val[order].view(np.uint32))
+
+
+@pytest.mark.parametrize("cols", [1, 2, 200, 300, 65_536, 16_777_217])
+def test_transpose_pass_counts(pkg, cols):
+    """One to four passes and last digits of 0 to 8 bits, a third of the entries in one
+    column, which stay in row order: bit-exact."""
+    rng = np.random.default_rng(cols)
+    lens = rng.integers(0, 9, 3001)
+    lens[1000] = 4096
+    col = rng.integers(0, cols, lens.sum()).astype(np.uint32)
+    col[::3] = cols - 1
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.uint64)
+    val = rng.standard_normal(len(col)).astype(np.float32)
+    cp, ri, v = pkg.transpose(rp, col, val, cols)
+    order = np.argsort(col, kind="stable")
+    np.testing.assert_array_equal(cp, np.concatenate([[0], np.cumsum(np.bincount(col, minlength=cols))]).astype(np.uint64))
+    np.testing.assert_array_equal(ri, np.repeat(np.arange(3001, dtype=np.uint32), lens)[order])
+    np.testing.assert_array_equal(v.view(np.uint32), val[order].view(np.uint32))
