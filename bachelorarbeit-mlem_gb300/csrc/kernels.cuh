@@ -30,10 +30,11 @@ struct EpiArgs {
     float* fwproj = nullptr;      // Correl: optional copy of the projection
     float* f = nullptr;           // Update: image, updated in place
     const float* norm = nullptr;  // Update
-    // csr-vector (DIRECT), D16 and merge-path row kernels: launched so that they may start while
-    // the previous kernel of the stream drains.  Set inside an MLEM loop: 8.15 ->
-    // 7.34 us per iteration on the 2-D ring, 43.9 -> 43.2 us with 6 M nonzeros,
-    // 4.26 -> 4.20 ms on the 3-D mid matrix; a single projection only pays for the
+    // csr-vector (DIRECT), D16 and merge-path row kernels (the scatter and the
+    // update after it likewise): launched so that they may start while the
+    // previous kernel of the stream drains.  Set inside an MLEM loop: 8.15 -> 7.34
+    // us per iteration on the 2-D ring, 43.9 -> 43.2 us with 6 M nonzeros, 4.26 ->
+    // 4.20 ms on the 3-D mid matrix; a single projection only pays for the
     // attribute (0.4 us of host time).
     bool overlap = false;
     // symmetry-compressed kernels only: also write the results in orbit
@@ -89,8 +90,8 @@ void launch_csr_tma(const DevCsr& op, const float* x, const EpiArgs& epi, uint32
 void launch_scatter_tma(const DevCsr& A, const float* ratio, float* bp, uint32_t* err, L2Window win,
                         cudaStream_t s);
 // bp[idx] += val * ratio[row] over the rows of A (calcBwProj_none_trans, kernel.cu:165-177);
-// lanes per row 8/16/32, unroll = entries per lane in flight (2 or 4).
-void launch_scatter(const DevCsr& A, const float* ratio, float* bp, int lanes, int unroll, L2Window win,
+// lanes per row 8/16/32, unroll = entries per lane in flight (2 or 4); overlap as in EpiArgs.
+void launch_scatter(const DevCsr& A, const float* ratio, float* bp, int lanes, int unroll, bool overlap, L2Window win,
                     cudaStream_t s);
 // One pass over A: sum = A[r,:]·x, ratio = g[r]/sum, bp[idx] += val*ratio.
 void launch_fused_fp_scatter(const DevCsr& A, const float* x, const int32_t* g, float* bp,
@@ -191,9 +192,9 @@ void launch_merge_spmv(const DevCsr& op, const MergePlan& plan, const float* x,
                        const EpiArgs& epi, L2Window win, cudaStream_t s);
 
 // ------------------------------------------------------------- transpose.cu
-// Stable counting sort by column of A (f32 values) -> Aᵀ with u32 row ids.
 // Zeroes the entries of idx and val past nnz (16-byte loads may touch them).
 void zero_padding(const DevCsr& c, cudaStream_t s);
+// Stable counting sort by column of A (f32 values) -> Aᵀ with u32 row ids.
 void transpose_device(const DevCsr& A, DevCsr& AT, cudaStream_t s);
 // norm[c] = (float) Σ (double) val over column c.
 void colsum_from_transpose(const DevCsr& AT, float* norm, cudaStream_t s);

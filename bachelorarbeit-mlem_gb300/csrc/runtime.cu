@@ -185,9 +185,9 @@ int scatter_lanes(mlem_matrix* m) {
         MLEM_CUDA(cudaEventCreate(&e1));
         for (int lanes : {8, 16, 32})
             for (int u : {2, 4}) {
-                launch_scatter(A, r, bp, lanes, u, {}, s);
+                launch_scatter(A, r, bp, lanes, u, false, {}, s);
                 MLEM_CUDA(cudaEventRecord(e0, s));
-                for (int q = 0; q < 2; ++q) launch_scatter(A, r, bp, lanes, u, {}, s);
+                for (int q = 0; q < 2; ++q) launch_scatter(A, r, bp, lanes, u, false, {}, s);
                 MLEM_CUDA(cudaEventRecord(e1, s));
                 MLEM_CUDA(cudaEventSynchronize(e1));
                 float ms = 0.f;
@@ -777,7 +777,7 @@ void enqueue_iteration(mlem_matrix* m, const mlem_run_opts& o, cudaStream_t s, d
                 ensure_workspace(m);
                 launch_scatter_tma(A, w.ratio, w.bp, w.err, wr, s);
             }
-            else launch_scatter(A, w.ratio, w.bp, sl, m->scatter_unroll, wr, s);
+            else launch_scatter(A, w.ratio, w.bp, sl, m->scatter_unroll, true, wr, s);
             launch_update_zero(w.f, w.bp, m->norm, A.ncols, s);
         }
         if (timer) timer->record(s);
@@ -1612,7 +1612,7 @@ mlem_status mlem_back_project(mlem_matrix* m, const float* ratio_dev, float* bp_
         } else {
             MLEM_CUDA(cudaMemsetAsync(out, 0, sizeof(float) * m->A.ncols, s));
             const int sl = scatter_lanes(m);  // sets m->scatter_unroll on the first call
-            launch_scatter(m->A, r, out, sl, m->scatter_unroll, {}, s);
+            launch_scatter(m->A, r, out, sl, m->scatter_unroll, false, {}, s);
         }
         if (perm) cols_out(m, bp_dev, out, s);
     });

@@ -328,13 +328,16 @@ __global__ void __launch_bounds__(256)
 k_scatter(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ idx,
           const V* __restrict__ val, const float* __restrict__ ratio, uint32_t nrows,
           float* __restrict__ bp) {
+    grid_release();
     const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t row = gt / LPR;
     const int sub = threadIdx.x & (LPR - 1);
-    if (row >= nrows) return;
-    // the ratio and the row bounds are loaded together (one round trip, not two)
-    const float r = ratio[row];
-    const uint64_t s = rowptr[row], t = rowptr[row + 1];
+    const bool live = row < nrows;
+    // the ratio and the row bounds are in flight together (one round trip, not two)
+    const uint64_t s = live ? rowptr[row] : 0, t = live ? rowptr[row + 1] : 0;
+    grid_wait();
+    if (!live) return;
+    const float r = ld_after(ratio + row);
     if (r == 0.0f) return;  // adds of val*0 leave bp unchanged
     scatter_row<V, LPR, U>(idx, val, s, t, sub, r, bp);
 }
@@ -413,6 +416,7 @@ k_fused_rescan(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__
                const V* __restrict__ val, const float* __restrict__ x, uint32_t nrows,
                const int32_t* __restrict__ g, float* __restrict__ bp, float* __restrict__ fwproj,
                const uint32_t* __restrict__ order) {
+    grid_release();  // for the update; launched plainly itself (with loads that may follow a wait: 12 GB class 1% slower)
     const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t k = gt / LPR;
     const int sub = threadIdx.x & (LPR - 1);
@@ -437,6 +441,8 @@ k_fused_rescan(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__
 
 __global__ void k_update_zero(float* __restrict__ f, float* __restrict__ bp,
                               const float* __restrict__ norm, uint32_t n) {
+    grid_release();
+    grid_wait();
     for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
         const float b = bp[c];
         bp[c] = 0.0f;
@@ -452,6 +458,8 @@ __global__ void k_update_zero4(float* __restrict__ f, float* __restrict__ bp, co
     float4* f4 = reinterpret_cast<float4*>(f);
     float4* b4 = reinterpret_cast<float4*>(bp);
     const float4* m4 = reinterpret_cast<const float4*>(norm);
+    grid_release();
+    grid_wait();
     for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n4; c += gridDim.x * blockDim.x) {
         const float4 b = b4[c];
         const float4 x = f4[c];
@@ -621,13 +629,13 @@ void csrvec_dispatch_lanes(const DevCsr& op, const float* x, const EpiArgs& e, i
 }
 
 template <typename V>
-void scatter_dispatch(const DevCsr& A, const float* ratio, float* bp, int lanes, int unroll, L2Window win,
-                      cudaStream_t s) {
+void scatter_dispatch(const DevCsr& A, const float* ratio, float* bp, int lanes, int unroll, bool overlap,
+                      L2Window win, cudaStream_t s) {
     const V* val = static_cast<const V*>(A.val);
     auto go = [&](auto kern, int lpr) {
         const uint64_t threads = (uint64_t)A.nrows * lpr;
-        launch_ex(kern, dim3(ceil_div_u(threads, 256)), dim3(256), 0, s, win, A.rowptr, A.idx, val,
-                  ratio, A.nrows, bp);
+        launch_attrs(overlap, kern, dim3(ceil_div_u(threads, 256)), dim3(256), 0, s, win, A.rowptr, A.idx, val,
+                     ratio, A.nrows, bp);
     };
     if (unroll >= 4) {
         if (lanes >= 32) go(k_scatter<V, 32, 4>, 32);
@@ -686,13 +694,13 @@ void launch_csrvec_pipe(const DevCsr& op, const float* x, const EpiArgs& epi, in
     }
 }
 
-void launch_scatter(const DevCsr& A, const float* ratio, float* bp, int lanes, int unroll, L2Window win,
+void launch_scatter(const DevCsr& A, const float* ratio, float* bp, int lanes, int unroll, bool overlap, L2Window win,
                     cudaStream_t s) {
     if (A.nrows == 0) return;
     switch (A.vt) {
-        case MLEM_VAL_F32: scatter_dispatch<float>(A, ratio, bp, lanes, unroll, win, s); break;
-        case MLEM_VAL_F16: scatter_dispatch<__half>(A, ratio, bp, lanes, unroll, win, s); break;
-        default: scatter_dispatch<__nv_bfloat16>(A, ratio, bp, lanes, unroll, win, s);
+        case MLEM_VAL_F32: scatter_dispatch<float>(A, ratio, bp, lanes, unroll, overlap, win, s); break;
+        case MLEM_VAL_F16: scatter_dispatch<__half>(A, ratio, bp, lanes, unroll, overlap, win, s); break;
+        default: scatter_dispatch<__nv_bfloat16>(A, ratio, bp, lanes, unroll, overlap, win, s);
     }
 }
 
@@ -761,12 +769,11 @@ void launch_update_zero(float* f, float* bp, const float* norm, uint32_t n, cuda
                            reinterpret_cast<uintptr_t>(norm)) & 15u) == 0;
     if (aligned) {
         const unsigned grid = std::max(1u, std::min<unsigned>(ceil_div_u(n >> 2, 256), 152u * 16u));
-        k_update_zero4<<<grid, 256, 0, s>>>(f, bp, norm, n);
+        launch_attrs(true, k_update_zero4, dim3(grid), dim3(256), 0, s, L2Window{}, f, bp, norm, n);
     } else {
         const unsigned grid = std::min<unsigned>(ceil_div_u(n, 256), 152u * 16u);
-        k_update_zero<<<grid, 256, 0, s>>>(f, bp, norm, n);
+        launch_attrs(true, k_update_zero, dim3(grid), dim3(256), 0, s, L2Window{}, f, bp, norm, n);
     }
-    MLEM_LAUNCHED();
 }
 
 void launch_loglik(const int32_t* g, const float* fwproj, uint32_t rows, double* part,
