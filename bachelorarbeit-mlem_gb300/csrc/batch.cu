@@ -6,14 +6,28 @@
 // every slot with iterations left): a row is handled by a segment of W lanes
 // of a warp (32/W rows per warp); each lane owns 4 instances of a nonzero and
 // reads their image entries with one 16-byte load, so W/4 lanes cover a
-// nonzero and a segment takes 4 nonzeros per gather instruction.  The
-// segment's lanes load the row 32 entries at a time (coalesced) and broadcast
-// them with shuffles.
+// nonzero and a segment takes 4 nonzeros per gather instruction.
 //
-// Every instance sums its row in 4 chains — nonzero k of the row goes to
-// chain k mod 4, each chain a sequential FMA chain in k order — combined as
-// (c0 + c1) + (c2 + c3).  That order depends on neither W nor BT nor the slot,
-// so an instance gives the same bits alone and in a full batch, in any tile.
+// Every instance sums its row in 4 chains: the row's 4-entry vectors (aligned
+// to multiples of 4 entries of the matrix) go to the chains in turn, each chain
+// a sequential FMA chain in entry order, combined as (c0 + c1) + (c2 + c3).  The
+// W/4 lanes of a chain load its vectors of indices and values themselves (one
+// request each per instruction).  That order depends on neither W nor BT nor
+// the slot, so an instance gives the same bits alone and in a full batch, in
+// any tile.
+//
+// What bounds it: a nonzero's gather of the slots' state, one 128-byte line
+// with 32 slots, and with it the L1 data pipe.  Handing 32 coalesced entries
+// round with shuffles, as an earlier form did, put 2 shuffles on that pipe for
+// every 4 nonzeros: one iteration of the 3-D mid matrix with 4 / 8 / 16 / 32
+// slots 1.28 / 1.38 / 2.01 / 3.25 -> 1.19 / 1.35 / 1.88 / 3.12 ms (FP16 values 1.28 /
+// 1.36 / 1.97 / 3.22 -> 1.14 / 1.30 / 1.87 / 2.98), of a matrix of 6 M nonzeros 0.134 /
+// 0.136 / 0.200 / 0.310 -> 0.131 / 0.136 / 0.181 / 0.278 ms; 24 sinograms of 5 to 20
+// iterations on the mid matrix 54.5 -> 51.4 ms.  6 blocks per SM (40
+// registers), one vector at a time; measured and not kept, 16 / 32 slots on the
+// mid matrix: 8 blocks (32 registers, spills) 2.41 / 3.76, 5 blocks 1.94 / 3.25,
+// the next vector loaded before the gathers 2.24 / 3.83 (5 blocks 1.99 / 3.31),
+// two vectors unrolled with 5 and 4 blocks 1.95 / 3.28 and 2.02 / 3.38 ms.
 //
 // Per-slot iteration counters live on the device (remaining[b]); an
 // iteration is FP, BP+update and a counter tick, replayable as one CUDA
@@ -33,9 +47,16 @@ namespace {
 // right only when no block of the same launch writes it; the persistent loop
 // below, whose phases write what the next phase gathers, uses plain loads.
 template <bool NC>
-__device__ __forceinline__ float4 load_state(const float* p) {
+__device__ __forceinline__ float4 load_state(const char* p) {
     if (NC) return __ldg(reinterpret_cast<const float4*>(p));
     return *reinterpret_cast<const float4*>(p);
+}
+
+__device__ __forceinline__ void fma_state(float4& acc, float v, const float4& x) {
+    acc.x = fmaf(v, x.x, acc.x);
+    acc.y = fmaf(v, x.y, acc.y);
+    acc.z = fmaf(v, x.z, acc.z);
+    acc.w = fmaf(v, x.w, acc.w);
 }
 
 template <typename V, int W, bool NC = true>
@@ -43,86 +64,52 @@ __device__ __forceinline__ void batch_rows(const uint64_t* __restrict__ rowptr, 
                                            const V* __restrict__ val, const float* x, uint32_t BT, uint32_t na,
                                            uint32_t row, bool ok, int lane, float4& acc) {
     constexpr int LPN = W / 4;  // lanes per nonzero
-    constexpr int E = 32 / W;   // entries per lane per 32-entry chunk
-    const int sl = lane % W, chain = sl / LPN, seg0 = lane - sl;
+    const int sl = lane % W, chain = sl / LPN;
     const uint32_t q4 = (sl % LPN) * 4;
     // lanes of slots that are not read repeat those of slot 0 (no bytes of their own)
-    const float* xq = x + (q4 < na ? q4 : 0);
+    const char* xq = reinterpret_cast<const char*>(x + (q4 < na ? q4 : 0));
+    const uint32_t stride = BT * (uint32_t)sizeof(float);
     uint64_t s = 0, t = 0;
     if (ok) {
         s = rowptr[row];
         t = rowptr[row + 1];
     }
-    // the warp runs as many chunks as its longest row needs (shuffles stay
-    // converged); from 16 slots on without checks as long as its shortest row is
-    // not used up (3-D mid matrix, FP32, both projections: 16 slots 2.71 -> 2.61
-    // ms, 32 slots 4.23 -> 4.03; with fewer slots, several entries per lane, the
-    // second loop's registers cost more than the checks)
-    uint32_t chunks = (uint32_t)((t - s + 31) >> 5), whole = W >= 16 ? (uint32_t)((t - s) >> 5) : 0;
+    if (s < t) {
+        const uint64_t v0 = s >> 2;
+        const uint4* ip = reinterpret_cast<const uint4*>(idx) + v0;
+        const V* vp = val + 4 * v0;
+        const uint32_t lo = (uint32_t)(s & 3), hi = (uint32_t)(t - 4 * v0);  // the row's entries, relative to 4 v0
+        auto part = [&](uint32_t v) {  // a vector that is not all the row's
+            const uint4 c = ld_stream(ip + v);
+            float a[4];
+            Val4<V>::load(vp, v, a);
+            const uint32_t cs[4] = {c.x, c.y, c.z, c.w};
 #pragma unroll
-    for (int o = W; o < 32; o <<= 1) {
-        chunks = max(chunks, __shfl_xor_sync(0xffffffffu, chunks, o));
-        if (W >= 16) whole = min(whole, __shfl_xor_sync(0xffffffffu, whole, o));
+            for (int k = 0; k < 4; ++k)
+                if (4 * v + k >= lo && 4 * v + k < hi)
+                    fma_state(acc, a[k], load_state<NC>(xq + (uint64_t)cs[k] * stride));
+        };
+        const uint32_t whole = hi >> 2;
+        uint32_t v = chain;
+        if (v == 0 && lo) {
+            part(0);
+            v = 4;
+        }
+#pragma unroll 1
+        for (; v < whole; v += 4) {
+            const uint4 c = ld_stream(ip + v);
+            float a[4];
+            Val4<V>::load(vp, v, a);
+            const uint32_t cs[4] = {c.x, c.y, c.z, c.w};
+            float4 xv[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) xv[k] = load_state<NC>(xq + (uint64_t)cs[k] * stride);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) fma_state(acc, a[k], xv[k]);
+        }
+        if (v == whole && (hi & 3)) part(v);
     }
-    const uint32_t* ip = idx + s + sl;
-    const V* vp = val + s + sl;
-    for (uint32_t ch = 0; ch < whole; ++ch) {
-        uint32_t c[E];
-        float v[E];
-#pragma unroll
-        for (int i = 0; i < E; ++i) {
-            c[i] = ld_stream(ip + i * W);
-            v[i] = Val4<V>::one(vp, i * W);
-        }
-        ip += 32;
-        vp += 32;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int src = seg0 + chain + (4 * q) % W;
-            const uint32_t ck = __shfl_sync(0xffffffffu, c[(4 * q) / W], src);
-            const float vk = __shfl_sync(0xffffffffu, v[(4 * q) / W], src);
-            const float4 xv = load_state<NC>(xq + (uint64_t)ck * BT);
-            acc.x = fmaf(vk, xv.x, acc.x);
-            acc.y = fmaf(vk, xv.y, acc.y);
-            acc.z = fmaf(vk, xv.z, acc.z);
-            acc.w = fmaf(vk, xv.w, acc.w);
-        }
-    }
-    for (uint32_t ch = whole; ch < chunks; ++ch) {
-        const uint64_t base = s + 32ull * ch;
-        // entry base + sl + i*W sits in slot i of lane sl
-        uint32_t c[E];
-        float v[E];
-#pragma unroll
-        for (int i = 0; i < E; ++i) {
-            const uint64_t e = base + sl + (uint64_t)i * W;
-            c[i] = 0;
-            v[i] = 0.f;
-            if (e < t) {
-                c[i] = ld_stream(idx + e);
-                v[i] = Val4<V>::one(val, e);
-            }
-        }
-        // entries of this row left in the chunk, less the chain offset
-        const int64_t left = (int64_t)t - (int64_t)base;
-        const int r = (int)(left < 0 ? 0 : left > 32 ? 32 : left) - chain;
-        // trip q: nonzero k = 4q + chain of the chunk, held by lane k % W in
-        // slot k / W = 4q / W; k % W = 4q % W + chain since chain < 4 <= W
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            if (W == 32 && 4 * q >= r + chain) break;  // one row per warp: uniform
-            const int src = seg0 + chain + (4 * q) % W;
-            const uint32_t ck = __shfl_sync(0xffffffffu, c[(4 * q) / W], src);
-            const float vk = __shfl_sync(0xffffffffu, v[(4 * q) / W], src);
-            if (4 * q < r) {
-                const float4 xv = load_state<NC>(xq + (uint64_t)ck * BT);
-                acc.x = fmaf(vk, xv.x, acc.x);
-                acc.y = fmaf(vk, xv.y, acc.y);
-                acc.z = fmaf(vk, xv.z, acc.z);
-                acc.w = fmaf(vk, xv.w, acc.w);
-            }
-        }
-    }
+    __syncwarp();
     // (c0 + c1) + (c2 + c3): chains sit LPN lanes apart inside the segment
 #pragma unroll
     for (int o = LPN; o < W; o <<= 1) {
@@ -142,7 +129,7 @@ __device__ __forceinline__ float update1(float f, float acc, float n) {
 
 // ratio[row*BT + b] = g/(A f)_b for the first W slots.
 template <typename V, int W>
-__global__ void __launch_bounds__(256, W >= 16 ? 6 : W == 8 ? 5 : 4)
+__global__ void __launch_bounds__(256, 6)
 k_batch_fp(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ idx,
            const V* __restrict__ val, const float* __restrict__ f, uint32_t rows, uint32_t BT, uint32_t na,
            const int32_t* __restrict__ g, float* __restrict__ ratio) {
@@ -164,7 +151,7 @@ k_batch_fp(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ idx
 
 // f[c*BT + b] = f·(Aᵀ ratio)_b / norm[c] for the slots b < W with iterations left.
 template <typename V, int W>
-__global__ void __launch_bounds__(256, W >= 16 ? 6 : W == 8 ? 5 : 4)
+__global__ void __launch_bounds__(256, 6)
 k_batch_bp(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ idx,
            const V* __restrict__ val, const float* __restrict__ ratio, uint32_t cols, uint32_t BT, uint32_t na,
            const float* __restrict__ norm, const uint32_t* __restrict__ remaining,
@@ -250,7 +237,7 @@ __global__ void k_batch_tick(uint32_t* remaining, uint32_t BT) {
 // chains, same order), so an instance's bits do not depend on which kernel
 // form runs it.
 template <typename V, int W>
-__global__ void __launch_bounds__(256, W == 32 ? 8 : 6)
+__global__ void __launch_bounds__(256, 6)
 k_batch_loop(const uint64_t* __restrict__ rp, const uint32_t* __restrict__ ix, const V* __restrict__ vl,
              uint32_t rows, const uint64_t* __restrict__ rpT, const uint32_t* __restrict__ ixT,
              const V* __restrict__ vlT, uint32_t cols, const float* __restrict__ norm, uint32_t BT,
@@ -320,9 +307,15 @@ void sc_bt(const DevCsr& A, const BatchArgs& b, float* bp, cudaStream_t s) {
     MLEM_LAUNCHED();
 }
 
+// Lanes per row for a launch of W slots: a matrix whose rows all fit the GPU at
+// once with 8 lanes each (48 warps per SM) takes no fewer, since only the
+// length of a row's chains counts there (1,770 rows, one iteration: 4 lanes 14.4,
+// 8 lanes 12.4 us; 108,000 / 663,000 rows: 4 lanes 5% / 12% faster).
+int row_lanes(uint32_t w, uint32_t rows) { return w == 4 && rows <= 152u * 48u * 4u ? 8 : (int)w; }
+
 template <typename V>
 void fp_v(const DevCsr& A, const BatchArgs& b, L2Window win, cudaStream_t s) {
-    switch (b.width()) {
+    switch (row_lanes(b.width(), A.nrows)) {
         case 4: fp_w<4, V>(A, b, win, s); break;
         case 8: fp_w<8, V>(A, b, win, s); break;
         case 16: fp_w<16, V>(A, b, win, s); break;
@@ -331,7 +324,7 @@ void fp_v(const DevCsr& A, const BatchArgs& b, L2Window win, cudaStream_t s) {
 }
 template <typename V>
 void bp_v(const DevCsr& AT, const float* norm, const BatchArgs& b, L2Window win, cudaStream_t s) {
-    switch (b.width()) {
+    switch (row_lanes(b.width(), AT.nrows)) {
         case 4: bp_w<4, V>(AT, norm, b, win, s); break;
         case 8: bp_w<8, V>(AT, norm, b, win, s); break;
         case 16: bp_w<16, V>(AT, norm, b, win, s); break;
