@@ -181,15 +181,19 @@ struct MergePlan {
     bool rows_kernel = false;
     bool whole = false;          // row kernel: tiles of whole rows, no carries and no fix-up launch
     int lanes = 16;              // row kernel: lanes per row (8 or 16)
+    int d16_u = 0;               // the operand's delta-coded copy is faster: its vectors per lane in flight
     int rows_u = 1;              // row kernel: vectors per lane in flight (1: 16 blocks per SM, 2: 12)
     void release();
 };
 // Builds the tile partition of `op` for a section size (device allocations).
 void merge_plan_build(const DevCsr& op, uint32_t secsize, MergePlan& plan, cudaStream_t s);
 // Merge-path product: one launch where the plan's tiles hold whole rows, else
-// two (deterministic carry fix-up).
+// two (deterministic carry fix-up).  launch_merge_d16 (spmv_d16.cu): the same
+// over the operand's delta-coded copy, for plans of whole rows.
 void launch_merge_spmv(const DevCsr& op, const MergePlan& plan, const float* x,
                        const EpiArgs& epi, L2Window win, cudaStream_t s);
+void launch_merge_d16(const DevCsr& op, const MergePlan& plan, const float* x, const EpiArgs& epi, int unroll,
+                      L2Window win, cudaStream_t s);
 
 // ------------------------------------------------------------- transpose.cu
 // Zeroes the entries of idx and val past nnz (16-byte loads may touch them).

@@ -334,65 +334,6 @@ FusedForm fused_form(mlem_matrix* m, const mlem_run_opts& o) {
     return best;
 }
 
-const MergePlan& merge_plan(mlem_matrix* m, bool transposed, uint32_t secsize) {
-    auto& plans = transposed ? m->plan_AT : m->plan_A;
-    auto it = plans.find(secsize);
-    if (it != plans.end()) return it->second;
-    MergePlan p;
-    const DevCsr& op = transposed ? m->AT : m->A;
-    cudaStream_t s = m->stream;
-    merge_plan_build(op, secsize, p, s);
-    MLEM_CUDA(cudaStreamSynchronize(s));
-    if (p.rows_kernel && op.nnz) {
-        // one or two vectors per lane in flight in the row kernel (16 or 12 blocks
-        // per SM), timed with a Raw epilogue on an image of ones; same sums
-        float *x = nullptr, *y = nullptr;
-        cudaEvent_t e0 = nullptr, e1 = nullptr;
-        float best = 1e30f;
-        int pick = 1;
-        try {
-            MLEM_CUDA(cudaMalloc(&x, sizeof(float) * std::max<uint32_t>(op.ncols, 1)));
-            MLEM_CUDA(cudaMalloc(&y, sizeof(float) * std::max<uint32_t>(op.nrows, 1)));
-            std::vector<float> ones(std::max<uint32_t>(op.ncols, 1), 1.0f);
-            MLEM_CUDA(cudaMemcpyAsync(x, ones.data(), sizeof(float) * ones.size(), cudaMemcpyHostToDevice, s));
-            MLEM_CUDA(cudaEventCreate(&e0));
-            MLEM_CUDA(cudaEventCreate(&e1));
-            EpiArgs e;
-            e.kind = Epi::Raw;
-            e.out = y;
-            for (int u : {1, 2}) {
-                p.rows_u = u;
-                launch_merge_spmv(op, p, x, e, L2Window{}, s);
-                MLEM_CUDA(cudaEventRecord(e0, s));
-                for (int q = 0; q < 2; ++q) launch_merge_spmv(op, p, x, e, L2Window{}, s);
-                MLEM_CUDA(cudaEventRecord(e1, s));
-                MLEM_CUDA(cudaEventSynchronize(e1));
-                float ms = 0.f;
-                MLEM_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-                if (ms < best) {
-                    best = ms;
-                    pick = u;
-                }
-            }
-        } catch (...) {
-            cudaStreamSynchronize(s);
-            cudaFree(x);
-            cudaFree(y);
-            if (e0) cudaEventDestroy(e0);
-            if (e1) cudaEventDestroy(e1);
-            p.release();
-            throw;
-        }
-        cudaFree(x);
-        cudaFree(y);
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        p.rows_u = pick;
-    }
-    return plans.emplace(secsize, p).first->second;
-}
-
-
 void check_run_opts(const mlem_matrix* m, const mlem_run_opts& o) {
     MLEM_REQUIRE(o.kernel <= MLEM_KERNEL_SYM, MLEM_EINVAL,
                  "kernel must be 0 direct, 1 tma, 2 persistent, 3 auto, 4 d16, 5 ilv, 6 ordered or 7 sym");
@@ -478,6 +419,85 @@ static bool may_copy_d16(const mlem_matrix* m, const DevCsr& op) {
     MLEM_CUDA(cudaMemGetInfo(&avail, &total));
     const uint64_t stream = op.nnz * (4 + val_bytes(op.vt)), copy = op.nnz * (2 + val_bytes(op.vt)) / 4 * 5;
     return stream > (uint64_t)l2 && copy <= avail / 4;
+}
+
+// Merge-path tiles of an operand for a section size, built on first use: one or
+// two vectors per lane in flight in the row kernel (16 or 12 blocks per SM; same
+// sums), and for tiles of whole rows the delta-coded copy where there is one or
+// may_copy_d16 allows one, timed with a Raw epilogue on a constant image.
+const MergePlan& merge_plan(mlem_matrix* m, bool transposed, uint32_t secsize) {
+    auto& plans = transposed ? m->plan_AT : m->plan_A;
+    auto it = plans.find(secsize);
+    if (it != plans.end()) return it->second;
+    MergePlan p;
+    DevCsr& op = transposed ? m->AT : m->A;
+    cudaStream_t s = m->stream;
+    merge_plan_build(op, secsize, p, s);
+    MLEM_CUDA(cudaStreamSynchronize(s));
+    if (p.rows_kernel && op.nnz) {
+        float *x = nullptr, *y = nullptr;
+        cudaEvent_t e0 = nullptr, e1 = nullptr;
+        float best = 1e30f;
+        try {
+            MLEM_CUDA(cudaMalloc(&x, sizeof(float) * std::max<uint32_t>(op.ncols, 1)));
+            MLEM_CUDA(cudaMalloc(&y, sizeof(float) * std::max<uint32_t>(op.nrows, 1)));
+            MLEM_CUDA(cudaMemsetAsync(x, 0x3f, sizeof(float) * std::max<uint32_t>(op.ncols, 1), s));
+            MLEM_CUDA(cudaEventCreate(&e0));
+            MLEM_CUDA(cudaEventCreate(&e1));
+            EpiArgs e;
+            e.kind = Epi::Raw;
+            e.out = y;
+            auto faster = [&](auto launch) {  // than the best so far
+                launch();
+                MLEM_CUDA(cudaEventRecord(e0, s));
+                for (int q = 0; q < 2; ++q) launch();
+                MLEM_CUDA(cudaEventRecord(e1, s));
+                MLEM_CUDA(cudaEventSynchronize(e1));
+                float ms = 0.f;
+                MLEM_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+                if (ms >= best) return false;
+                best = ms;
+                return true;
+            };
+            int pick = 1;
+            for (int u : {1, 2}) {
+                p.rows_u = u;
+                if (faster([&] { launch_merge_spmv(op, p, x, e, L2Window{}, s); })) pick = u;
+            }
+            p.rows_u = pick;
+            bool made = false;
+            if (p.whole && !op.d16_lost && may_copy_d16(m, op)) {
+                try {
+                    made = op.d16_tuned = build_d16(op, false, s);
+                } catch (const Error& err) {  // no room after all
+                    if (err.code != MLEM_ENOMEM) throw;
+                    cudaGetLastError();
+                }
+                op.d16_lost = !made;
+            }
+            if (p.whole && op.d16)
+                for (int u : {1, 2})
+                    if (faster([&] { launch_merge_d16(op, p, x, e, u, L2Window{}, s); })) p.d16_u = u;
+            if (made && !p.d16_u) {
+                free_d16(op);
+                op.d16_tuned = false;
+                op.d16_lost = true;
+            }
+        } catch (...) {
+            cudaStreamSynchronize(s);
+            cudaFree(x);
+            cudaFree(y);
+            if (e0) cudaEventDestroy(e0);
+            if (e1) cudaEventDestroy(e1);
+            p.release();
+            throw;
+        }
+        cudaFree(x);
+        cudaFree(y);
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+    }
+    return plans.emplace(secsize, p).first->second;
 }
 
 // Times the candidate configurations on the operand itself (Raw epilogue into
@@ -682,7 +702,12 @@ void project(mlem_matrix* m, bool transposed, const float* x, const EpiArgs& e, 
              L2Window win, cudaStream_t s) {
     const DevCsr& op = transposed ? m->AT : m->A;
     if (o.spmv == MLEM_SPMV_MERGE) {
-        launch_merge_spmv(op, merge_plan(m, transposed, transposed ? o.secsize_bp : o.secsize_fp), x, e, win, s);
+        const MergePlan& p = merge_plan(m, transposed, transposed ? o.secsize_bp : o.secsize_fp);
+        int u = 0;  // vectors in flight over the delta-coded copy; 0: the CSR arrays
+        if (o.kernel == MLEM_KERNEL_AUTO) u = p.d16_u;
+        else if (o.kernel == MLEM_KERNEL_D16 && p.whole && op.d16 && !op.d16_tuned) u = o.unroll == 1 ? 1 : 2;
+        if (u) launch_merge_d16(op, p, x, e, u, win, s);
+        else launch_merge_spmv(op, p, x, e, win, s);
         return;
     }
     launch_cfg(m, op, x, e, resolve_cfg(m, transposed, o), win, s);

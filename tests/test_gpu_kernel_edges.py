@@ -246,6 +246,51 @@ def test_merge_tiles_of_whole_rows(pkg, cuda, vt, mean, longest):
     m.close()
 
 
+@pytest.mark.parametrize("vt", [0, 1, 2])
+@pytest.mark.parametrize("long_rows", [True, False])
+@pytest.mark.parametrize("unroll", [1, 2])
+def test_merge_tiles_delta_coded(pkg, cuda, vt, long_rows, unroll):
+    """Merge-path tiles over delta-coded rows, among runs of empty rows longer than a
+    block, against FP64, and against the CSR tiles where x holds infinities and NaN."""
+    cols = 600_000
+    rng, rp, col, val = d16_rows(37, cols, long_rows)
+    gap = 150 if long_rows else 1000
+    at = (len(rp) - 1) // 2
+    rp = np.concatenate([np.zeros(gap // 2, np.uint64), rp[:at + 1], np.repeat(rp[at], gap), rp[at + 1:],
+                         np.repeat(rp[-1], gap // 5)])
+    rows = len(rp) - 1
+    lens = np.diff(rp.astype(np.int64))
+    rid, v = np.repeat(np.arange(rows), lens), stored(cuda, val, vt)
+    m = pkg.Matrix.from_csr(rp, col, val, cols, value_type=vt, compress=True)
+    x = rng.uniform(0.5, 1.5, cols).astype(np.float32)
+    r = rng.uniform(0.5, 1.5, rows).astype(np.float32)
+    g = cuda.from_numpy(rng.integers(0, 50, rows).astype(np.int32)).cuda()
+
+    def project(x, r, **kw):
+        dx, dr = cuda.from_numpy(x).cuda(), cuda.from_numpy(r).cuda()
+        ratio, fp, bp = (cuda.full((n,), -1.0, device="cuda") for n in (rows, rows, cols))
+        kw = dict(kw, spmv=pkg.SPMV_MERGE, secsize_fp=64, secsize_bp=64)
+        m.forward_project(dx.data_ptr(), g.data_ptr(), ratio.data_ptr(), fp.data_ptr(), **kw)
+        m.back_project(dr.data_ptr(), bp.data_ptr(), **kw)
+        return fp.cpu().numpy(), bp.cpu().numpy(), ratio.cpu().numpy()
+
+    fp, bp, ratio = project(x, r, kernel=pkg.KERNEL_D16, unroll=unroll)
+    want = np.bincount(rid, weights=v * x[col].astype(np.float64), minlength=rows)
+    assert np.all(np.abs(fp - want) <= (lens + 2) * 2.0**-24 * want)
+    gs = g.cpu().numpy().astype(np.float32)
+    np.testing.assert_array_equal(ratio, np.where(fp != 0, gs / np.where(fp != 0, fp, 1), 0))
+    want = np.bincount(col, weights=v * r[rid].astype(np.float64), minlength=cols)
+    assert np.all(np.abs(bp - want) <= (np.bincount(col, minlength=cols) + 2) * 2.0**-24 * want)
+    x[rng.choice(cols, 4000, replace=False)] = np.inf
+    x[rng.choice(cols, 4000, replace=False)] = np.nan
+    r[rng.choice(rows, 8, replace=False)] = -np.inf
+    for a, b in zip(project(x, r, kernel=pkg.KERNEL_D16, unroll=unroll), project(x, r, kernel=pkg.KERNEL_DIRECT)):
+        np.testing.assert_array_equal(np.isnan(a), np.isnan(b))
+        np.testing.assert_array_equal(a[np.isinf(b)], b[np.isinf(b)])
+        np.testing.assert_array_equal(np.isfinite(a), np.isfinite(b))
+    m.close()
+
+
 @pytest.mark.parametrize("vt", [0, 1])
 def test_batch_slots_and_row_lengths(pkg, O, cuda, vt):
     """Batches that leave slots of every width unused, on rows around the 32 entries
