@@ -289,7 +289,7 @@ __device__ __forceinline__ float group_part_dot(const uint4* __restrict__ idx4, 
                                                 const float* __restrict__ x, uint32_t s, uint32_t t, int sub) {
     // s, t: first and last entry + 1, relative to a multiple of 4 that idx4 and val start at
     const uint32_t v1 = (t + 3) >> 2;
-    float acc = 0.f;
+    float acc[2] = {0.f, 0.f};  // even and odd entries: as many chains with 8 lanes as with 16 and one sum
     // U = 2: two vectors per lane in flight; the FMAs still run in the lane's
     // vector order, so the sums are those of one vector at a time
     uint32_t v = (s >> 2) + sub;
@@ -307,10 +307,10 @@ __device__ __forceinline__ float group_part_dot(const uint4* __restrict__ idx4, 
         for (int k = 0; k < 4; ++k) g1[k] = (e1 + k < t) ? ld_after(x + cs1[k]) : 0.f;
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            if (e0 + k >= s) acc = fmaf(a0[k], g0[k], acc);
+            if (e0 + k >= s) acc[k & 1] = fmaf(a0[k], g0[k], acc[k & 1]);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            if (e1 + k < t) acc = fmaf(a1[k], g1[k], acc);
+            if (e1 + k < t) acc[k & 1] = fmaf(a1[k], g1[k], acc[k & 1]);
     }
     for (; v < v1; v += LPR) {
         const uint4 c = ld_stream(idx4 + v);
@@ -323,9 +323,9 @@ __device__ __forceinline__ float group_part_dot(const uint4* __restrict__ idx4, 
         for (int k = 0; k < 4; ++k) g[k] = (e + k >= s && e + k < t) ? ld_after(x + cs[k]) : 0.f;
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            if (e + k >= s && e + k < t) acc = fmaf(a[k], g[k], acc);
+            if (e + k >= s && e + k < t) acc[k & 1] = fmaf(a[k], g[k], acc[k & 1]);
     }
-    return acc;
+    return acc[0] + acc[1];
 }
 
 template <typename V, int LPR, int U, bool WHOLE>
