@@ -23,8 +23,8 @@
 // the 12 GB class.  Measured and not kept: a half step (4 entries per lane) at
 // a row's end, 4% / 7% of padding but rows that start inside a 128-byte line
 // (mid, FP32 / FP16 values: 0.442 / 0.361 ms per iteration against 0.431 /
-// 0.313).  The lane sums (two chains per lane, even and odd elements) are
-// reduced by a fixed xor tree: deterministic.
+// 0.313).  The lane sums (kSums chains per lane) are reduced by a fixed xor
+// tree: deterministic.
 #include "kernels.cuh"
 
 #include <algorithm>
@@ -86,6 +86,16 @@ __device__ __forceinline__ V pad_value() {
 template <>
 __device__ __forceinline__ float pad_value<float>() { return -0.0f; }
 
+// Sums per lane: element j of a lane's vector goes to sum j mod kSums, 16 chains
+// per row as with 16 lanes of one sum each.
+template <int LPR>
+constexpr int kSums = 16 / LPR;
+
+template <int LPR>
+__device__ __forceinline__ float lane_sum(const float* acc) {
+    return kSums<LPR> == 4 ? (acc[0] + acc[1]) + (acc[2] + acc[kSums<LPR> - 1]) : acc[0] + acc[1];
+}
+
 // A row's sum again, in the same order, without the dummies and the padding, by
 // one thread: for rows whose sum is NaN (see the head of the file).
 template <typename V, int LPR>
@@ -96,25 +106,25 @@ __device__ __noinline__ float d16_row_real(const uint64_t* __restrict__ dvptr, c
     float sum[LPR];
     for (int l = 0; l < LPR; ++l) {
         uint32_t col = dbase[row];
-        float acc[2] = {0.f, 0.f};
+        float acc[kSums<LPR>] = {};
         for (uint64_t v = v0 + l; v < v1; v += LPR)
             for (int j = 0; j < 8; ++j) {
                 col += d16[8 * v + j];
                 const float a = (float)dval[8 * v + j];
-                if (__float_as_uint(a) != 0x80000000u) acc[j & 1] = fmaf(a, ld_after(x + col), acc[j & 1]);
+                if (__float_as_uint(a) != 0x80000000u) acc[j % kSums<LPR>] = fmaf(a, ld_after(x + col), acc[j % kSums<LPR>]);
             }
-        sum[l] = acc[0] + acc[1];
+        sum[l] = lane_sum<LPR>(acc);
     }
     for (int o = LPR / 2; o > 0; o >>= 1)
         for (int l = 0; l < o; ++l) sum[l] += sum[l + o];
     return sum[0];
 }
 
-// N steps of a lane: loads, columns, gathers, FMAs (even elements into acc0,
-// odd ones into acc1).  dp, vp: the lane's delta and value vector of the first.
+// N steps of a lane: loads, columns, gathers, FMAs.  dp, vp: the lane's delta and
+// value vector of the first.
 template <typename V, int LPR, int N>
 __device__ __forceinline__ void d16_steps(const uint4* dp, const V* vp, const float* __restrict__ x, uint32_t& prev,
-                                          float& acc0, float& acc1) {
+                                          float (&acc)[kSums<LPR>]) {
     uint4 dw[N];
     float a[N][8];
 #pragma unroll
@@ -140,10 +150,7 @@ __device__ __forceinline__ void d16_steps(const uint4* dp, const V* vp, const fl
 #pragma unroll
     for (int u = 0; u < N; ++u)
 #pragma unroll
-        for (int j = 0; j < 8; j += 2) {
-            acc0 = fmaf(a[u][j], gx[u][j], acc0);
-            acc1 = fmaf(a[u][j + 1], gx[u][j + 1], acc1);
-        }
+        for (int j = 0; j < 8; ++j) acc[j % kSums<LPR>] = fmaf(a[u][j], gx[u][j], acc[j % kSums<LPR>]);
 }
 
 // A stretch of whole vectors into L2 ahead of the loads.
@@ -160,17 +167,17 @@ template <typename V, int LPR, int U>
 __device__ __forceinline__ float d16_row(const uint4* dp, const V* vp, const float* __restrict__ x, uint32_t col,
                                          uint32_t nsteps, uint32_t gl) {
     uint32_t prev = col;  // column of this lane's previous element
-    float acc0 = 0.f, acc1 = 0.f;
+    float acc[kSums<LPR>] = {};
     dp += gl;
     vp += 8 * gl;
     uint32_t k = 0;
     for (; k + U <= nsteps; k += U) {
-        d16_steps<V, LPR, U>(dp, vp, x, prev, acc0, acc1);
+        d16_steps<V, LPR, U>(dp, vp, x, prev, acc);
         dp += U * LPR;
         vp += U * 8 * LPR;
     }
-    if (U == 2 && k < nsteps) d16_steps<V, LPR, 1>(dp, vp, x, prev, acc0, acc1);
-    return acc0 + acc1;
+    if (U == 2 && k < nsteps) d16_steps<V, LPR, 1>(dp, vp, x, prev, acc);
+    return lane_sum<LPR>(acc);
 }
 
 template <int EPI>
