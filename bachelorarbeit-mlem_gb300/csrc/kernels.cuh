@@ -62,8 +62,11 @@ void launch_csr_ilv(const DevCsr& op, const float* x, const EpiArgs& epi, int un
 // Delta-compressed (16-bit) column indices: build from the u32 indices, and
 // the projection that reads them.
 // Rows out of column order are sorted on the host first (sort_rows) or leave
-// the operand without the copy (returns false).
-bool build_d16(DevCsr& op, bool sort_rows, cudaStream_t s);
+// the operand without the copy (returns false), as does a copy of more than
+// max_bytes: its size is known once the rows' positions are counted, padding
+// (32 or 64 positions per row at least) and dummies included, and nothing but
+// the row offsets is allocated before.
+bool build_d16(DevCsr& op, bool sort_rows, uint64_t max_bytes, cudaStream_t s);
 void free_d16(DevCsr& op);
 // Mean row length from which rows get 8 lanes: bfloat16 A / A^T of rows of 239 /
 // 210 entries 0.109 / 0.118 ms with 8 lanes, 0.121 / 0.126 ms with 4; below

@@ -406,25 +406,44 @@ static void d16_cands(const DevCsr& op, std::vector<ProjCfg>& cand) {
 // Whether the tuner may give the operand a delta-coded copy of its own (a
 // handle created without compress_indices): the stream it would replace
 // crosses HBM on every projection (an operand that fits in L2 gains nothing:
-// 2-D ring 8.9 us per iteration without the copy, 9.9 with it), the copy takes
-// at most a quarter of the free memory, and the handle outlives the build.
-// Building a copy costs about 15 projections and saves a fifth of each, so a
-// handle made for one call of fewer than kCopyPays iterations goes without.
+// 2-D ring 8.9 us per iteration without the copy, 9.9 with it), and the handle
+// outlives the build.  Building a copy costs about 15 projections and saves a
+// fifth of each, so a handle made for one call of fewer than kCopyPays
+// iterations goes without.
+// Returns the bytes that the copy may take, 0 for none: at most a quarter of the
+// free memory, and less than the stream that it replaces (rows much shorter than
+// a step of 32 or 64 positions, or with columns far apart, would take several
+// times that: such an operand keeps its CSR arrays, and nothing is allocated).
 constexpr uint32_t kCopyPays = 100;
-static bool may_copy_d16(const mlem_matrix* m, const DevCsr& op) {
-    if (op.d16 || m->sym.fp_rowptr || (m->one_call && m->one_call < kCopyPays)) return false;
+static uint64_t copy_bytes_d16(const mlem_matrix* m, const DevCsr& op) {
+    if (op.d16 || m->sym.fp_rowptr || (m->one_call && m->one_call < kCopyPays)) return 0;
     int l2 = 0;
     size_t avail = 0, total = 0;
     MLEM_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, m->device));
     MLEM_CUDA(cudaMemGetInfo(&avail, &total));
-    const uint64_t stream = op.nnz * (4 + val_bytes(op.vt)), copy = op.nnz * (2 + val_bytes(op.vt)) / 4 * 5;
-    return stream > (uint64_t)l2 && copy <= avail / 4;
+    const uint64_t stream = op.nnz * (4 + val_bytes(op.vt));
+    return stream > (uint64_t)l2 ? std::min<uint64_t>(avail / 4, stream) : 0;
+}
+
+// Gives the operand that copy if it may have one; false: it has none.
+static bool try_copy_d16(const mlem_matrix* m, DevCsr& op, cudaStream_t s) {
+    const uint64_t max_bytes = copy_bytes_d16(m, op);
+    if (!max_bytes) return false;
+    try {
+        op.d16_tuned = build_d16(op, false, max_bytes, s);
+        op.d16_lost |= !op.d16_tuned;  // rows out of order or too sparse: they stay so
+        return op.d16_tuned;
+    } catch (const Error& err) {  // no room after all: the operand stays as it is
+        if (err.code != MLEM_ENOMEM) throw;
+        cudaGetLastError();
+        return false;
+    }
 }
 
 // Merge-path tiles of an operand for a section size, built on first use: one or
 // two vectors per lane in flight in the row kernel (16 or 12 blocks per SM; same
 // sums), and for tiles of whole rows the delta-coded copy where there is one or
-// may_copy_d16 allows one, timed with a Raw epilogue on a constant image.
+// try_copy_d16 makes one, timed with a Raw epilogue on a constant image.
 const MergePlan& merge_plan(mlem_matrix* m, bool transposed, uint32_t secsize) {
     auto& plans = transposed ? m->plan_AT : m->plan_A;
     auto it = plans.find(secsize);
@@ -466,15 +485,7 @@ const MergePlan& merge_plan(mlem_matrix* m, bool transposed, uint32_t secsize) {
             }
             p.rows_u = pick;
             bool made = false;
-            if (p.whole && !op.d16_lost && may_copy_d16(m, op)) {
-                try {
-                    made = op.d16_tuned = build_d16(op, false, s);
-                } catch (const Error& err) {  // no room after all
-                    if (err.code != MLEM_ENOMEM) throw;
-                    cudaGetLastError();
-                }
-                op.d16_lost = !made;
-            }
+            if (p.whole && !op.d16_lost) made = try_copy_d16(m, op, s);
             if (p.whole && op.d16)
                 for (int u : {1, 2})
                     if (faster([&] { launch_merge_d16(op, p, x, e, u, L2Window{}, s); })) p.d16_u = u;
@@ -609,23 +620,13 @@ static void tune_projection(mlem_matrix* m, bool transposed) {
             if (c.ms < best.ms) best = c;
         };
         for (ProjCfg& c : cand) time(c);
-        if (may_copy_d16(m, op)) {
-            bool built = false;
-            try {
-                built = build_d16(op, false, s);
-            } catch (const Error& err) {  // no room after all: the operand stays as it is
-                if (err.code != MLEM_ENOMEM) throw;
-                cudaGetLastError();
-            }
-            if (built) {
-                op.d16_tuned = true;
-                std::vector<ProjCfg> more;
-                d16_cands(op, more);
-                for (ProjCfg& c : more) time(c);
-                if (best.kind != MLEM_KERNEL_D16) {
-                    free_d16(op);
-                    op.d16_tuned = false;
-                }
+        if (try_copy_d16(m, op, s)) {
+            std::vector<ProjCfg> more;
+            d16_cands(op, more);
+            for (ProjCfg& c : more) time(c);
+            if (best.kind != MLEM_KERNEL_D16) {
+                free_d16(op);
+                op.d16_tuned = false;
             }
         }
         check_device_error(m, s);
@@ -959,8 +960,8 @@ static void postprocess_matrix(mlem_matrix* m, const mlem_matrix_opts& o) {
     }
     m->vt = o.value_type;
     if (o.compress_indices) {
-        build_d16(A, true, s);
-        if (m->has_t) build_d16(m->AT, true, s);
+        build_d16(A, true, ~0ull, s);
+        if (m->has_t) build_d16(m->AT, true, ~0ull, s);
     }
     if (o.interleave) {
         build_ilv(A, s);

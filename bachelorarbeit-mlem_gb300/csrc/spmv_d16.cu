@@ -345,19 +345,28 @@ __device__ __forceinline__ uint32_t d16_slice(const uint32_t* __restrict__ col, 
 __device__ __forceinline__ unsigned group_mask(int L) { return ((1u << L) - 1u) << ((threadIdx.x & 31) & ~(L - 1)); }
 
 // Vectors per row (positions rounded up to whole steps of 8·L).  L lanes per row.
+// *sparse sums the vectors of the rows that hold more than twice their entries
+// (and a step); once they alone are above max_vec no further row is walked, so
+// that an operand that will not get a copy costs no long walks over dummies.
 template <int L>
 __global__ void __launch_bounds__(256)
 k_d16_count(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ col, uint32_t rows,
-            uint32_t* __restrict__ nvec) {
+            uint32_t* __restrict__ nvec, uint64_t max_vec, unsigned long long* sparse) {
     const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) / L;
     const int gl = threadIdx.x % L;
     if (r >= rows) return;  // whole group
     const unsigned mask = group_mask(L);
     uint64_t e = rowptr[r], ent;
-    const uint64_t t = rowptr[r + 1];
+    const uint64_t t = rowptr[r + 1], len = t - e;
+    const bool over = __shfl_sync(mask, *(volatile unsigned long long*)sparse, 0, L) > max_vec;
     uint32_t n = 0, ring = e < t ? col[e] : 0u;
-    for (; e < t; ++n) d16_slice<L>(col, t, e, ring, ent, mask, gl);
-    if (gl == 0) nvec[r] = (n + 7) / 8 * L;
+    if (!over)
+        for (; e < t; ++n) d16_slice<L>(col, t, e, ring, ent, mask, gl);
+    n = (n + 7) / 8 * L;
+    if (gl == 0) {
+        nvec[r] = n;
+        if (n > L && n / 2 > (len + 7) / 8) atomicAdd(sparse, (unsigned long long)n);
+    }
 }
 
 // Deltas and values at their positions, padding included.  L lanes per row; a
@@ -514,7 +523,10 @@ void free_d16(DevCsr& op) {
     op.d16_lanes = 0;
 }
 
-bool build_d16(DevCsr& op, bool sort_rows, cudaStream_t s) {
+bool build_d16(DevCsr& op, bool sort_rows, uint64_t max_bytes, cudaStream_t s) {
+    const uint64_t per_vec = 8 * (sizeof(uint16_t) + val_bytes(op.vt)), per_row = 12ull * op.nrows + 8;
+    if (per_row >= max_bytes) return false;
+    const uint64_t max_vec = (max_bytes - per_row) / per_vec;
     const uint64_t R = std::max<uint32_t>(op.nrows, 1);
     // 8 lanes per row cover more neighbouring columns per gather, 4 pad short
     // rows less (steps of 64 or 32 entries)
@@ -525,19 +537,22 @@ bool build_d16(DevCsr& op, bool sort_rows, cudaStream_t s) {
     uint32_t* sidx = nullptr;
     void* sval = nullptr;
     uint32_t* nvec = nullptr;
-    int* flag = nullptr;
+    unsigned long long* word = nullptr;  // [0] k_d16_check's flag, [1] k_d16_count's sum
     int unsorted = 0;
+    bool fits = true;
     try {
-        MLEM_CUDA(cudaMallocAsync(&flag, sizeof(int), s));
-        MLEM_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), s));
+        MLEM_CUDA(cudaMallocAsync(&word, 16, s));
+        MLEM_CUDA(cudaMemsetAsync(word, 0, 16, s));
         if (op.nrows) {
-            k_d16_check<<<grid_rows(op.nrows), 256, 0, s>>>(op.rowptr, op.idx, op.nrows, flag);
+            k_d16_check<<<grid_rows(op.nrows), 256, 0, s>>>(op.rowptr, op.idx, op.nrows, reinterpret_cast<int*>(word));
             MLEM_LAUNCHED();
         }
-        MLEM_CUDA(cudaMemcpyAsync(&unsorted, flag, sizeof(int), cudaMemcpyDeviceToHost, s));
-        MLEM_CUDA(cudaFreeAsync(flag, s));
+        MLEM_CUDA(cudaMemcpyAsync(&unsorted, word, sizeof(int), cudaMemcpyDeviceToHost, s));
         MLEM_CUDA(cudaStreamSynchronize(s));
-        if (unsorted && !sort_rows) return false;
+        if (unsorted && !sort_rows) {
+            cudaFreeAsync(word, s);
+            return false;
+        }
         if (unsorted) {
             sorted_copy(op, sidx, sval, s);
             idx = sidx;
@@ -547,20 +562,26 @@ bool build_d16(DevCsr& op, bool sort_rows, cudaStream_t s) {
         MLEM_CUDA(cudaMallocAsync(&nvec, sizeof(uint32_t) * R, s));
         MLEM_CUDA(cudaMalloc(&op.dvptr, sizeof(uint64_t) * (R + 1)));
         if (op.nrows) {
-            if (lanes == 4) k_d16_count<4><<<grid_groups(op.nrows, 4), 256, 0, s>>>(op.rowptr, idx, op.nrows, nvec);
-            else k_d16_count<8><<<grid_groups(op.nrows, 8), 256, 0, s>>>(op.rowptr, idx, op.nrows, nvec);
+            if (lanes == 4)
+                k_d16_count<4><<<grid_groups(op.nrows, 4), 256, 0, s>>>(op.rowptr, idx, op.nrows, nvec, max_vec, word + 1);
+            else
+                k_d16_count<8><<<grid_groups(op.nrows, 8), 256, 0, s>>>(op.rowptr, idx, op.nrows, nvec, max_vec, word + 1);
             MLEM_LAUNCHED();
         }
         scan_counts_u64(nvec, op.dvptr, op.nrows, s);
-        uint64_t nv = 0;
+        uint64_t nv = 0, sparse = 0;
         MLEM_CUDA(cudaMemcpyAsync(&nv, op.dvptr + op.nrows, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+        MLEM_CUDA(cudaMemcpyAsync(&sparse, word + 1, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
         MLEM_CUDA(cudaStreamSynchronize(s));
-        op.dvec = nv;
+        fits = std::max(nv, sparse) <= max_vec;
         const uint64_t slots = 8 * std::max<uint64_t>(nv, 1);
-        MLEM_CUDA(cudaMalloc(&op.dbase, sizeof(uint32_t) * R));
-        MLEM_CUDA(cudaMalloc(&op.d16, sizeof(uint16_t) * slots));
-        MLEM_CUDA(cudaMalloc(&op.dval, val_bytes(op.vt) * slots));
-        if (op.nrows) {
+        if (fits) {
+            op.dvec = nv;
+            MLEM_CUDA(cudaMalloc(&op.dbase, sizeof(uint32_t) * R));
+            MLEM_CUDA(cudaMalloc(&op.d16, sizeof(uint16_t) * slots));
+            MLEM_CUDA(cudaMalloc(&op.dval, val_bytes(op.vt) * slots));
+        }
+        if (fits && op.nrows) {
             switch (op.vt) {
                 case MLEM_VAL_F32: d16_fill<float>(op, idx, val, s); break;
                 case MLEM_VAL_F16: d16_fill<__half>(op, idx, val, s); break;
@@ -570,16 +591,19 @@ bool build_d16(DevCsr& op, bool sort_rows, cudaStream_t s) {
         MLEM_CUDA(cudaStreamSynchronize(s));
     } catch (...) {
         cudaStreamSynchronize(s);
+        cudaFree(word);
         cudaFree(nvec);
         cudaFree(sidx);
         cudaFree(sval);
         free_d16(op);
         throw;
     }
+    cudaFree(word);
     cudaFree(nvec);
     cudaFree(sidx);
     cudaFree(sval);
-    return true;
+    if (!fits) free_d16(op);
+    return fits;
 }
 
 void launch_csr_d16(const DevCsr& op, const float* x, const EpiArgs& epi, int unroll, L2Window win, cudaStream_t s) {

@@ -240,9 +240,11 @@ typedef enum {
     MLEM_KERNEL_PERSISTENT = 2,
     MLEM_KERNEL_AUTO = 3, /* autotuned per matrix operand (lanes per row, vectors in flight, variant).
                              An operand larger than L2 with ascending columns in every row also gets
-                             a delta-coded copy (the D16 form, ~1.1 * nnz * (2 + value) bytes) on its
-                             first AUTO run (csr-vector or merge-based) if that fits a quarter of the
-                             free memory; it is kept where it is the fastest and counts in
+                             a delta-coded copy (the D16 form: positions * (2 + value) bytes, rows
+                             padded to 32 or 64 positions; ~1.1 * nnz positions where rows are long)
+                             on its first AUTO run (csr-vector or merge-based) if that takes at most
+                             a quarter of the free memory and less than its nnz * (4 + value) bytes;
+                             it is kept where it is the fastest and counts in
                              mlem_matrix_info.device_bytes */
     MLEM_KERNEL_D16 = 4,  /* delta-coded indices (matrix created with compress_indices = 1) */
     MLEM_KERNEL_ILV = 5,  /* lane-interleaved copy (matrix created with interleave = 1) */

@@ -1,0 +1,60 @@
+"""What a handle holds, reports and takes over many calls (GPU): the autotuner's
+own delta-coded copies, graphs of any iteration count, batches of any size, the
+server's account of device memory."""
+from __future__ import annotations
+
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+class Sampler(threading.Thread):
+    """Calls `read` over and over while a block runs; `seen` holds what it returned."""
+
+    def __init__(self, read):
+        super().__init__()
+        self.read, self.seen, self.go = read, [], True
+
+    def run(self):
+        while self.go:
+            self.seen.append(self.read())
+
+    def __enter__(self):
+        self.start()
+        return self
+
+    def __exit__(self, *a):
+        self.go = False
+        self.join()
+
+
+@pytest.mark.parametrize("spmv", [0, 1])
+def test_copy_of_short_rows_with_wide_gaps_is_not_made(pkg, cuda, spmv):
+    """Rows of 1 to 8 entries, a third of them with columns up to 300,000 apart: a
+    delta-coded copy would take several times the CSR stream, so none is made."""
+    rng = np.random.default_rng(8)
+    rows, cols = 6_000_000, 20_000_000
+    lens = rng.integers(1, 9, rows)
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.uint64)
+    gap = rng.integers(1, np.repeat(np.where(rng.random(rows) < 1 / 3, 300_000, 40), lens))
+    at = np.cumsum(gap)
+    base = np.repeat(at[rp[:-1].astype(np.int64)], lens)
+    col = (np.repeat(rng.integers(0, cols - 2_500_000, rows), lens) + at - base).astype(np.uint32)
+    val = np.ones(len(col), np.float32)
+    m = pkg.Matrix.from_csr(rp, col, val, cols, build_transpose=False)
+    x, g = cuda.ones(cols, device="cuda"), cuda.ones(rows, dtype=cuda.int32, device="cuda")
+    ratio, fp = cuda.empty(rows, device="cuda"), cuda.empty(rows, device="cuda")
+    cuda.cuda.synchronize()
+    before = cuda.cuda.mem_get_info()[0]
+    with Sampler(lambda: cuda.cuda.mem_get_info()[0]) as s:
+        m.forward_project(x.data_ptr(), g.data_ptr(), ratio.data_ptr(), fp.data_ptr(), spmv=spmv,
+                          bp_mode=pkg.BP_SCATTER)
+        cuda.cuda.synchronize()
+    np.testing.assert_allclose(fp.cpu().numpy(), lens, rtol=1e-6)
+    # the workspace, the trials' two vectors, the rows' counts, offsets and scan, and
+    # 64 MB for the allocator's granularity; a copy of 32 positions per row is 1.2 GB
+    assert before - min(s.seen) < (12 * rows + 8 * cols) + 4 * (rows + cols) + 24 * rows + (64 << 20)
+    m.close()
