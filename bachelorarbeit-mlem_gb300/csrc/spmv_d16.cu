@@ -76,6 +76,10 @@ struct Val8<__nv_bfloat16> {
     }
 };
 
+// The row of this thread's group of L lanes (threads may outnumber 2^32).
+template <int L>
+__device__ __forceinline__ uint32_t group_row() { return blockIdx.x * (blockDim.x / L) + threadIdx.x / L; }
+
 // The value of dummies and padding.
 template <typename V>
 __device__ __forceinline__ V pad_value() {
@@ -206,7 +210,7 @@ k_csr_d16(const uint64_t* __restrict__ dvptr, const uint32_t* __restrict__ dbase
           const V* __restrict__ dval, const float* __restrict__ x, uint32_t nrows, const int32_t* __restrict__ g,
           float* __restrict__ out, float* __restrict__ fwproj, float* __restrict__ f, const float* __restrict__ norm) {
     grid_release();
-    const uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) / LPR;
+    const uint32_t row = group_row<LPR>();
     const uint32_t gl = threadIdx.x % LPR;
     const bool live = row < nrows;
     const uint64_t v0 = live ? dvptr[row] : 0, v1 = live ? dvptr[row + 1] : 0;
@@ -352,7 +356,7 @@ template <int L>
 __global__ void __launch_bounds__(256)
 k_d16_count(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ col, uint32_t rows,
             uint32_t* __restrict__ nvec, uint64_t max_vec, unsigned long long* sparse) {
-    const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) / L;
+    const uint32_t r = group_row<L>();
     const int gl = threadIdx.x % L;
     if (r >= rows) return;  // whole group
     const unsigned mask = group_mask(L);
@@ -380,7 +384,7 @@ k_d16_fill(const uint64_t* __restrict__ rowptr, const uint32_t* __restrict__ col
            uint16_t* __restrict__ d16, V* __restrict__ dval) {
     __shared__ __align__(16) uint16_t sd[256][8];
     __shared__ __align__(16) V sv[256][8];
-    const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) / L;
+    const uint32_t r = group_row<L>();
     const int gl = threadIdx.x % L;
     if (r >= rows) return;  // whole group
     const unsigned mask = group_mask(L);

@@ -58,3 +58,29 @@ def test_copy_of_short_rows_with_wide_gaps_is_not_made(pkg, cuda, spmv):
     # 64 MB for the allocator's granularity; a copy of 32 positions per row is 1.2 GB
     assert before - min(s.seen) < (12 * rows + 8 * cols) + 4 * (rows + cols) + 24 * rows + (64 << 20)
     m.close()
+
+
+def test_delta_coded_rows_beyond_2_30(pkg, cuda):
+    """More rows than 2^32 threads hold at 4 lanes each, nearly all empty."""
+    rows, cols = (1 << 30) + 70, 4000
+    at = np.array([0, 5, 69, 1 << 20, (1 << 30) - 1, 1 << 30, (1 << 30) + 5, rows - 1])
+    lens = np.array([3, 70, 1, 40, 33, 31, 64, 9])
+    rng = np.random.default_rng(4)
+    col = np.concatenate([np.sort(rng.choice(cols, n, replace=False)) for n in lens]).astype(np.uint32)
+    rp = np.empty(rows + 1, np.uint64)
+    for i, n in enumerate(np.cumsum(lens)):
+        rp[at[i] + 1:at[i + 1] + 1 if i + 1 < len(at) else None] = n
+    rp[0] = 0
+    x, val = rng.uniform(0.5, 1.5, cols).astype(np.float32), rng.uniform(0.05, 1.0, len(col)).astype(np.float32)
+    m = pkg.Matrix.from_csr(rp, col, val, cols, build_transpose=False, compress=True)
+    del rp
+    dx, g = cuda.from_numpy(x).cuda(), cuda.zeros(rows, dtype=cuda.int32, device="cuda")
+    ratio, fp = cuda.full((rows,), -1.0, device="cuda"), cuda.full((rows,), -1.0, device="cuda")
+    m.forward_project(dx.data_ptr(), g.data_ptr(), ratio.data_ptr(), fp.data_ptr(), kernel=pkg.KERNEL_D16,
+                      bp_mode=pkg.BP_SCATTER)
+    cuda.cuda.synchronize()
+    want = np.add.reduceat(val.astype(np.float64) * x[col], np.cumsum(lens) - lens)
+    got = fp[cuda.from_numpy(at).cuda()].cpu().numpy()
+    assert np.all(np.abs(got - want) <= (lens + 2) * 2.0**-24 * want)
+    assert int(cuda.count_nonzero(fp)) == len(at) and int(cuda.count_nonzero(ratio)) == 0
+    m.close()
