@@ -125,6 +125,7 @@ void ensure_workspace(mlem_matrix* m) {
         MLEM_CUDA(cudaMalloc(&w.tmp_cols, sizeof(float) * C));
     }
     MLEM_CUDA(cudaStreamSynchronize(m->stream));
+    std::lock_guard<std::mutex> lk(m->info_mu);
     w.ready = true;
 }
 
@@ -289,7 +290,17 @@ FusedForm fused_form(mlem_matrix* m, const mlem_run_opts& o) {
     auto staged = [&]() {
         if (!p.staged_threads) {
             ensure_workspace(m);
-            if (!p.built) fused_plan_build(m->A, p, m->stream);
+            if (!p.built) {
+                FusedPlan made;
+                try {
+                    fused_plan_build(m->A, made, m->stream);
+                } catch (...) {
+                    made.release();
+                    throw;
+                }
+                std::lock_guard<std::mutex> lk(m->info_mu);
+                p = made;
+            }
             prepare_fused_staged(m->A.vt);
             FusedForm a, b;
             a.kind = b.kind = 1;
@@ -425,19 +436,38 @@ static uint64_t copy_bytes_d16(const mlem_matrix* m, const DevCsr& op) {
     return stream > (uint64_t)l2 ? std::min<uint64_t>(avail / 4, stream) : 0;
 }
 
+static void set_copy_d16(mlem_matrix* m, DevCsr& op, const DevCsr& c) {
+    std::lock_guard<std::mutex> lk(m->info_mu);
+    op.dvptr = c.dvptr;
+    op.dbase = c.dbase;
+    op.d16 = c.d16;
+    op.dval = c.dval;
+    op.dvec = c.dvec;
+    op.d16_lanes = c.d16_lanes;
+    op.d16_tuned = c.d16_tuned;
+}
+
 // Gives the operand that copy if it may have one; false: it has none.
-static bool try_copy_d16(const mlem_matrix* m, DevCsr& op, cudaStream_t s) {
+static bool try_copy_d16(mlem_matrix* m, DevCsr& op, cudaStream_t s) {
     const uint64_t max_bytes = copy_bytes_d16(m, op);
     if (!max_bytes) return false;
+    DevCsr c = op;
     try {
-        op.d16_tuned = build_d16(op, false, max_bytes, s);
-        op.d16_lost |= !op.d16_tuned;  // rows out of order or too sparse: they stay so
-        return op.d16_tuned;
+        c.d16_tuned = build_d16(c, false, max_bytes, s);
     } catch (const Error& err) {  // no room after all: the operand stays as it is
         if (err.code != MLEM_ENOMEM) throw;
         cudaGetLastError();
         return false;
     }
+    op.d16_lost |= !c.d16_tuned;  // rows out of order or too sparse: they stay so
+    set_copy_d16(m, op, c);
+    return op.d16_tuned;
+}
+
+static void drop_copy_d16(mlem_matrix* m, DevCsr& op) {
+    DevCsr c = op;
+    set_copy_d16(m, op, DevCsr());
+    free_d16(c);
 }
 
 // Merge-path tiles of an operand for a section size, built on first use: one or
@@ -490,8 +520,7 @@ const MergePlan& merge_plan(mlem_matrix* m, bool transposed, uint32_t secsize) {
                 for (int u : {1, 2})
                     if (faster([&] { launch_merge_d16(op, p, x, e, u, L2Window{}, s); })) p.d16_u = u;
             if (made && !p.d16_u) {
-                free_d16(op);
-                op.d16_tuned = false;
+                drop_copy_d16(m, op);
                 op.d16_lost = true;
             }
         } catch (...) {
@@ -508,6 +537,7 @@ const MergePlan& merge_plan(mlem_matrix* m, bool transposed, uint32_t secsize) {
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
     }
+    std::lock_guard<std::mutex> lk(m->info_mu);
     return plans.emplace(secsize, p).first->second;
 }
 
@@ -624,10 +654,7 @@ static void tune_projection(mlem_matrix* m, bool transposed) {
             std::vector<ProjCfg> more;
             d16_cands(op, more);
             for (ProjCfg& c : more) time(c);
-            if (best.kind != MLEM_KERNEL_D16) {
-                free_d16(op);
-                op.d16_tuned = false;
-            }
+            if (best.kind != MLEM_KERNEL_D16) drop_copy_d16(m, op);
         }
         check_device_error(m, s);
     } catch (...) {
@@ -1295,6 +1322,7 @@ mlem_status mlem_matrix_destroy(mlem_matrix* m) {
 mlem_status mlem_matrix_get_info(const mlem_matrix* m, mlem_matrix_info* info) {
     return guarded([&] {
         MLEM_REQUIRE(m && info, MLEM_EINVAL, "NULL argument");
+        std::lock_guard<std::mutex> lk(m->info_mu);
         info->rows = m->A.nrows;
         info->cols = m->A.ncols;
         info->nnz = m->A.nnz;

@@ -146,6 +146,9 @@ struct mlem_matrix {
     bool tuned[2] = {false, false};   // csr-vector configuration of A / Aᵀ measured
     mlem::ProjCfg proj[2];
     std::mutex mu;
+    // Held while a run (under mu) changes what mlem_matrix_get_info reads, and by
+    // that query, which so waits for no run: workspace, plans, a tuner's copies.
+    mutable std::mutex info_mu;
     uint64_t bytes() const;
 };
 

@@ -3,12 +3,32 @@ own delta-coded copies, graphs of any iteration count, batches of any size, the
 server's account of device memory."""
 from __future__ import annotations
 
+import ctypes as C
 import threading
 
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
+
+
+def info(pkg, m):
+    i = pkg.MatrixInfo()
+    pkg.load_library().mlem_matrix_get_info(m.handle, C.byref(i))
+    return i
+
+
+@pytest.fixture(scope="module")
+def large(pkg):
+    """18 M nonzeros in ascending rows of 450 (144 MB, more than L2): the tuner makes
+    delta-coded copies of A and of its transpose.  Host arrays and a sinogram."""
+    rng = np.random.default_rng(5)
+    rows, cols, n = 40_000, 50_000, 450
+    start = rng.integers(0, cols - 2 * n, rows)
+    col = (start[:, None] + np.arange(0, 2 * n, 2)[None, :]).astype(np.uint32).ravel()
+    rp = (np.arange(rows + 1) * n).astype(np.uint64)
+    val = rng.uniform(0.05, 1.0, col.size).astype(np.float32)
+    return rp, col, val, cols, rng.poisson(50.0, rows).astype(np.int32)
 
 
 class Sampler(threading.Thread):
@@ -84,3 +104,21 @@ def test_delta_coded_rows_beyond_2_30(pkg, cuda):
     assert np.all(np.abs(got - want) <= (lens + 2) * 2.0**-24 * want)
     assert int(cuda.count_nonzero(fp)) == len(at) and int(cuda.count_nonzero(ratio)) == 0
     m.close()
+
+
+def test_info_while_the_tuner_builds_its_copies(pkg, large):
+    """A query beside the first AUTO run never reports the copies that the tuner makes
+    as ones that the handle was asked for, and waits for no run."""
+    rp, col, val, cols, g = large
+    for _ in range(3):
+        m = pkg.Matrix.from_csr(rp, col, val, cols)
+
+        def read():
+            i = info(pkg, m)
+            return i.d16_slots, i.d16_slots_t, i.d16_lanes, i.d16_lanes_t
+
+        with Sampler(read) as s:
+            m.run(g, 2)
+        assert set(s.seen) == {(0, 0, 0, 0)}
+        assert len(s.seen) > 100  # the run takes tens of milliseconds, a query microseconds
+        m.close()
