@@ -297,12 +297,11 @@ class Matrix:
     def __init__(self, handle: int, keep=None):
         self._h = C.c_void_p(handle)
         self._keep = keep
-        info = MatrixInfo()
-        _check(load_library().mlem_matrix_get_info(self._h, C.byref(info)))
+        info = self._info()
         self.rows, self.cols, self.nnz = info.rows, info.cols, info.nnz
         self.value_type = info.value_type
         self.has_transpose = bool(info.has_transpose)
-        self.device_bytes = info.device_bytes
+        self._bytes = info.device_bytes
         self.max_row_nnz, self.max_col_nnz = info.max_row_nnz, info.max_col_nnz
         self.symmetry = {"lor_rows": info.sym_lor_rows, "voxel_rows": info.sym_voxel_rows,
                          "fp_nnz": info.sym_fp_nnz, "bp_nnz": info.sym_bp_nnz} if info.sym_lor_rows else None
@@ -369,6 +368,7 @@ class Matrix:
 
     def close(self) -> None:
         if self._h and self._h.value:
+            self.device_bytes  # the last value stays
             _check(load_library().mlem_matrix_destroy(self._h))
             self._h = C.c_void_p(None)
 
@@ -387,6 +387,19 @@ class Matrix:
     @property
     def handle(self):
         return self._h
+
+    def _info(self) -> MatrixInfo:
+        info = MatrixInfo()
+        _check(load_library().mlem_matrix_get_info(self._h, C.byref(info)))
+        return info
+
+    @property
+    def device_bytes(self) -> int:
+        """Device memory that the handle holds now: runs add their workspace, plans
+        and the autotuner's copies to it.  Of a closed handle, what it held before."""
+        if self._h and self._h.value:
+            self._bytes = self._info().device_bytes
+        return self._bytes
 
     # accessors ------------------------------------------------------------
     def norm(self) -> np.ndarray:

@@ -122,3 +122,17 @@ def test_info_while_the_tuner_builds_its_copies(pkg, large):
         assert set(s.seen) == {(0, 0, 0, 0)}
         assert len(s.seen) > 100  # the run takes tens of milliseconds, a query microseconds
         m.close()
+
+
+def test_device_bytes_follow_the_handle(pkg, large):
+    rp, col, val, cols, g = large
+    m = pkg.Matrix.from_csr(rp, col, val, cols)
+    new = m.device_bytes
+    m.run(g, 2, kernel=pkg.KERNEL_DIRECT)
+    direct = m.device_bytes
+    assert direct == new + 12 * m.rows + 8 * m.cols == info(pkg, m).device_bytes
+    m.run(g, 2)
+    assert m.device_bytes == info(pkg, m).device_bytes >= direct
+    held = m.device_bytes
+    m.close()
+    assert m.device_bytes == held
