@@ -235,6 +235,7 @@ struct DevCsr {
     uint64_t dvec = 0;           // vectors
     int d16_lanes = 0;           // lanes per row the D16 layout is built for (4 or 8)
     bool d16_tuned = false;      // made by a tuner, not asked for by compress_indices
+    bool d16_asked() const { return d16 && !d16_tuned; }
     bool d16_lost = false;       // it cannot be made, or merge-path tiles were faster without it: not tried for them again
     // optional processing order of the rows (locality of the gathers); the
     // k-th row group handles row order[k].  Results are written per row.

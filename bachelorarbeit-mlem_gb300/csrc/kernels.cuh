@@ -186,6 +186,9 @@ struct MergePlan {
     int lanes = 16;              // row kernel: lanes per row (8 or 16)
     int d16_u = 0;               // the operand's delta-coded copy is faster: its vectors per lane in flight
     int rows_u = 1;              // row kernel: vectors per lane in flight (1: 16 blocks per SM, 2: 12)
+    float ms = 1e30f;            // measured time of two launches of the form chosen so far
+    bool timed = false;          // rows_u is measured
+    bool copy_timed = false;     // ... and d16_u
     void release();
 };
 // Builds the tile partition of `op` for a section size (device allocations).

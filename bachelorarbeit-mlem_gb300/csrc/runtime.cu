@@ -470,50 +470,58 @@ static void drop_copy_d16(mlem_matrix* m, DevCsr& op) {
     free_d16(c);
 }
 
-// Merge-path tiles of an operand for a section size, built on first use: one or
-// two vectors per lane in flight in the row kernel (16 or 12 blocks per SM; same
-// sums), and for tiles of whole rows the delta-coded copy where there is one or
-// try_copy_d16 makes one, timed with a Raw epilogue on a constant image.
-const MergePlan& merge_plan(mlem_matrix* m, bool transposed, uint32_t secsize) {
-    auto& plans = transposed ? m->plan_AT : m->plan_A;
-    auto it = plans.find(secsize);
-    if (it != plans.end()) return it->second;
-    MergePlan p;
-    DevCsr& op = transposed ? m->AT : m->A;
+static bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+    cudaGetLastError();  // the default stream beside another stream's capture
+    return true;
+}
+
+// Times a plan with a Raw epilogue on a constant image: one or two vectors per
+// lane in flight in the row kernel (16 or 12 blocks per SM; same sums) where that
+// is not known yet, and with copy, for tiles of whole rows, the delta-coded copy
+// where there is one or try_copy_d16 makes one.
+static void tune_merge(mlem_matrix* m, DevCsr& op, MergePlan& p, bool copy) {
     cudaStream_t s = m->stream;
-    merge_plan_build(op, secsize, p, s);
-    MLEM_CUDA(cudaStreamSynchronize(s));
-    if (p.rows_kernel && op.nnz) {
-        float *x = nullptr, *y = nullptr;
-        cudaEvent_t e0 = nullptr, e1 = nullptr;
-        float best = 1e30f;
-        try {
-            MLEM_CUDA(cudaMalloc(&x, sizeof(float) * std::max<uint32_t>(op.ncols, 1)));
-            MLEM_CUDA(cudaMalloc(&y, sizeof(float) * std::max<uint32_t>(op.nrows, 1)));
-            MLEM_CUDA(cudaMemsetAsync(x, 0x3f, sizeof(float) * std::max<uint32_t>(op.ncols, 1), s));
-            MLEM_CUDA(cudaEventCreate(&e0));
-            MLEM_CUDA(cudaEventCreate(&e1));
-            EpiArgs e;
-            e.kind = Epi::Raw;
-            e.out = y;
-            auto faster = [&](auto launch) {  // than the best so far
-                launch();
-                MLEM_CUDA(cudaEventRecord(e0, s));
-                for (int q = 0; q < 2; ++q) launch();
-                MLEM_CUDA(cudaEventRecord(e1, s));
-                MLEM_CUDA(cudaEventSynchronize(e1));
-                float ms = 0.f;
-                MLEM_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-                if (ms >= best) return false;
-                best = ms;
-                return true;
-            };
+    float *x = nullptr, *y = nullptr;
+    cudaEvent_t e0 = nullptr, e1 = nullptr;
+    auto done = [&] {
+        cudaFree(x);
+        cudaFree(y);
+        if (e0) cudaEventDestroy(e0);
+        if (e1) cudaEventDestroy(e1);
+    };
+    try {
+        MLEM_CUDA(cudaMalloc(&x, sizeof(float) * std::max<uint32_t>(op.ncols, 1)));
+        MLEM_CUDA(cudaMalloc(&y, sizeof(float) * std::max<uint32_t>(op.nrows, 1)));
+        MLEM_CUDA(cudaMemsetAsync(x, 0x3f, sizeof(float) * std::max<uint32_t>(op.ncols, 1), s));
+        MLEM_CUDA(cudaEventCreate(&e0));
+        MLEM_CUDA(cudaEventCreate(&e1));
+        EpiArgs e;
+        e.kind = Epi::Raw;
+        e.out = y;
+        auto faster = [&](auto launch) {  // than the best so far
+            launch();
+            MLEM_CUDA(cudaEventRecord(e0, s));
+            for (int q = 0; q < 2; ++q) launch();
+            MLEM_CUDA(cudaEventRecord(e1, s));
+            MLEM_CUDA(cudaEventSynchronize(e1));
+            float ms = 0.f;
+            MLEM_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+            if (ms >= p.ms) return false;
+            p.ms = ms;
+            return true;
+        };
+        if (!p.timed) {
             int pick = 1;
             for (int u : {1, 2}) {
                 p.rows_u = u;
                 if (faster([&] { launch_merge_spmv(op, p, x, e, L2Window{}, s); })) pick = u;
             }
             p.rows_u = pick;
+            p.timed = true;
+        }
+        if (copy) {
             bool made = false;
             if (p.whole && !op.d16_lost) made = try_copy_d16(m, op, s);
             if (p.whole && op.d16)
@@ -523,19 +531,40 @@ const MergePlan& merge_plan(mlem_matrix* m, bool transposed, uint32_t secsize) {
                 drop_copy_d16(m, op);
                 op.d16_lost = true;
             }
+            p.copy_timed = true;
+        }
+    } catch (...) {
+        cudaStreamSynchronize(s);
+        done();
+        throw;
+    }
+    done();
+}
+
+// Merge-path tiles of an operand for a section size, built and timed on first use.
+// copy: the caller may run them over a tuner's delta-coded copy (kernel AUTO); a
+// plan that other kernels used before tries it then, unless user_stream is being
+// captured, where nothing can be timed.
+const MergePlan& merge_plan(mlem_matrix* m, bool transposed, uint32_t secsize, bool copy, cudaStream_t user_stream) {
+    auto& plans = transposed ? m->plan_AT : m->plan_A;
+    DevCsr& op = transposed ? m->AT : m->A;
+    auto it = plans.find(secsize);
+    if (it != plans.end()) {
+        MergePlan& p = it->second;
+        if (copy && p.timed && !p.copy_timed && !capturing(user_stream)) tune_merge(m, op, p, true);
+        return p;
+    }
+    MergePlan p;
+    cudaStream_t s = m->stream;
+    merge_plan_build(op, secsize, p, s);
+    MLEM_CUDA(cudaStreamSynchronize(s));
+    if (p.rows_kernel && op.nnz) {
+        try {
+            tune_merge(m, op, p, copy);
         } catch (...) {
-            cudaStreamSynchronize(s);
-            cudaFree(x);
-            cudaFree(y);
-            if (e0) cudaEventDestroy(e0);
-            if (e1) cudaEventDestroy(e1);
             p.release();
             throw;
         }
-        cudaFree(x);
-        cudaFree(y);
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
     }
     std::lock_guard<std::mutex> lk(m->info_mu);
     return plans.emplace(secsize, p).first->second;
@@ -548,15 +577,18 @@ const MergePlan& merge_plan(mlem_matrix* m, bool transposed, uint32_t secsize) {
 // made for one call tries the plain kernel with three lane counts only: the
 // other forms are within a few percent of it, and timing them all takes longer
 // than 100 iterations (30 M nonzeros: 12.2 ms for both operands; 1.0 ms so).
-static void tune_projection(mlem_matrix* m, bool transposed) {
-    if (m->tuned[transposed]) return;
+// copy: the caller's projections read this operand, so that it may get a
+// delta-coded copy (try_copy_d16), now or where it was tuned without before.
+static void tune_projection(mlem_matrix* m, bool transposed, bool copy) {
+    const bool known = m->tuned[transposed];
+    if (known && (!copy || m->copy_timed[transposed])) return;
     DevCsr& op = transposed ? m->AT : m->A;
     cudaStream_t s = m->stream;
     std::vector<ProjCfg> cand;
     const int base = pick_lanes(op.nnz, op.nrows);
     const bool brief = m->one_call != 0;
     for (int lanes : {base / 2, base, base * 2})
-        if (lanes >= 4 && lanes <= 32) {
+        if (!known && lanes >= 4 && lanes <= 32) {
             if (brief) {
                 cand.push_back(ProjCfg{MLEM_KERNEL_DIRECT, lanes, 2, 0.f, false, false});
                 continue;
@@ -569,10 +601,10 @@ static void tune_projection(mlem_matrix* m, bool transposed) {
                             if ((ord || pipe) && (!ord || op.order))
                                 cand.push_back(ProjCfg{MLEM_KERNEL_DIRECT, lanes, u, 0.f, ord, pipe});
         }
-    if (!brief) {
+    if (!brief && !known) {
         if (base >= 16) cand.push_back(ProjCfg{MLEM_KERNEL_PERSISTENT, base, 1, 0.f, false, false});
         cand.push_back(ProjCfg{MLEM_KERNEL_TMA, 32, 2, 0.f});
-        if (op.d16) d16_cands(op, cand);
+        if (op.d16_asked()) d16_cands(op, cand);
         if (op.idx_ilv)
             for (int u : {1, 2, 4}) cand.push_back(ProjCfg{MLEM_KERNEL_ILV, 32, u, 0.f});
         if (m->sym.fp_rowptr)
@@ -590,6 +622,7 @@ static void tune_projection(mlem_matrix* m, bool transposed) {
     MLEM_CUDA(cudaEventCreate(&e1));
     ProjCfg best;
     best.ms = 1e30f;
+    if (known) best = m->proj[transposed];
     try {
         // every byte 0x3f: x = 0.747
         MLEM_CUDA(cudaMemsetAsync(x, 0x3f, sizeof(float) * std::max<uint32_t>(op.ncols, 1), s));
@@ -650,11 +683,12 @@ static void tune_projection(mlem_matrix* m, bool transposed) {
             if (c.ms < best.ms) best = c;
         };
         for (ProjCfg& c : cand) time(c);
-        if (try_copy_d16(m, op, s)) {
+        if (copy && !op.d16_asked()) {
+            const bool made = try_copy_d16(m, op, s);  // a merge plan may have made one before
             std::vector<ProjCfg> more;
-            d16_cands(op, more);
+            if (op.d16) d16_cands(op, more);
             for (ProjCfg& c : more) time(c);
-            if (best.kind != MLEM_KERNEL_D16) drop_copy_d16(m, op);
+            if (made && best.kind != MLEM_KERNEL_D16) drop_copy_d16(m, op);
         }
         check_device_error(m, s);
     } catch (...) {
@@ -670,15 +704,27 @@ static void tune_projection(mlem_matrix* m, bool transposed) {
     cudaEventDestroy(e1);
     m->proj[transposed] = best;
     m->tuned[transposed] = true;
+    m->copy_timed[transposed] |= copy;
 }
 
-void prepare_kernel(mlem_matrix* m, const mlem_run_opts& o) {
+// reads_a, reads_at: the operands that the caller's csr-vector projections read;
+// only these may get a copy.  user_stream: the stream they go to; while it is
+// being captured nothing can be timed, and what is tuned already stays as it is.
+void prepare_kernel(mlem_matrix* m, const mlem_run_opts& o, bool reads_a, bool reads_at, cudaStream_t user_stream) {
     if (o.kernel == MLEM_KERNEL_TMA) prepare_csr_tma(m->vt);
     else if (o.kernel == MLEM_KERNEL_PERSISTENT) prepare_csrvec_pipe(m->vt);
     else if (o.kernel == MLEM_KERNEL_AUTO) {
-        tune_projection(m, false);
-        if (m->has_t) tune_projection(m, true);
+        auto pending = [&](bool t, bool reads) { return reads && m->tuned[t] && !m->copy_timed[t]; };
+        if ((pending(false, reads_a) || pending(true, reads_at)) && capturing(user_stream)) reads_a = reads_at = false;
+        tune_projection(m, false, reads_a);
+        if (m->has_t) tune_projection(m, true, reads_at);
     }
+}
+
+// ... for MLEM runs: the fused pass and the scatter read A by kernels of their own.
+static void prepare_run(mlem_matrix* m, const mlem_run_opts& o, cudaStream_t s) {
+    if (o.spmv == MLEM_SPMV_CSR_VECTOR)
+        prepare_kernel(m, o, o.bp_mode != MLEM_BP_FUSED, o.bp_mode == MLEM_BP_TRANS, s);
 }
 
 // The csr-vector configuration a projection of A (or Aᵀ) uses under opts o.
@@ -696,7 +742,7 @@ static ProjCfg resolve_cfg(const mlem_matrix* m, bool transposed, const mlem_run
     } else if (o.kernel == MLEM_KERNEL_TMA) {
         c.kind = MLEM_KERNEL_TMA;
     } else if (o.kernel == MLEM_KERNEL_D16) {
-        MLEM_REQUIRE(op.d16 != nullptr && !op.d16_tuned, MLEM_EINVAL,
+        MLEM_REQUIRE(op.d16_asked(), MLEM_EINVAL,
                      "kernel D16 needs a matrix created with compress_indices = 1");
         c.kind = MLEM_KERNEL_D16;
         c.lanes = op.d16_lanes;
@@ -730,10 +776,11 @@ void project(mlem_matrix* m, bool transposed, const float* x, const EpiArgs& e, 
              L2Window win, cudaStream_t s) {
     const DevCsr& op = transposed ? m->AT : m->A;
     if (o.spmv == MLEM_SPMV_MERGE) {
-        const MergePlan& p = merge_plan(m, transposed, transposed ? o.secsize_bp : o.secsize_fp);
+        const MergePlan& p =
+            merge_plan(m, transposed, transposed ? o.secsize_bp : o.secsize_fp, o.kernel == MLEM_KERNEL_AUTO, s);
         int u = 0;  // vectors in flight over the delta-coded copy; 0: the CSR arrays
         if (o.kernel == MLEM_KERNEL_AUTO) u = p.d16_u;
-        else if (o.kernel == MLEM_KERNEL_D16 && p.whole && op.d16 && !op.d16_tuned) u = o.unroll == 1 ? 1 : 2;
+        else if (o.kernel == MLEM_KERNEL_D16 && p.whole && op.d16_asked()) u = o.unroll == 1 ? 1 : 2;
         if (u) launch_merge_d16(op, p, x, e, u, win, s);
         else launch_merge_spmv(op, p, x, e, win, s);
         return;
@@ -916,10 +963,11 @@ static uint32_t run_iterations(mlem_matrix* m, const mlem_run_opts& o, uint32_t 
         auto it = m->ws.graphs.find(key);
         if (it != m->ws.graphs.end()) return it->second;
         // plans and kernel attributes must exist before capture
-        if (o.spmv == MLEM_SPMV_CSR_VECTOR) prepare_kernel(m, o);
+        prepare_run(m, o, s);
         if (o.spmv == MLEM_SPMV_MERGE && o.bp_mode != MLEM_BP_FUSED) {
-            merge_plan(m, false, o.secsize_fp);
-            if (o.bp_mode == MLEM_BP_TRANS) merge_plan(m, true, o.secsize_bp);
+            const bool copy = o.kernel == MLEM_KERNEL_AUTO;
+            merge_plan(m, false, o.secsize_fp, copy, s);
+            if (o.bp_mode == MLEM_BP_TRANS) merge_plan(m, true, o.secsize_bp, copy, s);
         }
         if (o.bp_mode == MLEM_BP_SCATTER) scatter_lanes(m);
         if (o.bp_mode == MLEM_BP_FUSED) fused_form(m, o);
@@ -1335,7 +1383,7 @@ mlem_status mlem_matrix_get_info(const mlem_matrix* m, mlem_matrix_info* info) {
         info->sym_voxel_rows = m->sym.J;
         info->sym_fp_nnz = m->sym.fp_nnz;
         info->sym_bp_nnz = m->sym.bp_nnz;
-        const bool d = m->A.d16 && !m->A.d16_tuned, dt = m->has_t && m->AT.d16 && !m->AT.d16_tuned;
+        const bool d = m->A.d16_asked(), dt = m->has_t && m->AT.d16_asked();
         info->d16_slots = d ? 8 * m->A.dvec : 0;
         info->d16_slots_t = dt ? 8 * m->AT.dvec : 0;
         info->d16_lanes = d ? (uint32_t)m->A.d16_lanes : 0;
@@ -1364,7 +1412,7 @@ mlem_status mlem_matrix_get_tuning(mlem_matrix* m, uint32_t transposed, int* ker
             *ms = f.ms;
             return;
         }
-        tune_projection(m, transposed != 0);
+        tune_projection(m, transposed != 0, true);
         const ProjCfg& c = m->proj[transposed];
         *kernel = c.kind;
         *lanes = c.lanes;
@@ -1493,7 +1541,7 @@ mlem_status mlem_run(mlem_matrix* m, const int32_t* g, const float* f0, uint32_t
         cudaStream_t s = m->stream;
         const uint32_t rows = m->A.nrows, cols = m->A.ncols;
         Workspace& w = m->ws;
-        if (o.spmv == MLEM_SPMV_CSR_VECTOR) prepare_kernel(m, o);
+        prepare_run(m, o, s);
         const bool perm = permuted(m);
         if (perm) {  // natural order staged, then permuted into the workspace
             int32_t* gt = reinterpret_cast<int32_t*>(w.tmp_rows);
@@ -1593,7 +1641,7 @@ mlem_status mlem_run_device(mlem_matrix* m, const int32_t* g_dev, float* f_dev, 
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         const uint32_t rows = m->A.nrows, cols = m->A.ncols;
         Workspace& w = m->ws;
-        if (o.spmv == MLEM_SPMV_CSR_VECTOR) prepare_kernel(m, o);
+        prepare_run(m, o, s);
         (void)rows;
         (void)cols;
         rows_in_i32(m, w.g, g_dev, s);
@@ -1614,7 +1662,7 @@ mlem_status mlem_forward_project(mlem_matrix* m, const float* f_dev, const int32
         std::lock_guard<std::mutex> lk(m->mu);
         DeviceGuard dg(m->device);
         cudaStream_t s = static_cast<cudaStream_t>(stream);
-        if (o.spmv == MLEM_SPMV_CSR_VECTOR) prepare_kernel(m, o);
+        if (o.spmv == MLEM_SPMV_CSR_VECTOR) prepare_kernel(m, o, true, false, s);
         EpiArgs fe;
         fe.kind = Epi::Correl;
         if (!permuted(m)) {
@@ -1661,7 +1709,7 @@ mlem_status mlem_back_project(mlem_matrix* m, const float* ratio_dev, float* bp_
             EpiArgs be;
             be.kind = Epi::Raw;
             be.out = out;
-            if (o.spmv == MLEM_SPMV_CSR_VECTOR) prepare_kernel(m, o);
+            if (o.spmv == MLEM_SPMV_CSR_VECTOR) prepare_kernel(m, o, false, true, s);
             project(m, true, r, be, o, {}, s);
         } else {
             MLEM_CUDA(cudaMemsetAsync(out, 0, sizeof(float) * m->A.ncols, s));

@@ -144,6 +144,7 @@ struct mlem_matrix {
     mlem::FusedForm fused_auto;       // fastest form of the fused pass (timed once; ms = 0: not yet)
     uint32_t one_call = 0;            // iterations of the only call this handle is made for (0: a caller's handle)
     bool tuned[2] = {false, false};   // csr-vector configuration of A / Aᵀ measured
+    bool copy_timed[2] = {false, false};  // ... with a delta-coded copy among the candidates
     mlem::ProjCfg proj[2];
     std::mutex mu;
     // Held while a run (under mu) changes what mlem_matrix_get_info reads, and by
@@ -155,7 +156,7 @@ struct mlem_matrix {
 namespace mlem {
 // Shared by the single, batched and server paths.
 void ensure_workspace(mlem_matrix* m);
-const MergePlan& merge_plan(mlem_matrix* m, bool transposed, uint32_t secsize);
+const MergePlan& merge_plan(mlem_matrix* m, bool transposed, uint32_t secsize, bool copy, cudaStream_t user_stream);
 // Form of the fused single pass for the run's options (timed once per matrix
 // where the options leave it open).
 FusedForm fused_form(mlem_matrix* m, const mlem_run_opts& o);
@@ -177,7 +178,7 @@ void enqueue_batch_iteration(mlem_matrix* m, BatchState& b, cudaStream_t s, uint
 float reference_initial_value(const mlem_matrix* m, const int32_t* g);
 void check_run_opts(const mlem_matrix* m, const mlem_run_opts& o);
 // Settles kernel attributes / occupancy of the selected variant (outside captures).
-void prepare_kernel(mlem_matrix* m, const mlem_run_opts& o);
+void prepare_kernel(mlem_matrix* m, const mlem_run_opts& o, bool reads_a, bool reads_at, cudaStream_t user_stream);
 // Reads and clears the workspace error flag; fails with MLEM_ETIMEOUT if set.
 void check_device_error(mlem_matrix* m, cudaStream_t s);
 // One projection of `op` (A or Aᵀ) with the kernel the options select.

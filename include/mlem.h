@@ -242,7 +242,8 @@ typedef enum {
                              An operand larger than L2 with ascending columns in every row also gets
                              a delta-coded copy (the D16 form: positions * (2 + value) bytes, rows
                              padded to 32 or 64 positions; ~1.1 * nnz positions where rows are long)
-                             on its first AUTO run (csr-vector or merge-based) if that takes at most
+                             on the first AUTO run or projection that reads it (csr-vector or
+                             merge-based; the fused pass and the scatter do not) if that takes at most
                              a quarter of the free memory and less than its nnz * (4 + value) bytes;
                              it is kept where it is the fastest and counts in
                              mlem_matrix_info.device_bytes */
