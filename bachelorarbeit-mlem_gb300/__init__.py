@@ -408,8 +408,9 @@ class Matrix:
         return out
 
     def tuning(self, transposed=False) -> dict:
-        """The csr-vector configuration the autotuner chose for A or Aᵀ
-        (transposed = 2: the form of the fused single pass)."""
+        """The fastest csr-vector configuration of A or Aᵀ that run options can name
+        (an AUTO run may use a copy of the tuner's own instead; transposed = 2: the
+        form of the fused single pass)."""
         k, ln, u, od, pp, ms = C.c_int(), C.c_int(), C.c_int(), C.c_int(), C.c_int(), C.c_float()
         _check(load_library().mlem_matrix_get_tuning(self._h, int(transposed), C.byref(k), C.byref(ln),
                                                      C.byref(u), C.byref(od), C.byref(pp), C.byref(ms)))

@@ -683,6 +683,7 @@ static void tune_projection(mlem_matrix* m, bool transposed, bool copy) {
             if (c.ms < best.ms) best = c;
         };
         for (ProjCfg& c : cand) time(c);
+        if (!known) m->named[transposed] = best;
         if (copy && !op.d16_asked()) {
             const bool made = try_copy_d16(m, op, s);  // a merge plan may have made one before
             std::vector<ProjCfg> more;
@@ -1412,8 +1413,8 @@ mlem_status mlem_matrix_get_tuning(mlem_matrix* m, uint32_t transposed, int* ker
             *ms = f.ms;
             return;
         }
-        tune_projection(m, transposed != 0, true);
-        const ProjCfg& c = m->proj[transposed];
+        tune_projection(m, transposed != 0, false);
+        const ProjCfg& c = m->named[transposed];
         *kernel = c.kind;
         *lanes = c.lanes;
         *unroll = c.unroll;

@@ -145,7 +145,8 @@ struct mlem_matrix {
     uint32_t one_call = 0;            // iterations of the only call this handle is made for (0: a caller's handle)
     bool tuned[2] = {false, false};   // csr-vector configuration of A / Aᵀ measured
     bool copy_timed[2] = {false, false};  // ... with a delta-coded copy among the candidates
-    mlem::ProjCfg proj[2];
+    mlem::ProjCfg proj[2];            // and what it is
+    mlem::ProjCfg named[2];           // the fastest that a caller's options can name: no tuner's copy
     std::mutex mu;
     // Held while a run (under mu) changes what mlem_matrix_get_info reads, and by
     // that query, which so waits for no run: workspace, plans, a tuner's copies.

@@ -166,11 +166,13 @@ typedef struct {
 } mlem_matrix_info;
 
 mlem_status mlem_matrix_get_info(const mlem_matrix* m, mlem_matrix_info* info);
-/* Configuration the autotuner chose for the csr-vector projection of A
- * (transposed = 0) or Aᵀ (1): kernel (mlem_kernel), lanes per row, vectors in
+/* Fastest configuration that the autotuner measured for the csr-vector
+ * projection of A (transposed = 0) or Aᵀ (1) among those that mlem_run_opts can
+ * name on this handle: kernel (mlem_kernel), lanes per row, vectors in
  * flight per lane, whether rows run in locality order, whether the row's
  * vector loads are software-pipelined, and the measured
- * milliseconds of one launch.  Tunes on first call if needed.
+ * milliseconds of one launch.  Tunes on first call if needed.  An AUTO run uses
+ * it, or a copy of the tuner's own where that is faster (MLEM_KERNEL_AUTO).
  * transposed = 2: the fused single pass (bp_mode 2) the AUTO switch picks —
  * kernel = the switch that selects that form (TMA staged, PERSISTENT
  * register, DIRECT / ordered rescan), lanes = lanes per row (staged: threads

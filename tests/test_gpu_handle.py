@@ -221,3 +221,22 @@ def test_captured_projection_after_other_runs(pkg, cuda, large, spmv):
     want = np.add.reduceat(val.astype(np.float64), rp[:-1].astype(np.int64))
     assert np.all(np.abs(got - want) <= 452 * 2.0**-24 * want)
     m.close()
+
+
+def test_tuning_names_a_configuration_that_runs(pkg, large):
+    """What get_tuning reports can be asked for, before and after a run that uses a
+    copy of the tuner's own, and asking makes no copy."""
+    rp, col, val, cols, g = large
+    kinds = {"direct": pkg.KERNEL_DIRECT, "tma": pkg.KERNEL_TMA, "persistent": pkg.KERNEL_PERSISTENT,
+             "d16": pkg.KERNEL_D16}
+    m = pkg.Matrix.from_csr(rp, col, val, cols)
+    before = m.device_bytes
+    for step in range(2):
+        for t in (m.tuning(False), m.tuning(True)):
+            assert 0 < t["ms"] < 1e3
+            kw = dict(lanes=t["lanes_per_row"], unroll=t["vectors_in_flight"]) if t["kernel"] != "tma" else {}
+            m.run(g, 1, kernel=kinds[t["kernel"]], pipeline=t["pipelined"], row_order=t["locality_order"], **kw)
+        if step == 0:
+            assert copies(m, before) == 0
+        m.run(g, 3)
+    m.close()
