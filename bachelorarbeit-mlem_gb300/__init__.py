@@ -131,6 +131,7 @@ _SIGS = {
     "mlem_matrix_destroy": (C.c_int, [_P]),
     "mlem_matrix_get_info": (C.c_int, [_P, _P]),
     "mlem_matrix_get_norm": (C.c_int, [_P, _P]),
+    "mlem_matrix_own_copies": (C.c_int, [_P, C.c_uint32, _P, _P]),
     "mlem_matrix_get_tuning": (C.c_int, [_P, C.c_uint32, _P, _P, _P, _P, _P, _P]),
     "mlem_matrix_get_transpose": (C.c_int, [_P, _P, _P, _P]),
     "mlem_matrix_get_csr": (C.c_int, [_P, _P, _P, _P]),
@@ -419,6 +420,15 @@ class Matrix:
             names = {0: "rescan", 1: "staged", 2: "register"}
         return {"kernel": names.get(k.value, k.value), "lanes_per_row": ln.value, "vectors_in_flight": u.value,
                 "locality_order": bool(od.value), "pipelined": bool(pp.value), "ms": ms.value}
+
+    def own_copies(self, allow: bool | None = None) -> tuple[int, int]:
+        """Device bytes of the delta-coded copies of A and Aᵀ that AUTO runs made for
+        themselves.  allow = False releases them and makes none from now on, True
+        allows them again, None (default) changes nothing."""
+        b, bt = C.c_uint64(), C.c_uint64()
+        _check(load_library().mlem_matrix_own_copies(self._h, 2 if allow is None else int(bool(allow)),
+                                                     C.byref(b), C.byref(bt)))
+        return b.value, bt.value
 
     def transpose(self):
         cp = np.zeros(self.cols + 1, np.uint64)

@@ -32,9 +32,14 @@ const char* get_error() { return t_error.c_str(); }
 
 [[noreturn]] void fail(mlem_status code, const std::string& msg) { throw Error{code, msg}; }
 
-void Workspace::release() {
+void Workspace::drop_graphs() {
     for (auto& kv : graphs) cudaGraphExecDestroy(kv.second);
     graphs.clear();
+    graph_nodes.clear();
+}
+
+void Workspace::release() {
+    drop_graphs();
     cudaFree(g);
     cudaFree(f);
     cudaFree(ratio);
@@ -96,11 +101,15 @@ static void free_csr(DevCsr& c) {
     c = DevCsr();
 }
 
+static uint64_t d16_bytes(const DevCsr& c) {
+    return 12ull * c.nrows + 8 + (sizeof(uint16_t) + val_bytes(c.vt)) * 8 * c.dvec;
+}
+
 static uint64_t csr_bytes(const DevCsr& c) {
     if (!c.rowptr) return 0;
     uint64_t b = sizeof(uint64_t) * ((uint64_t)c.nrows + 1) + sizeof(uint32_t) * padded(c.nnz) +
                  val_bytes(c.vt) * padded(c.nnz);
-    if (c.d16) b += 12ull * c.nrows + 8 + (sizeof(uint16_t) + val_bytes(c.vt)) * 8 * c.dvec;
+    if (c.d16) b += d16_bytes(c);
     if (c.idx_ilv) b += (sizeof(uint32_t) + val_bytes(c.vt)) * c.ilv_len;
     if (c.order) b += sizeof(uint32_t) * c.nrows;
     return b;
@@ -427,7 +436,7 @@ static void d16_cands(const DevCsr& op, std::vector<ProjCfg>& cand) {
 // times that: such an operand keeps its CSR arrays, and nothing is allocated).
 constexpr uint32_t kCopyPays = 100;
 static uint64_t copy_bytes_d16(const mlem_matrix* m, const DevCsr& op) {
-    if (op.d16 || m->sym.fp_rowptr || (m->one_call && m->one_call < kCopyPays)) return 0;
+    if (!m->copies || op.d16 || m->sym.fp_rowptr || (m->one_call && m->one_call < kCopyPays)) return 0;
     int l2 = 0;
     size_t avail = 0, total = 0;
     MLEM_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, m->device));
@@ -468,6 +477,11 @@ static void drop_copy_d16(mlem_matrix* m, DevCsr& op) {
     DevCsr c = op;
     set_copy_d16(m, op, DevCsr());
     free_d16(c);
+}
+
+// Bytes of an operand's copy that its tuner made.
+static uint64_t own_copy_bytes(const DevCsr& op) {
+    return op.d16 && op.d16_tuned ? d16_bytes(op) : 0;
 }
 
 static bool capturing(cudaStream_t s) {
@@ -551,7 +565,7 @@ const MergePlan& merge_plan(mlem_matrix* m, bool transposed, uint32_t secsize, b
     auto it = plans.find(secsize);
     if (it != plans.end()) {
         MergePlan& p = it->second;
-        if (copy && p.timed && !p.copy_timed && !capturing(user_stream)) tune_merge(m, op, p, true);
+        if (copy && !p.copy_timed && p.rows_kernel && op.nnz && !capturing(user_stream)) tune_merge(m, op, p, true);
         return p;
     }
     MergePlan p;
@@ -1421,6 +1435,37 @@ mlem_status mlem_matrix_get_tuning(mlem_matrix* m, uint32_t transposed, int* ker
         *ordered = c.ordered ? 1 : 0;
         *pipelined = c.pipelined ? 1 : 0;
         *ms = c.ms;
+    });
+}
+
+mlem_status mlem_matrix_own_copies(mlem_matrix* m, uint32_t allow, uint64_t* bytes, uint64_t* bytes_t) {
+    return guarded([&] {
+        MLEM_REQUIRE(m, MLEM_EINVAL, "NULL argument");
+        MLEM_REQUIRE(allow <= 2, MLEM_EINVAL, "allow must be 0 (none), 1 (allowed) or 2 (as it is)");
+        if (allow < 2) {
+            std::lock_guard<std::mutex> lk(m->mu);
+            DeviceGuard dg(m->device);
+            const bool change = m->copies != (allow == 1);
+            m->copies = allow == 1;
+            if (change && !m->copies) MLEM_CUDA(cudaDeviceSynchronize());  // runs on callers' streams read them
+            for (bool t : {false, true}) {
+                if (!change) break;
+                DevCsr& op = t ? m->AT : m->A;
+                m->proj[t] = m->named[t];
+                m->copy_timed[t] = false;
+                for (auto& kv : t ? m->plan_AT : m->plan_A) {
+                    MergePlan& p = kv.second;
+                    if (!op.d16_asked()) p.d16_u = 0;
+                    p.timed = p.copy_timed = false;
+                    p.ms = 1e30f;
+                }
+                if (own_copy_bytes(op)) drop_copy_d16(m, op);
+            }
+            if (change) m->ws.drop_graphs();  // captured with the copies, or without
+        }
+        std::lock_guard<std::mutex> lk(m->info_mu);
+        if (bytes) *bytes = own_copy_bytes(m->A);
+        if (bytes_t) *bytes_t = own_copy_bytes(m->AT);
     });
 }
 

@@ -70,6 +70,7 @@ struct Workspace {
     float* tmp_cols = nullptr; // [cols] staging in natural order (locality layout only)
     std::map<RunKey, cudaGraphExec_t> graphs;
     std::map<RunKey, uint64_t> graph_nodes;
+    void drop_graphs();
     void release();
 };
 
@@ -144,6 +145,7 @@ struct mlem_matrix {
     mlem::FusedForm fused_auto;       // fastest form of the fused pass (timed once; ms = 0: not yet)
     uint32_t one_call = 0;            // iterations of the only call this handle is made for (0: a caller's handle)
     bool tuned[2] = {false, false};   // csr-vector configuration of A / Aᵀ measured
+    bool copies = true;               // the tuners may make delta-coded copies (mlem_matrix_own_copies)
     bool copy_timed[2] = {false, false};  // ... with a delta-coded copy among the candidates
     mlem::ProjCfg proj[2];            // and what it is
     mlem::ProjCfg named[2];           // the fastest that a caller's options can name: no tuner's copy

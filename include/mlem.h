@@ -179,6 +179,13 @@ mlem_status mlem_matrix_get_info(const mlem_matrix* m, mlem_matrix_info* info);
  * per CTA), unroll and ordered as for the rescan form. */
 mlem_status mlem_matrix_get_tuning(mlem_matrix* m, uint32_t transposed, int* kernel, int* lanes,
                                    int* unroll, int* ordered, int* pipelined, float* ms);
+/* The delta-coded copies that AUTO runs make for themselves (MLEM_KERNEL_AUTO).
+ * allow = 0: releases them and makes none from now on, 1: allows them (the
+ * default), 2: changes nothing.  bytes / bytes_t (may be NULL) receive the device
+ * bytes of those of A / A^T held now.  0 waits for the device; as with
+ * mlem_matrix_destroy, no CUDA graph that the caller captured projections of this
+ * handle into may be replayed after it.  2 waits for no run. */
+mlem_status mlem_matrix_own_copies(mlem_matrix* m, uint32_t allow, uint64_t* bytes, uint64_t* bytes_t);
 /* Copies the sensitivity image (f32[cols]) to the host. */
 mlem_status mlem_matrix_get_norm(const mlem_matrix* m, float* norm_out);
 /* Copies the device-built transpose to the host: colptr u64[cols+1],
@@ -247,8 +254,9 @@ typedef enum {
                              on the first AUTO run or projection that reads it (csr-vector or
                              merge-based; the fused pass and the scatter do not) if that takes at most
                              a quarter of the free memory and less than its nnz * (4 + value) bytes;
-                             it is kept where it is the fastest and counts in
-                             mlem_matrix_info.device_bytes */
+                             it is kept where it is the fastest, counts in
+                             mlem_matrix_info.device_bytes and can be released or ruled out with
+                             mlem_matrix_own_copies */
     MLEM_KERNEL_D16 = 4,  /* delta-coded indices (matrix created with compress_indices = 1) */
     MLEM_KERNEL_ILV = 5,  /* lane-interleaved copy (matrix created with interleave = 1) */
     MLEM_KERNEL_ORDERED = 6, /* DIRECT with rows in locality order (generated matrices:

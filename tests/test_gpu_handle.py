@@ -240,3 +240,38 @@ def test_tuning_names_a_configuration_that_runs(pkg, large):
             assert copies(m, before) == 0
         m.run(g, 3)
     m.close()
+
+
+def test_own_copies_can_be_ruled_out(pkg, large):
+    """Without them a handle takes no more than its arrays, workspace and plans, and
+    its images are those of the configurations that options can name; released and
+    allowed again, AUTO runs make them anew."""
+    rp, col, val, cols, g = large
+    m = pkg.Matrix.from_csr(rp, col, val, cols)
+    before = m.device_bytes
+    assert m.own_copies(False) == (0, 0)
+    plain = m.run(g, 40)
+    assert m.own_copies() == (0, 0) and copies(m, before) == 0
+    t, tt = m.tuning(False), m.tuning(True)
+    merge = m.run(g, 40, spmv=pkg.SPMV_MERGE)
+    np.testing.assert_array_equal(merge, m.run(g, 40, spmv=pkg.SPMV_MERGE, kernel=pkg.KERNEL_DIRECT))
+    assert m.own_copies(True) == (0, 0)
+    auto = m.run(g, 40)
+    held = m.own_copies()
+    assert (m.tuning(False), m.tuning(True)) == (t, tt)
+    assert np.linalg.norm(auto - plain) <= 1e-5 * np.linalg.norm(plain)
+    auto_merge = m.run(g, 40, spmv=pkg.SPMV_MERGE)
+    assert np.linalg.norm(auto_merge - merge) <= 1e-5 * np.linalg.norm(merge)
+    held = m.own_copies()
+    assert m.own_copies(False) == (0, 0)
+    np.testing.assert_array_equal(m.run(g, 40), plain)
+    np.testing.assert_array_equal(m.run(g, 40, spmv=pkg.SPMV_MERGE), merge)
+    assert copies(m, before) < len(col)  # merge plans
+    m.close()
+    m = pkg.Matrix.from_csr(rp, col, val, cols, compress=True)  # asked for: not the tuner's own
+    m.run(g, 2)
+    assert m.own_copies(False) == (0, 0)
+    m.run(g, 2, kernel=pkg.KERNEL_D16)
+    m.close()
+    if not all(held):
+        pytest.skip("the tuners kept the CSR arrays on this GPU: no copy was released")
