@@ -484,6 +484,11 @@ static uint64_t own_copy_bytes(const DevCsr& op) {
     return op.d16 && op.d16_tuned ? d16_bytes(op) : 0;
 }
 
+uint64_t own_copies_bytes(const mlem_matrix* m) {
+    std::lock_guard<std::mutex> lk(m->info_mu);
+    return own_copy_bytes(m->A) + own_copy_bytes(m->AT);
+}
+
 static bool capturing(cudaStream_t s) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;

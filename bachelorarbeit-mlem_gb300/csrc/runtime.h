@@ -160,6 +160,8 @@ namespace mlem {
 // Shared by the single, batched and server paths.
 void ensure_workspace(mlem_matrix* m);
 const MergePlan& merge_plan(mlem_matrix* m, bool transposed, uint32_t secsize, bool copy, cudaStream_t user_stream);
+// Device bytes of the handle's delta-coded copies that its tuners made.
+uint64_t own_copies_bytes(const mlem_matrix* m);
 // Form of the fused single pass for the run's options (timed once per matrix
 // where the options leave it open).
 FusedForm fused_form(mlem_matrix* m, const mlem_run_opts& o);

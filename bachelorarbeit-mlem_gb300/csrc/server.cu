@@ -310,6 +310,7 @@ struct MatrixSlots {
     std::vector<uint64_t> slot_req;   // 0 = free
     std::vector<uint32_t> slot_left;
     uint32_t tile = 0;
+    uint64_t copies0 = 0;             // own_copies_bytes(m) when the matrix was added
     PinnedPool pin_g, pin_f;          // staging of sinograms in and images out
     bool active() const { return active_slots() > 0; }
     // one past the highest occupied slot
@@ -378,7 +379,16 @@ bool mlem_server::admit_locked() {
         }
         if (!ms.allocated) {
             const uint64_t need = batch_state_bytes(rows, cols, ms.tile, !ms.m->has_t);
-            if (in_use + need > budget) {
+            // the measured budget (free memory at creation) shrinks by copies that
+            // runs on the served handles have made since they were added; a request
+            // with no other state to wait for is tried all the same
+            auto over = [&] {
+                uint64_t taken = 0;
+                if (!opts.hbm_budget_bytes && in_use)
+                    for (auto& o : mats) taken += std::max(own_copies_bytes(o.m), o.copies0) - o.copies0;
+                return in_use + taken + need > budget;
+            };
+            if (over()) {
                 // release the state of idle matrices, then retry once
                 for (auto& o : mats)
                     if (o.allocated && !o.inflight && !o.active()) {
@@ -387,7 +397,7 @@ bool mlem_server::admit_locked() {
                         o.bs.release();
                         o.allocated = false;
                     }
-                if (in_use + need > budget) {
+                if (over()) {
                     ++it;
                     continue;
                 }
@@ -774,6 +784,7 @@ mlem_status mlem_server_add_matrix(mlem_server* s, mlem_matrix* m, uint32_t* mat
         s->device = m->device;
         MatrixSlots ms;
         ms.m = m;
+        ms.copies0 = own_copies_bytes(m);
         DeviceGuard dg(m->device);
         // slots per matrix: fixed by the options, or the batch tile the
         // autotuner finds best for this matrix (the image tile of a large

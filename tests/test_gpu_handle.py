@@ -275,3 +275,28 @@ def test_own_copies_can_be_ruled_out(pkg, large):
     m.close()
     if not all(held):
         pytest.skip("the tuners kept the CSR arrays on this GPU: no copy was released")
+
+
+def test_server_budget_counts_copies_made_later(pkg, cuda, large):
+    """A server whose measured budget holds the slot state of two matrices, but no
+    longer once a run on one of them has made its copies: the two take turns."""
+    rp, col, val, cols, g = large
+    ms = [pkg.Matrix.from_csr(rp, col, val, cols) for _ in range(2)]
+    state = 8 * 8 * ms[0].rows + 8 * 4 * cols + 4 * (ms[0].rows + cols) + 192
+    cuda.cuda.synchronize()
+    free = cuda.cuda.mem_get_info()[0]
+    srv = pkg.Server(slots_per_matrix=8, hbm_reserve_bytes=free - 3 * state)
+    ids = [srv.add_matrix(m) for m in ms]
+    want = [m.batch_run(g[None], [300])[0] for m in ms]
+    ms[0].run(g, 2)
+    made = sum(ms[0].own_copies())
+    with Sampler(lambda: srv.stats()["hbm_in_use"]) as s:
+        reqs = [srv.submit(i, g, 300) for i in ids]
+        for r, w in zip(reqs, want):
+            np.testing.assert_array_equal(srv.wait(r, timeout_ms=60_000)[0], w)
+    srv.close()
+    for m in ms:
+        m.close()
+    if made < 3 * state:
+        pytest.skip("the tuners kept the CSR arrays on this GPU: the budget was not touched")
+    assert max(s.seen) == state
