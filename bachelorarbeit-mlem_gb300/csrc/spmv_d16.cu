@@ -101,7 +101,12 @@ __device__ __forceinline__ float lane_sum(const float* acc) {
 }
 
 // A row's sum again, in the same order, without the dummies and the padding, by
-// one thread: for rows whose sum is NaN (see the head of the file).
+// one thread: for rows whose sum is NaN (see the head of the file).  It ends as
+// soon as a lane's sum is NaN, as the row's then is: where the image holds NaN,
+// after a few entries.  An iteration of the 12 GB class on an image of NaN 2.99 ms
+// (FP16 values 2.31), walking every row to its end 29.3 (29.5); on an ordinary
+// image 2.79 (2.04).  Measured and not kept: by the row's group of lanes, which
+// needs no early end, but the call costs ordinary images 2% with FP16 values.
 template <typename V, int LPR>
 __device__ __noinline__ float d16_row_real(const uint64_t* __restrict__ dvptr, const uint32_t* __restrict__ dbase,
                                            const uint16_t* __restrict__ d16, const V* __restrict__ dval,
@@ -111,12 +116,14 @@ __device__ __noinline__ float d16_row_real(const uint64_t* __restrict__ dvptr, c
     for (int l = 0; l < LPR; ++l) {
         uint32_t col = dbase[row];
         float acc[kSums<LPR>] = {};
-        for (uint64_t v = v0 + l; v < v1; v += LPR)
+        for (uint64_t v = v0 + l; v < v1; v += LPR) {
             for (int j = 0; j < 8; ++j) {
                 col += d16[8 * v + j];
                 const float a = (float)dval[8 * v + j];
                 if (__float_as_uint(a) != 0x80000000u) acc[j % kSums<LPR>] = fmaf(a, ld_after(x + col), acc[j % kSums<LPR>]);
             }
+            if (isnan(lane_sum<LPR>(acc))) return lane_sum<LPR>(acc);  // as it will be whatever follows
+        }
         sum[l] = lane_sum<LPR>(acc);
     }
     for (int o = LPR / 2; o > 0; o >>= 1)

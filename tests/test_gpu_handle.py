@@ -300,3 +300,52 @@ def test_server_budget_counts_copies_made_later(pkg, cuda, large):
     if made < 3 * state:
         pytest.skip("the tuners kept the CSR arrays on this GPU: the budget was not touched")
     assert max(s.seen) == state
+
+
+@pytest.mark.parametrize("spmv", [0, 1])
+def test_image_of_nan_is_not_slow(pkg, large, spmv):
+    """Rows whose sum is NaN are summed a second time over the delta-coded copy: at
+    most a few times the time of an ordinary image."""
+    rp, col, val, cols, g = large
+    m = pkg.Matrix.from_csr(rp, col, val, cols)
+    t = []
+    for f0 in (np.ones(cols, np.float32), np.full(cols, np.nan, np.float32)):
+        m.run(g, 40, f0=f0, spmv=spmv)
+        t.append(min(m.run(g, 40, f0=f0, spmv=spmv, stats=True)[1]["seconds_iterations"] for _ in range(3)))
+    print(f"\nordinary {1e3 * t[0]:.2f} ms, NaN {1e3 * t[1]:.2f} ms")
+    assert t[1] < 4 * t[0]
+    m.close()
+
+
+@pytest.mark.parametrize("vt", [0, 1])
+def test_rows_of_infinities_over_the_copy(pkg, cuda, vt):
+    """NaN sums that arise late in a row: infinities of both signs in entries of
+    different lanes and steps, zeros times infinity, beside rows where only a
+    dummy or the padding meets one."""
+    rng = np.random.default_rng(12)
+    cols, n = 400_000, 300
+    rows = [np.sort(rng.choice(cols, n, replace=False)) for _ in range(400)]
+    rp = (np.arange(401) * n).astype(np.uint64)
+    col = np.concatenate(rows).astype(np.uint32)
+    val = rng.uniform(0.05, 1.0, len(col)).astype(np.float32)
+    val[rng.random(len(col)) < 0.02] = 0.0
+    x = rng.uniform(0.5, 1.5, cols).astype(np.float32)
+    x[rng.choice(cols, 1500, replace=False)] = np.inf
+    x[rng.choice(cols, 300, replace=False)] = -np.inf
+    m = pkg.Matrix.from_csr(rp, col, val, cols, value_type=vt, build_transpose=False, compress=True)
+    dx, g = cuda.from_numpy(x).cuda(), cuda.zeros(400, dtype=cuda.int32, device="cuda")
+    out = []
+    for kw in (dict(kernel=pkg.KERNEL_D16, unroll=1), dict(kernel=pkg.KERNEL_D16, unroll=2),
+               dict(kernel=pkg.KERNEL_D16, spmv=pkg.SPMV_MERGE, secsize_fp=64), dict(kernel=pkg.KERNEL_DIRECT)):
+        ratio, fp = cuda.empty(400, device="cuda"), cuda.empty(400, device="cuda")
+        m.forward_project(dx.data_ptr(), g.data_ptr(), ratio.data_ptr(), fp.data_ptr(), bp_mode=pkg.BP_SCATTER, **kw)
+        cuda.cuda.synchronize()
+        out.append(fp.cpu().numpy())
+    want = out.pop()
+    assert np.isnan(want).sum() > 20 and np.isposinf(want).sum() > 20 and np.isneginf(want).sum() > 5
+    assert np.isfinite(want).sum() > 20
+    for got in out:
+        np.testing.assert_array_equal(np.isnan(got), np.isnan(want))
+        np.testing.assert_array_equal(got[np.isinf(want)], want[np.isinf(want)])
+        np.testing.assert_allclose(got[np.isfinite(want)], want[np.isfinite(want)], rtol=302 * 2.0**-24)
+    m.close()
