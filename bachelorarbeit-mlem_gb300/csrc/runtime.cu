@@ -36,6 +36,7 @@ void Workspace::drop_graphs() {
     for (auto& kv : graphs) cudaGraphExecDestroy(kv.second);
     graphs.clear();
     graph_nodes.clear();
+    last_rest.clear();
 }
 
 void Workspace::release() {
@@ -973,13 +974,18 @@ static uint32_t run_iterations(mlem_matrix* m, const mlem_run_opts& o, uint32_t 
         }
         return iters;
     }
-    // 32 iterations per graph and one graph of what is left (at most 32 graphs
-    // per set of options): 50 iterations of the 2-D ring take two launches; as
-    // six graphs of 8 and two of 1 they took 3% longer
+    // Graphs of 32, 16, 8, 4, 2 and 1 iterations, the rest of a run as its binary
+    // parts, so that a count not run before captures none of its own: a capture
+    // takes 0.1 to 0.8 ms, a further launch 3 us.  For the caller who always runs
+    // one count, the first rest and one that comes twice in a row get a graph (31
+    // iterations of the 2-D ring 219 us in one graph, 234 in five).
     constexpr uint32_t kChunk = 32;
+    auto key_of = [&](uint32_t chunk) {
+        return RunKey{(int)o.spmv, (int)o.bp_mode, (int)o.secsize_fp, (int)o.secsize_bp, (int)o.l2_window, (int)chunk,
+                      (int)(o.kernel | o.lanes << 8 | o.unroll << 16 | o.row_order << 24 | o.pipeline << 25)};
+    };
     auto get_graph = [&](uint32_t chunk) -> cudaGraphExec_t {
-        RunKey key{(int)o.spmv, (int)o.bp_mode, (int)o.secsize_fp, (int)o.secsize_bp, (int)o.l2_window,
-                   (int)chunk, (int)(o.kernel | o.lanes << 8 | o.unroll << 16 | o.row_order << 24 | o.pipeline << 25)};
+        const RunKey key = key_of(chunk);
         auto it = m->ws.graphs.find(key);
         if (it != m->ws.graphs.end()) return it->second;
         // plans and kernel attributes must exist before capture
@@ -1014,19 +1020,24 @@ static uint32_t run_iterations(mlem_matrix* m, const mlem_run_opts& o, uint32_t 
         m->ws.graph_nodes[key] = nodes;
         return exec;
     };
-    const uint32_t full = iters / kChunk, rest = iters % kChunk;
     auto replay = [&](uint32_t chunk, uint32_t times) {
         cudaGraphExec_t ge = get_graph(chunk);
-        const RunKey key{(int)o.spmv, (int)o.bp_mode, (int)o.secsize_fp, (int)o.secsize_bp,
-                         (int)o.l2_window, (int)chunk, (int)(o.kernel | o.lanes << 8 | o.unroll << 16 | o.row_order << 24 | o.pipeline << 25)};
+        const RunKey key = key_of(chunk);
         const uint64_t nodes = m->ws.graph_nodes[key];
         for (uint32_t q = 0; q < times; ++q) {
             MLEM_CUDA(cudaGraphLaunch(ge, s));
             count_launch(nodes);
         }
     };
-    if (full) replay(kChunk, full);
-    if (rest) replay(rest, 1);
+    const uint32_t rest = iters % kChunk;
+    const auto last = m->ws.last_rest.emplace(key_of(0), rest).first;
+    const bool whole = last->second == rest || m->ws.graphs.count(key_of(rest));
+    last->second = rest;
+    if (iters >= kChunk) replay(kChunk, iters / kChunk);
+    if (rest && whole) replay(rest, 1);
+    else
+        for (uint32_t part = kChunk / 2; part; part /= 2)
+            if (rest & part) replay(part, 1);
     return iters;
 }
 

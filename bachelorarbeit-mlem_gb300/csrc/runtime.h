@@ -70,6 +70,7 @@ struct Workspace {
     float* tmp_cols = nullptr; // [cols] staging in natural order (locality layout only)
     std::map<RunKey, cudaGraphExec_t> graphs;
     std::map<RunKey, uint64_t> graph_nodes;
+    std::map<RunKey, uint32_t> last_rest;  // by options (chunk 0): iterations past the last whole chunk, last run
     void drop_graphs();
     void release();
 };

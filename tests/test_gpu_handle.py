@@ -5,6 +5,7 @@ from __future__ import annotations
 
 import ctypes as C
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -348,4 +349,31 @@ def test_rows_of_infinities_over_the_copy(pkg, cuda, vt):
         np.testing.assert_array_equal(np.isnan(got), np.isnan(want))
         np.testing.assert_array_equal(got[np.isinf(want)], want[np.isinf(want)])
         np.testing.assert_allclose(got[np.isfinite(want)], want[np.isfinite(want)], rtol=302 * 2.0**-24)
+    m.close()
+
+
+def test_iteration_counts_share_graphs(pkg):
+    """Images of any count are those of launches one by one, and on a handle that has
+    run a few counts (graphs of 32, 16, 8, 4, 2 and 1 iterations) another captures
+    no graph in its first run, which takes about what its later ones take."""
+    m = pkg.Matrix.generate(pkg.preset("ring2d"))
+    g = np.random.default_rng(3).poisson(20.0, m.rows).astype(np.int32)
+    f0 = np.ones(m.cols, np.float32)
+    first = m.run(g, 63, f0=f0)
+    np.testing.assert_array_equal(m.run(g, 63, f0=f0, use_graph=False), first)
+    for n in (1, 2, 5, 31, 32, 33, 64, 70):
+        np.testing.assert_array_equal(m.run(g, n, f0=f0), m.run(g, n, f0=f0, use_graph=False))
+    m.close()
+    m = pkg.Matrix.generate(pkg.preset("ring2d"))
+    for n in (63, 30, 29):
+        m.run(g, n, f0=f0)
+    rel = []
+    for n in range(1, 32):
+        ts = []
+        for _ in range(6):
+            t0 = time.perf_counter()
+            m.run(g, n, f0=f0)
+            ts.append(time.perf_counter() - t0)
+        rel.append(ts[0] / min(ts[1:]))
+    assert np.median(rel) < 1.5
     m.close()
