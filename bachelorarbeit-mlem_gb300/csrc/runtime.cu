@@ -593,12 +593,19 @@ const MergePlan& merge_plan(mlem_matrix* m, bool transposed, uint32_t secsize, b
 // Times the candidate configurations on the operand itself (Raw epilogue into
 // a scratch vector, constant x) and keeps the fastest.  A candidate that its
 // first launch shows to be a quarter slower than the best so far gets no
-// further ones; short kernels are timed from a graph.  Runs once per operand, outside any stream capture.  A handle
-// made for one call tries the plain kernel with three lane counts only: the
-// other forms are within a few percent of it, and timing them all takes longer
-// than 100 iterations (30 M nonzeros: 12.2 ms for both operands; 1.0 ms so).
+// further ones; short kernels are timed from a graph.  Runs once per operand,
+// outside any stream capture.  A handle made for one call tries the plain kernel
+// with three lane counts only: the other forms are within a few percent of it,
+// and timing them all takes longer than 100 iterations (30 M nonzeros: 12.2 ms for
+// both operands; 1.0 ms so).  For its short kernels, where one launch tells
+// nothing and 16 from a graph take 0.2 ms, a rule: the lanes of the mean row
+// length, doubled while the launch keeps within half of the threads that the GPU
+// holds.  A call of 20 / 1,000 / 5,000 iterations, 14 k nonzeros: 0.65 / 4.2 / 18.5
+// ms by rule, 1.45 / 5.0 / 19.4 timed from graphs, 0.86 / 4.9-5.5 / 20-24 by single
+// launches; 0.5 M: 1.04 / 8.6 / 38.6, 2.5 / 9.9-11.1 / 41-45, 1.22 / 8.7-10.1 / 38-44.
 // copy: the caller's projections read this operand, so that it may get a
 // delta-coded copy (try_copy_d16), now or where it was tuned without before.
+constexpr uint64_t kShort = 4ull << 20;  // nonzeros; a projection of fewer takes under 10 us
 static void tune_projection(mlem_matrix* m, bool transposed, bool copy) {
     const bool known = m->tuned[transposed];
     if (known && (!copy || m->copy_timed[transposed])) return;
@@ -606,7 +613,19 @@ static void tune_projection(mlem_matrix* m, bool transposed, bool copy) {
     cudaStream_t s = m->stream;
     std::vector<ProjCfg> cand;
     const int base = pick_lanes(op.nnz, op.nrows);
-    const bool brief = m->one_call != 0;
+    const bool brief = m->one_call != 0, is_short = op.nnz <= kShort;
+    if (known && !op.d16 && !copy_bytes_d16(m, op)) {
+        m->copy_timed[transposed] = true;
+        return;
+    }
+    if (brief && is_short) {
+        ProjCfg c;
+        c.lanes = base;
+        while (c.lanes < 32 && (uint64_t)op.nrows * c.lanes * 2 <= 152u * 1024u) c.lanes *= 2;
+        m->proj[transposed] = m->named[transposed] = c;
+        m->tuned[transposed] = m->copy_timed[transposed] = true;
+        return;
+    }
     for (int lanes : {base / 2, base, base * 2})
         if (!known && lanes >= 4 && lanes <= 32) {
             if (brief) {
@@ -650,7 +669,6 @@ static void tune_projection(mlem_matrix* m, bool transposed, bool copy) {
         e.kind = Epi::Raw;
         e.out = y;
         const int reps = brief ? 1 : op.nnz > (50ull << 20) ? 2 : 4;
-        constexpr uint64_t kShort = 4ull << 20;  // nonzeros; a projection of fewer takes under 10 us
         auto launches = [&](const ProjCfg& c, int n) {  // milliseconds of one launch, the mean of n
             MLEM_CUDA(cudaEventRecord(e0, s));
             for (int r = 0; r < n; ++r) launch_cfg(m, op, x, e, c, {}, s);
@@ -698,7 +716,7 @@ static void tune_projection(mlem_matrix* m, bool transposed, bool copy) {
         auto time = [&](ProjCfg& c) {
             launch_cfg(m, op, x, e, c, {}, s);  // warm-up
             c.ms = launches(c, 1);
-            if (!brief && op.nnz <= kShort) c.ms = replayed(c, 16);
+            if (is_short) c.ms = replayed(c, 16);
             else if (reps > 1 && c.ms < 1.25f * best.ms) c.ms = launches(c, reps);
             if (c.ms < best.ms) best = c;
         };

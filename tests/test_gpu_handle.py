@@ -377,3 +377,24 @@ def test_iteration_counts_share_graphs(pkg):
         rel.append(ts[0] / min(ts[1:]))
     assert np.median(rel) < 1.5
     m.close()
+
+
+@pytest.mark.parametrize("name", ["ring2d", "cyl3d_tiny"])
+def test_one_call_reconstruction_is_not_left_to_chance(pkg, name):
+    """The kernels of a call on a small matrix follow from the matrix, not from a
+    timing: every call gives the same bits and takes about the same time."""
+    m = pkg.Matrix.generate(pkg.preset(name))
+    rp, col, val = m.csr()
+    norm, rows, cols = m.norm(), m.rows, m.cols
+    m.close()
+    g = np.random.default_rng(3).poisson(20.0, rows).astype(np.int32)
+    f0, out, ts = np.ones(cols, np.float32), [], []
+    for _ in range(8):
+        f = np.empty(cols, np.float32)
+        t0 = time.perf_counter()
+        pkg.mlem(rp, col, val, None, None, None, g, norm, f0, f, rows, cols, len(col), 2000, 1, 1, 5, 5, 0)
+        ts.append(time.perf_counter() - t0)
+        out.append(f)
+    for f in out[1:]:
+        np.testing.assert_array_equal(f, out[0])
+    assert np.median(ts) < 1.1 * min(ts)
