@@ -317,7 +317,7 @@ struct BatchArgs {
     float* f = nullptr;
     float* ratio = nullptr;
     uint32_t* remaining = nullptr;
-    // slots the projections cover: the smallest power of two >= active, 4..tile
+    // lanes of a row's segment in the projections: the smallest power of two >= active, 4..tile
     uint32_t width() const {
         const uint32_t a = active ? std::min(active, tile) : tile;
         uint32_t w = 4;
@@ -327,22 +327,15 @@ struct BatchArgs {
     // slots whose state the projections read and write: `active` rounded up to 4
     uint32_t slots() const { return (std::min(active ? active : tile, tile) + 3) / 4 * 4; }
 };
-// Slots the projections cover for `active` leading slots in a tile (4..tile).
-inline uint32_t batch_width(uint32_t tile, uint32_t active) {
-    BatchArgs a;
-    a.tile = tile;
-    a.active = active;
-    return a.width();
-}
 // `steps` whole iterations of the tile (FP, BP + update, tick) in one
 // persistent cooperative launch with grid-wide barriers; count (one word,
 // zeroed here before the launch) carries the barriers, *err becomes 1 if a
 // barrier wait ran out (the launch then ends early).  Needs Aᵀ.
 void launch_batch_loop(const DevCsr& A, const DevCsr& AT, const float* norm, const BatchArgs& b, uint32_t steps,
                        unsigned* count, int* err, cudaStream_t s);
-// ratio[r][b] = g[r][b] / (A f_b)[r] for the slots b < width().
+// ratio[r][b] = g[r][b] / (A f_b)[r] for the slots b < slots().
 void launch_batch_fp(const DevCsr& A, const BatchArgs& b, L2Window win, cudaStream_t s);
-// f_b = f_b * (Aᵀ ratio_b) / norm for slots b < width() with remaining > 0.
+// f_b = f_b * (Aᵀ ratio_b) / norm for slots b < slots() with remaining > 0.
 void launch_batch_bp_update(const DevCsr& AT, const float* norm, const BatchArgs& b,
                             L2Window win, cudaStream_t s);
 // remaining[b] -= 1 where positive.

@@ -137,8 +137,9 @@ struct mlem_matrix {
     mlem::Workspace ws;
     std::map<uint32_t, mlem::MergePlan> plan_A, plan_AT;
     uint32_t batch_tile = 0;          // autotuned batch tile (0 = not yet)
-    float batch_ms[3][8] = {};        // and the iteration times behind it: tile 8 / 16 / 32, slots 4 .. 32 by 4
-    uint32_t batch_form = 0;          // autotuned batch form: 1 graphs, 2 persistent (0 = not yet)
+    float batch_ms[3][8] = {};        // and the iteration times behind it: tile 8 / 16 / 32, slots 4 .. 32 by 4 (those
+                                      // of 12 and 20 .. 28 are those of 16 and 32)
+    uint32_t batch_form[3] = {};      // autotuned batch form of tile 8 / 16 / 32: 1 graphs, 2 persistent (0 = not yet)
     int scatter_lanes = 0;            // autotuned lanes per row of the scatter back projection (0 = not yet)
     int scatter_unroll = 4;           // and its entries per lane in flight
     bool scatter_tma = false;         // the TMA-ring scatter timed faster than those lanes

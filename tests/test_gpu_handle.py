@@ -398,3 +398,20 @@ def test_one_call_reconstruction_is_not_left_to_chance(pkg, name):
     for f in out[1:]:
         np.testing.assert_array_equal(f, out[0])
     assert np.median(ts) < 1.1 * min(ts)
+
+
+def test_batch_form_belongs_to_its_tile(pkg):
+    """The form of a batch, graphs or the persistent kernel (which shows in the number
+    of launches), is measured at the batch's own tile, whatever ran before on the
+    handle.  On this matrix (1 M nonzeros, 784,000 voxels) 8 slots are 24% faster
+    with graphs, 32 slots 12% faster with the persistent kernel."""
+    geo = pkg.preset("cyl3d_mid", row_stride=200)
+    G = np.random.default_rng(2).poisson(30.0, (32, 3315)).astype(np.int32)
+    out = {}
+    for tiles in ((8, 32), (32, 8)):
+        m = pkg.Matrix.generate(geo, layout=pkg.LAYOUT_LOCALITY)
+        for t in tiles:
+            m.batch_run(G[:t], [12] * t, tile=t)  # times the forms
+            out.setdefault(t, []).append(m.batch_run(G[:t], [12] * t, tile=t, stats=True)[1]["kernel_launches"])
+        m.close()
+    assert out[8][0] == out[8][1] and out[32][0] == out[32][1]
