@@ -16,10 +16,12 @@
 // the slot, so an instance gives the same bits alone and in a full batch, in
 // any tile.
 //
-// What bounds it: a nonzero's gather of the slots' state, one 128-byte line
-// with 32 slots, and with it the L1 data pipe.  Handing 32 coalesced entries
-// round with shuffles, as an earlier form did, put 2 shuffles on that pipe for
-// every 4 nonzeros: one iteration of the 3-D mid matrix with 4 / 8 / 16 / 32
+// What bounds it: the latency of a nonzero's gather of the slots' state, one
+// 128-byte line with 32 slots, mostly from L2 (28% L1 hits in the forward, 68% in
+// the back projection), at the 67-71% of the warps that 40 registers leave; no
+// unit is saturated (L1 data pipe 65-67%, issue 35%).  Handing 32 coalesced entries
+// round with shuffles, as an earlier form did, put 2 shuffles on the L1 data pipe
+// for every 4 nonzeros: one iteration of the 3-D mid matrix with 4 / 8 / 16 / 32
 // slots 1.28 / 1.38 / 2.01 / 3.25 -> 1.19 / 1.35 / 1.88 / 3.12 ms (FP16 values 1.28 /
 // 1.36 / 1.97 / 3.22 -> 1.14 / 1.30 / 1.87 / 2.98), of a matrix of 6 M nonzeros 0.134 /
 // 0.136 / 0.200 / 0.310 -> 0.131 / 0.136 / 0.181 / 0.278 ms; 24 sinograms of 5 to 20

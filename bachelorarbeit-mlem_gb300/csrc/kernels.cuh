@@ -175,10 +175,10 @@ struct MergePlan {
     uint64_t ntiles = 0;
     uint32_t* tile_i = nullptr;   // [ntiles+1]
     uint64_t* tile_j = nullptr;   // [ntiles+1]
-    float* carry = nullptr;       // [ntiles]
+    float* carry = nullptr;       // [ntiles]; with carry_row and head only where tiles share rows
     uint32_t* carry_row = nullptr;// [ntiles]
     float* head = nullptr;        // [ntiles]
-    size_t smem = 0;
+    size_t smem = 0;              // per-thread walk only
     // true: the row-parallel tile kernel (library-owned, padded operands);
     // false: the per-thread walk over shared-memory products (any arrays)
     bool rows_kernel = false;

@@ -483,35 +483,13 @@ void merge_plan_build(const DevCsr& op, uint32_t secsize, MergePlan& plan, cudaS
     plan.whole = op.max_row <= TS;
     plan.ntiles = (items + TS - 1) / TS;
     MLEM_REQUIRE(plan.ntiles < (1ull << 31), MLEM_EUNSUPPORTED, "merge path: too many tiles");
-    plan.smem = 0;
     const uint64_t nt = std::max<uint64_t>(plan.ntiles, 1);
     MLEM_CUDA(cudaMalloc(&plan.tile_i, sizeof(uint32_t) * (nt + 1)));
     MLEM_CUDA(cudaMalloc(&plan.tile_j, sizeof(uint64_t) * (nt + 1)));
-    MLEM_CUDA(cudaMalloc(&plan.carry, sizeof(float) * nt));
-    MLEM_CUDA(cudaMalloc(&plan.carry_row, sizeof(uint32_t) * nt));
-    MLEM_CUDA(cudaMalloc(&plan.head, sizeof(float) * nt));
-    // Opt in to the tile's shared memory outside any stream capture.  The
-    // attribute belongs to the kernel, which all plans of a value type share,
-    // so it only ever grows.
-    {
-        static std::mutex mu;
-        static std::map<int, size_t> cur;  // (device * 4 + value type) -> bytes
-        std::lock_guard<std::mutex> lk(mu);
-        int dev = 0;
-        cudaGetDevice(&dev);
-        const int t = dev * 4 + (int)op.vt;
-        if (plan.smem > cur[t]) {
-            cudaError_t e;
-            if (op.vt == MLEM_VAL_F32)
-                e = cudaFuncSetAttribute(k_merge_tile<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem);
-            else if (op.vt == MLEM_VAL_F16)
-                e = cudaFuncSetAttribute(k_merge_tile<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem);
-            else
-                e = cudaFuncSetAttribute(k_merge_tile<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)plan.smem);
-            MLEM_CUDA(e);
-            cur[t] = plan.smem;
-        }
+    if (!plan.whole) {
+        MLEM_CUDA(cudaMalloc(&plan.carry, sizeof(float) * nt));
+        MLEM_CUDA(cudaMalloc(&plan.carry_row, sizeof(uint32_t) * nt));
+        MLEM_CUDA(cudaMalloc(&plan.head, sizeof(float) * nt));
     }
     const unsigned grid = std::max(1u, std::min<unsigned>(ceil_div_u(plan.ntiles + 1, 256), 152u * 16u));
     k_tile_coords<<<grid, 256, 0, s>>>(op.rowptr, op.nrows, op.nnz, TS, plan.ntiles, plan.whole, plan.tile_i,

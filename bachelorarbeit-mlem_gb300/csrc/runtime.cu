@@ -1271,8 +1271,8 @@ using namespace mlem;
 
 uint64_t mlem_matrix::bytes() const {
     uint64_t b = csr_bytes(A) + csr_bytes(AT) + sizeof(float) * (uint64_t)A.ncols + sym.bytes();
-    for (auto& kv : plan_A) b += kv.second.ntiles * 24;
-    for (auto& kv : plan_AT) b += kv.second.ntiles * 24;
+    for (auto* plans : {&plan_A, &plan_AT})
+        for (auto& kv : *plans) b += kv.second.ntiles * (kv.second.whole ? 12 : 24);
     b += fused.nchunks * sizeof(FusedChunk) + fused.meta_len * sizeof(uint32_t);
     if (ws.ready) b += (uint64_t)A.nrows * 12 + (uint64_t)A.ncols * 8;
     return b;

@@ -295,8 +295,8 @@ __device__ __forceinline__ void scatter4(float* __restrict__ bp, uint32_t ncols,
 // one), against 0.54 / 0.48 requests when each lane held four consecutive
 // entries and sent them as 16-byte vector reductions.  Measured, every ratio
 // nonzero: k_scatter 0.717 -> 0.485 ms (mid) and 4.12 -> 2.87 ms (12 GB
-// class); k_fused_rescan 4.40 -> 3.19 ms.  No slower in sum, hence not built:
-// 16-byte groups compacted in shared memory (3.01 ms), the next entries
+// class); k_fused_rescan 4.40 -> 3.19 ms.  Measured against the 2.87 ms and not
+// kept: 16-byte groups compacted in shared memory (3.01 ms), the next entries
 // loaded before the reductions (3.06), the row prefetched into L2 (2.98), 8
 // entries in flight (2.95).
 template <typename V, int LPR, int U>
