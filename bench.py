@@ -79,20 +79,29 @@ KERNEL_NAMES = {"direct": "k_csrvec", "persistent": "k_csrvec_pipe", "tma": "k_c
                 "ilv": "k_csr_ilv", "sym": "k_sym_orbit"}
 
 
+def auto_kernels(m):
+    """Kernels of A and Aᵀ that AUTO runs of the handle use: D16 over a copy of the
+    autotuner's own where it holds one, else the configuration that it reports."""
+    return tuple("d16" if own else m.tuning(t)["kernel"] for t, own in zip((False, True), m.own_copies()))
+
+
 def algorithmic_bytes(rows, cols, nnz, sv, m=None, kinds=None):
     """Per-launch algorithmic bytes of the two kernels of an iteration.  With m
-    given and an operand run on its D16 copy (kinds = the FP and BP kernel
-    names, else the autotuner's choices), that operand is counted as its stored
+    given and an operand run on a D16 copy (kinds = the FP and BP kernel names of
+    a named kernel, else those of AUTO runs), that operand is counted as its stored
     entries (2 index bytes + sv each, dummies and padding included) and its
     vector pointers and base columns."""
-    fp = nnz * (sv + 4) + 8 * (rows + 1) + 4 * cols + 4 * rows + 4 * rows   # A, rowptr, x once, g, ratio
-    bp = nnz * (sv + 4) + 8 * (cols + 1) + 4 * rows + 12 * cols             # Aᵀ, colptr, ratio once, norm, f r/w
-    if m is not None and m.d16:
-        kinds = kinds or (m.tuning(False)["kernel"], m.tuning(True)["kernel"])
-        if kinds[0] == "d16":
-            fp = m.d16["slots"] * (sv + 2) + 12 * rows + 8 + 4 * cols + 4 * rows + 4 * rows
-        if kinds[1] == "d16":
-            bp = m.d16["slots_t"] * (sv + 2) + 12 * cols + 8 + 4 * rows + 12 * cols
+    fp_vec = 4 * cols + 4 * rows + 4 * rows     # x once, g, ratio
+    bp_vec = 4 * rows + 12 * cols               # ratio once, norm, f r/w
+    fp = nnz * (sv + 4) + 8 * (rows + 1) + fp_vec   # A, rowptr
+    bp = nnz * (sv + 4) + 8 * (cols + 1) + bp_vec   # Aᵀ, colptr
+    if m is not None:
+        own = m.own_copies() if kinds is None else (0, 0)
+        kinds = kinds or auto_kernels(m)
+        if own[0] or (m.d16 and kinds[0] == "d16"):
+            fp = (own[0] or m.d16["slots"] * (sv + 2) + 12 * rows + 8) + fp_vec
+        if own[1] or (m.d16 and kinds[1] == "d16"):
+            bp = (own[1] or m.d16["slots_t"] * (sv + 2) + 12 * cols + 8) + bp_vec
     return fp, bp
 
 
@@ -881,17 +890,19 @@ def main():
     kt_tma = time_kernels(pkg, m, torch, g, f0, kernel=1)
     kt_pers = time_kernels(pkg, m, torch, g, f0, kernel=2)
     kinds = None if args.kernel == "auto" else (args.kernel, args.kernel)
+    used = kinds or auto_kernels(m)
     fp_b, bp_b = algorithmic_bytes(m.rows, m.cols, m.nnz, sv, m, kinds)
     dom = "fp" if kt["fp"] >= kt["bp"] else "bp"
     dom_bytes = fp_b if dom == "fp" else bp_b
     peak, peak_kind = peaks()
     achieved = dom_bytes / (kt[dom] * 1e-3) / 1e9
     iter_bytes = fp_b + bp_b
+    kernel = KERNEL_NAMES.get(used[dom == "bp"], "k_csrvec")
     traffic = None
     tf = PROFILES / "dram_traffic.json"
-    if tf.exists() and default_form:
+    if tf.exists() and default_form:  # of the kernel that ran, where it was captured
         key = f"{name}/{dom}" + ("/locality" if LAYOUT else "")
-        traffic = json.loads(tf.read_text()).get(key)
+        traffic = json.loads(tf.read_text()).get(kernel, {}).get(key)
 
     line = {
         "metric": "MLEM iterations/s", "value": value, "unit": "iter/s", "n_gpus": world,
@@ -909,9 +920,7 @@ def main():
         "e2e": {"value": e2e_value, "unit": "iter/s", "h2d_bytes_per_step": int(4 * m.rows + 4 * m.cols),
                 "d2h_bytes_per_step": int(4 * m.cols)},
         "gpu_launches": int(launches),
-        "roofline": {"bound": "hbm", "kernel": KERNEL_NAMES.get(kinds[dom == "bp"] if kinds else
-                                                               m.tuning(dom == "bp")["kernel"], "k_csrvec") + " "
-                     + ("(FP, fused correlation)" if dom == "fp" else "(BP over Aᵀ, fused update)"),
+        "roofline": {"bound": "hbm", "kernel": kernel + " " + ("(FP, fused correlation)" if dom == "fp" else "(BP over Aᵀ, fused update)"),
                      "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_kind": peak_kind, "traffic": traffic,
                      "algorithmic_bytes": dom_bytes, "kernel_ms": kt[dom],
@@ -920,6 +929,7 @@ def main():
                                    "frac": iter_bytes / (ms / args.steps / iters * 1e-3) / 1e9 / peak},
                      "fp_ms": kt["fp"], "bp_ms": kt["bp"],
                      "variants_ms": {"autotuned": kt, "direct": kt_direct, "tma": kt_tma, "persistent": kt_pers},
+                     "kernels": {"fp": used[0], "bp": used[1]}, "own_copies_bytes": m.own_copies(),
                      "autotuned": {"fp": m.tuning(False), "bp": m.tuning(True)}},
         "clocks": clk.summary(),
     }
@@ -940,11 +950,12 @@ def main():
         b.record(s)
         torch.cuda.synchronize()
         f_rate = args.steps * iters / (a.elapsed_time(b) * 1e-3)
-        # its algorithmic bytes: one forward-projection stream (A once, the row
-        # pointers, g, f) per iteration; the update's vectors are left out
+        # its algorithmic bytes: one forward-projection stream of the CSR arrays (A
+        # once, the row pointers, g, f) per iteration; the update's vectors are left out
+        fused_b = algorithmic_bytes(m.rows, m.cols, m.nnz, sv)[0]
         line["fused_pass"] = {"iterations_per_s": f_rate, "vs_fp32_plain": f_rate / (value / world),
-                              "form": m.tuning(2), "bytes_per_iteration": fp_b,
-                              "achieved_gbs": fp_b * f_rate / 1e9, "frac": fp_b * f_rate / 1e9 / peak}
+                              "form": m.tuning(2), "bytes_per_iteration": fused_b,
+                              "achieved_gbs": fused_b * f_rate / 1e9, "frac": fused_b * f_rate / 1e9 / peak}
     m.close()
     if args.forms == "modes":
         line["forms"] = run_modes(pkg, torch, name)
