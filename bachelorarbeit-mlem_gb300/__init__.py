@@ -277,19 +277,27 @@ def siddon_host(geo: Geometry):
 # -------------------------------------------------------------------- matrix
 @functools.lru_cache(maxsize=64, typed=True)
 def _kept_opts(**opts):
+    """The run options of a device-pointer call, kept by the types and values of
+    plain numbers: filling the struct field by field took a third of a small
+    projection's host time (the library copies the struct; callers here do not
+    change it)."""
+    if not all(type(v) in (int, bool, float) for v in opts.values()):
+        raise TypeError  # not kept; a tensor or array of one number say
     return C.byref(Matrix.run_opts(**opts))
 
 
 def _device_opts(opts):
-    """The run options of a device-pointer call.  Those of plain numbers are kept
-    by their types and values: filling the struct field by field took a third of a
-    small projection's host time (the library copies the struct; callers here do
-    not change it).  Others, tensors or arrays of one number say, are read on every
-    call."""
-    for v in opts.values():
-        if type(v) not in (int, bool, float):
-            return C.byref(Matrix.run_opts(**opts))
-    return _kept_opts(**opts)
+    try:
+        return _kept_opts(**opts)
+    except TypeError:  # read on every call, with its own error if it has one
+        return C.byref(Matrix.run_opts(**opts))
+
+
+def _addresses(*ptrs):
+    """What a device-pointer call was given in place of integers, through c_void_p,
+    which refuses what is no address: the library's own argument conversion would
+    take bytes, str and ctypes arrays too."""
+    return [_P(p) for p in ptrs]
 
 
 class Matrix:
@@ -485,21 +493,24 @@ class Matrix:
             res.append({k: getattr(st, k) for k, _ in Stats._fields_})
         return res[0] if len(res) == 1 else tuple(res)
 
-    # device-pointer calls: _P (c_void_p) takes integers and None; the library's
-    # own argument conversion would take bytes, str and ctypes arrays too
     def run_device(self, g_dev: int, f_dev: int, iterations: int, stream: int = 0, **opts) -> None:
         """MLEM on device pointers (e.g. torch tensor .data_ptr()); f_dev is updated in place."""
-        _check(load_library().mlem_run_device(self._h, _P(g_dev), _P(f_dev), iterations, _device_opts(opts),
-                                              _P(stream or None)))
+        if not type(g_dev) is type(f_dev) is type(stream) is int:
+            g_dev, f_dev, stream = _addresses(g_dev, f_dev, stream or None)
+        _check(load_library().mlem_run_device(self._h, g_dev, f_dev, iterations, _device_opts(opts), stream))
 
     def forward_project(self, f_dev: int, g_dev: int, ratio_dev: int, fwproj_dev: int = 0, stream: int = 0,
                         **opts) -> None:
-        _check(load_library().mlem_forward_project(self._h, _P(f_dev), _P(g_dev), _P(ratio_dev),
-                                                   _P(fwproj_dev or None), _device_opts(opts), _P(stream or None)))
+        if not type(f_dev) is type(g_dev) is type(ratio_dev) is type(fwproj_dev) is type(stream) is int:
+            f_dev, g_dev, ratio_dev, fwproj_dev, stream = _addresses(f_dev, g_dev, ratio_dev, fwproj_dev or None,
+                                                                     stream or None)
+        _check(load_library().mlem_forward_project(self._h, f_dev, g_dev, ratio_dev, fwproj_dev, _device_opts(opts),
+                                                   stream))
 
     def back_project(self, ratio_dev: int, bp_dev: int, stream: int = 0, **opts) -> None:
-        _check(load_library().mlem_back_project(self._h, _P(ratio_dev), _P(bp_dev), _device_opts(opts),
-                                                _P(stream or None)))
+        if not type(ratio_dev) is type(bp_dev) is type(stream) is int:
+            ratio_dev, bp_dev, stream = _addresses(ratio_dev, bp_dev, stream or None)
+        _check(load_library().mlem_back_project(self._h, ratio_dev, bp_dev, _device_opts(opts), stream))
 
     def batch_run(self, g, iterations, f0=None, tile=0, use_graph=True, order_by_iterations=True,
                   stats=False, form=0):

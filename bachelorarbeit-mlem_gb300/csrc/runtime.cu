@@ -614,7 +614,7 @@ static void tune_projection(mlem_matrix* m, bool transposed, bool copy) {
     std::vector<ProjCfg> cand;
     const int base = pick_lanes(op.nnz, op.nrows);
     const bool brief = m->one_call != 0, is_short = op.nnz <= kShort;
-    if (known && !op.d16 && !copy_bytes_d16(m, op)) {
+    if (known && (op.d16_asked() || (!op.d16 && !copy_bytes_d16(m, op)))) {  // no copy to try
         m->copy_timed[transposed] = true;
         return;
     }
@@ -1048,7 +1048,7 @@ static uint32_t run_iterations(mlem_matrix* m, const mlem_run_opts& o, uint32_t 
         }
     };
     const uint32_t rest = iters % kChunk;
-    const auto last = m->ws.last_rest.emplace(key_of(0), rest).first;
+    const auto last = m->ws.last_rest.try_emplace(key_of(0), rest).first;
     const bool whole = last->second == rest || m->ws.graphs.count(key_of(rest));
     last->second = rest;
     if (iters >= kChunk) replay(kChunk, iters / kChunk);
